@@ -1,0 +1,64 @@
+"""The radix sorts at the sizes where their paths change: one block up to 2048
+and 8192 items, tiles of 1024 up to 303104, then tiles of 4096 (pairs) or 3072
+(64-bit keys with values); pairs by runs of equal left rows, or by all digits
+where rows have many pairs (on average, or one row more than 1024)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+SIZES = [1, 2, 33, 2047, 2048, 2049, 8191, 8192, 8193, 1024 * 9, 1024 * 9 + 1, 303_104, 303_105, 4096 * 80 + 7]
+
+
+@pytest.mark.parametrize("n", SIZES)
+@pytest.mark.parametrize("rows", ["random", "equal", "one_digit", "wide", "short_runs", "long_run", "few_left"])
+def test_pairs(vsabi, ctx, n, rows):
+    import torch
+
+    rng = np.random.default_rng(n)
+    hi = {"random": (50_000_000, 1_000_000), "equal": (1, 1), "one_digit": (1, 200), "wide": (2**31 - 1, 2**31 - 1),
+          "short_runs": (max(1, n // 5), 1000), "long_run": (n, 5000), "few_left": (3, 2**20)}
+    left, right = (rng.integers(0, h, n).astype(np.int32) for h in hi[rows])
+    if rows == "long_run":
+        left[: min(n, 3000)] = n // 2
+        rng.shuffle(left)
+    dl, dr = torch.from_numpy(left).cuda(), torch.from_numpy(right).cuda()
+    vsabi.sort_pairs(ctx, dl, dr)
+    order = np.lexsort((right, left))
+    assert np.array_equal(dl.cpu().numpy(), left[order])
+    assert np.array_equal(dr.cpu().numpy(), right[order])
+
+
+@pytest.mark.parametrize("n", SIZES)
+@pytest.mark.parametrize("bits", [8, 13, 40, 64])
+def test_keys_with_values_are_stable(vsabi, ctx, n, bits):
+    import torch
+
+    rng = np.random.default_rng(n + bits)
+    keys = rng.integers(0, 2**63, n, dtype=np.uint64) & np.uint64(2**bits - 1)
+    keys[n // 2:] = keys[: n - n // 2]  # equal keys keep their order
+    vals = np.arange(n, dtype=np.int32)
+    dk, dv = torch.from_numpy(keys.view(np.int64)).cuda(), torch.from_numpy(vals).cuda()
+    vsabi.radix_sort_pairs(ctx, dk, dv, bits)
+    order = np.argsort(keys, kind="stable")
+    assert np.array_equal(dk.cpu().numpy().view(np.uint64), keys[order])
+    assert np.array_equal(dv.cpu().numpy(), vals[order])
+
+
+def test_join_order(vsabi, ctx, oracle):
+    """A sorted join's pairs (left rows below 2^19, 9-bit digits) equal the sorted unsorted join's."""
+    import torch
+
+    from vibespatial_b200.testing import synthetic as syn
+
+    w = syn.star_join(seed=3, n_points=300_007, n_polys=2_000)
+    dx, dy = torch.from_numpy(w.px).cuda(), torch.from_numpy(w.py).cuda()
+    t = {k: torch.from_numpy(getattr(w.polys, k)).cuda() for k in ("x", "y", "ring_off", "part_off", "geom_off")}
+    idx = vsabi.DeviceIndex(ctx, vsabi.make_polygons(*t.values()), learned=True)
+    pts = vsabi.make_points(dx, dy)
+    left, right, _ = idx.join(pts, vsabi.PRED_WITHIN, vsabi.METHOD_LEARNED, sort=True)
+    ul, ur, _ = idx.join(pts, vsabi.PRED_WITHIN, vsabi.METHOD_LEARNED, sort=False)
+    ul, ur = ul.cpu().numpy(), ur.cpu().numpy()
+    order = np.lexsort((ur, ul))
+    assert np.array_equal(left.cpu().numpy(), ul[order])
+    assert np.array_equal(right.cpu().numpy(), ur[order])

@@ -195,7 +195,8 @@ int vs_index_build(vs_context* ctx, const vs_polygons* polys, const vs_index_opt
     idx->device = ctx->device;
     EventPair ev;
     cudaEventRecord(ev.a, ctx->stream);
-    int st = build_rtree(ctx, polys, idx);
+    int st = clear_sort_error(ctx);
+    if (st == VS_OK) st = build_rtree(ctx, polys, idx);
     if (st == VS_OK) st = build_ring_bins(ctx, idx, opts ? opts->ring_bin_min_vertices : 0);
     if (st == VS_OK && opts && (opts->method_mask & 2)) st = build_learned_index(ctx, idx, opts);
     if (st != VS_OK) {
@@ -205,12 +206,12 @@ int vs_index_build(vs_context* ctx, const vs_polygons* polys, const vs_index_opt
         return st;
     }
     cudaEventRecord(ev.b, ctx->stream);
-    cudaError_t e = cudaStreamSynchronize(ctx->stream);
-    if (e != cudaSuccess) {
-        set_error("index build failed: %s", cudaGetErrorString(e));
+    st = finish_sort(ctx);
+    if (st != VS_OK) {
+        cudaStreamSynchronize(ctx->stream);
         free_index_memory(idx);
         delete idx;
-        return VS_E_CUDA;
+        return st;
     }
     idx->build_ms = ev.ms();
     *out = idx;
@@ -349,8 +350,8 @@ int vs_join(vs_context* ctx, const vs_index* idx, const vs_points* pts, int32_t 
         cudaEventRecord(es.a, s);
         VS_TRY(sort_pairs(ctx, d_left, d_right, n, (uint64_t)pts->n, (uint64_t)idx->n_geoms));
         cudaEventRecord(es.b, s);
-        VS_CUDA_TRY(cudaStreamSynchronize(s));
         if (stats) {
+            VS_CUDA_TRY(cudaEventSynchronize(es.b));
             stats->sort_ms = es.ms();
             stats->kernel_launches = g_launches - launches0;
         }
@@ -386,9 +387,7 @@ int vs_sort_pairs(vs_context* ctx, int32_t* d_left, int32_t* d_right, int64_t n)
         return VS_E_ARG;
     }
     VS_TRY(use_device(ctx->device));
-    VS_TRY(sort_pairs(ctx, d_left, d_right, n, 0xffffffffull, 0xffffffffull));
-    VS_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-    return VS_OK;
+    return n > 1 ? sort_pairs(ctx, d_left, d_right, n, 0xffffffffull, 0xffffffffull) : VS_OK;
 }
 
 int vs_radix_sort_pairs(vs_context* ctx, uint64_t* d_keys, uint32_t* d_vals, int64_t n, int32_t key_bits) {
@@ -397,9 +396,9 @@ int vs_radix_sort_pairs(vs_context* ctx, uint64_t* d_keys, uint32_t* d_vals, int
         return VS_E_ARG;
     }
     VS_TRY(use_device(ctx->device));
-    VS_TRY(radix_sort_u64_u32(d_keys, d_vals, n, key_bits, ctx->stream));
-    VS_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-    return VS_OK;
+    VS_TRY(clear_sort_error(ctx));
+    VS_TRY(radix_sort_u64_u32(d_keys, d_vals, n, key_bits, ctx->stream, 0, &ctx->d_counters[kSortErr]));
+    return finish_sort(ctx);
 }
 
 int vs_hilbert_keys(vs_context* ctx, const double* d_x, const double* d_y, int64_t n, double minx, double miny,

@@ -617,7 +617,7 @@ int finish_join(vs_context* ctx, const vs_index* idx, const vs_points* pts, uint
         cudaEventRecord(es.a, s);
         VS_TRY(sort_pairs(ctx, d_left, d_right, n, (uint64_t)pts->n, (uint64_t)idx->n_geoms));
         cudaEventRecord(es.b, s);
-        VS_CUDA_TRY(cudaStreamSynchronize(s));
+        if (stats) VS_CUDA_TRY(cudaEventSynchronize(es.b));
         if (stats) {
             stats->sort_ms = es.ms();
             stats->kernel_launches = g_launches - launches0;
@@ -1094,7 +1094,7 @@ int vs_join_nearest_polygons(vs_context* ctx, const vs_index* point_index, const
     poly_query_key_kernel<<<resident_grid(poly_query_key_kernel, nq, 256), 256, 0, s>>>(
         *queries, point_index->frame, qbox.p, keys.p, order.p, n_valid.p);
     VS_LAUNCHED("poly_query_key", s);
-    VS_TRY(radix_sort_u32_u32(keys.p, order.p, nq, 32, s, 0));
+    VS_TRY(radix_sort_u32_u32(keys.p, order.p, nq, 32, s, 0, &ctx->d_counters[4]));
     PolyArgs a{};
     a.x = queries->d_x;
     a.y = queries->d_y;

@@ -18,6 +18,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "join.cuh"
 #include "primitives.cuh"
 #include "vs_common.cuh"
 
@@ -342,7 +343,8 @@ int vs_join_export(vs_context* ctx, const int32_t* d_left, const int32_t* d_righ
         VS_TRY(perm.alloc((size_t)m, s));
         export_right_keys_kernel<<<grid_of(export_right_keys_kernel, m), 256, 0, s>>>(kl, kr, m, rkeys.p, perm.p);
         VS_LAUNCHED("export_right_keys", s);
-        VS_TRY(radix_sort_u64_u32(rkeys.p, perm.p, m, 64, s));
+        VS_TRY(clear_sort_error(ctx));
+        VS_TRY(radix_sort_u64_u32(rkeys.p, perm.p, m, 64, s, 0, &ctx->d_counters[kSortErr]));
     }
     const uint32_t* p_perm = right && m > 1 ? perm.p : nullptr;
     // 3. counts per driving row, tile sums and their scan
@@ -404,6 +406,7 @@ int vs_join_export(vs_context* ctx, const int32_t* d_left, const int32_t* d_righ
             missing.p, mpos.p, n_right, body, d_out_left, d_out_right, d_out_src);
         VS_LAUNCHED("export_append", s);
     }
+    if (p_perm) return finish_sort(ctx);
     VS_CUDA_TRY(cudaStreamSynchronize(s));
     return VS_OK;
 }

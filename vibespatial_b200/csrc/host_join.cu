@@ -221,6 +221,7 @@ int vs_join_host(vs_context* ctx, const vs_index* idx, const double* h_x, const 
     int64_t total = 0;
     bool over = false;
     const long long launches0 = g_launches;
+    VS_TRY(clear_sort_error(ctx));
     VS_TRY(copy_in(0));
     for (int64_t k = 0; k < n_chunks; ++k) {
         const int b = (int)(k & 1);
@@ -232,7 +233,8 @@ int vs_join_host(vs_context* ctx, const vs_index* idx, const double* h_x, const 
         unsigned long long* c = ctx->h_counter;
         for (int attempt = 0;; ++attempt) {
             const DeferSink ds{ctx->defer_buf, ctx->defer_cap, &ctx->d_counters[7]};
-            VS_CUDA_TRY(cudaMemsetAsync(ctx->d_counters, 0, kDevCounters * sizeof(unsigned long long), s));
+            // (the sort's error word keeps what earlier chunks set)
+            VS_CUDA_TRY(cudaMemsetAsync(ctx->d_counters, 0, kSortErr * sizeof(unsigned long long), s));
             if (method == VS_METHOD_LEARNED)
                 VS_TRY(launch_learned_join(ctx, idx, &pts, mask, bf.left[b], bf.right[b], bf.cap[b], ds, first));
             else
@@ -267,7 +269,7 @@ int vs_join_host(vs_context* ctx, const vs_index* idx, const double* h_x, const 
         const int64_t cnt = (int64_t)c[0];
         for (int q = 1; q < 8; ++q) totals[q] += c[q];
         if (cnt > 0 && (flags & VS_JOIN_SORT)) {
-            VS_TRY(sort_pairs(ctx, bf.left[b], bf.right[b], cnt, (uint64_t)n, (uint64_t)idx->n_geoms));
+            VS_TRY(enqueue_sort_pairs(ctx, bf.left[b], bf.right[b], cnt, (uint64_t)n, (uint64_t)idx->n_geoms, false));
             VS_CUDA_TRY(cudaEventRecord(st.comp[b], s));
         }
         if (!over && total + cnt <= capacity) {
@@ -285,7 +287,7 @@ int vs_join_host(vs_context* ctx, const vs_index* idx, const double* h_x, const 
     VS_CUDA_TRY(cudaEventRecord(st.t1, st.out));
     VS_CUDA_TRY(cudaStreamSynchronize(st.out));
     VS_CUDA_TRY(cudaStreamSynchronize(st.in));
-    VS_CUDA_TRY(cudaStreamSynchronize(s));
+    VS_TRY(finish_sort(ctx));
     *n_pairs = total;
     if (stats) {
         stats->exact_fallbacks = (int64_t)totals[1];

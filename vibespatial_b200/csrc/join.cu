@@ -369,23 +369,6 @@ __global__ void locate_aligned_kernel(vs_points pts, vs_polygons polys, uint8_t*
     if (n_exact) atomicAdd(&counters[1], (unsigned long long)n_exact);
 }
 
-__global__ void pack_pairs_kernel(const int32_t* __restrict__ l, const int32_t* __restrict__ r, int64_t n, int rbits,
-                                  uint64_t* __restrict__ keys, uint32_t* __restrict__ vals) {
-    for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x) {
-        keys[k] = ((uint64_t)(uint32_t)l[k] << rbits) | (uint64_t)(uint32_t)r[k];
-        vals[k] = 0;
-    }
-}
-
-__global__ void unpack_pairs_kernel(const uint64_t* __restrict__ keys, int64_t n, int rbits, int32_t* __restrict__ l,
-                                    int32_t* __restrict__ r) {
-    const uint64_t rmask = rbits >= 64 ? ~0ull : ((1ull << rbits) - 1);
-    for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x) {
-        l[k] = (int32_t)(keys[k] >> rbits);
-        r[k] = (int32_t)(keys[k] & rmask);
-    }
-}
-
 int bits_for(uint64_t v) {
     int b = 1;
     while (b < 63 && (1ull << b) <= v) ++b;
@@ -417,7 +400,7 @@ int prepare_queries(vs_context* ctx, const vs_index* idx, const vs_points* pts, 
     VS_LAUNCHED("point_sort_key", s);
     // Sorting by the top 24 key bits (a level-12 Hilbert cell) already makes
     // a warp's 32 points spatially coherent; the low byte is left unsorted.
-    VS_TRY(radix_sort_u32_u32(q.keys.p, q.order.p, n, 32, s, 8));
+    VS_TRY(radix_sort_u32_u32(q.keys.p, q.order.p, n, 32, s, 8, &ctx->d_counters[4]));
     return VS_OK;
 }
 
@@ -511,25 +494,42 @@ int launch_locate_aligned(vs_context* ctx, const vs_points* pts, const vs_polygo
     return VS_OK;
 }
 
-int sort_pairs(vs_context* ctx, int32_t* d_left, int32_t* d_right, int64_t n, uint64_t max_left,
-               uint64_t max_right) {
-    if (n <= 1) return VS_OK;
-    const int rbits = bits_for(max_right);
-    const int lbits = bits_for(max_left);
-    if (rbits + lbits > 64) {
-        set_error("pair key does not fit 64 bits");
+int enqueue_sort_pairs(vs_context* ctx, int32_t* d_left, int32_t* d_right, int64_t n, uint64_t max_left,
+                       uint64_t max_right, bool by_runs) {
+    const int lbits = bits_for(max_left), rbits = bits_for(max_right);
+    if (lbits > 32 || rbits > 32) {
+        set_error("pair rows do not fit 32 bits");
         return VS_E_ARG;
     }
+    const int64_t n_left = max_left < 0xffffffffull ? (int64_t)max_left : 0;
+    return radix_sort_pairs(d_left, d_right, n, lbits, rbits, n_left, by_runs, ctx->stream,
+                            &ctx->d_counters[kSortErr]);
+}
+
+int sort_pairs(vs_context* ctx, int32_t* d_left, int32_t* d_right, int64_t n, uint64_t max_left, uint64_t max_right) {
+    for (int attempt = 0; attempt < 2; ++attempt) {
+        VS_TRY(clear_sort_error(ctx));
+        VS_TRY(enqueue_sort_pairs(ctx, d_left, d_right, n, max_left, max_right, attempt == 0));
+        VS_TRY(finish_sort(ctx));
+        if (!(ctx->h_counter[kHostCounters - 1] & 4)) break;  // else: a left row with very many pairs
+    }
+    return VS_OK;
+}
+
+int clear_sort_error(vs_context* ctx) {
+    VS_CUDA_TRY(cudaMemsetAsync(&ctx->d_counters[kSortErr], 0, sizeof(unsigned long long), ctx->stream));
+    return VS_OK;
+}
+
+int finish_sort(vs_context* ctx) {
     cudaStream_t s = ctx->stream;
-    Scratch<uint64_t> keys;
-    Scratch<uint32_t> vals;
-    VS_TRY(keys.alloc((size_t)n, s));
-    VS_TRY(vals.alloc((size_t)n, s));
-    pack_pairs_kernel<<<grid_for(n, 256), 256, 0, s>>>(d_left, d_right, n, rbits, keys.p, vals.p);
-    VS_LAUNCHED("pack_pairs", s);
-    VS_TRY(radix_sort_u64_u32(keys.p, vals.p, n, rbits + lbits, s));
-    unpack_pairs_kernel<<<grid_for(n, 256), 256, 0, s>>>(keys.p, n, rbits, d_left, d_right);
-    VS_LAUNCHED("unpack_pairs", s);
+    unsigned long long* flags = &ctx->h_counter[kHostCounters - 1];
+    VS_CUDA_TRY(cudaMemcpyAsync(flags, &ctx->d_counters[kSortErr], sizeof(*flags), cudaMemcpyDeviceToHost, s));
+    VS_CUDA_TRY(cudaStreamSynchronize(s));
+    if (*flags & 2) {
+        set_error("a bounded device wait (radix sort) gave up; the order is incomplete");
+        return VS_E_TIMEOUT;
+    }
     return VS_OK;
 }
 

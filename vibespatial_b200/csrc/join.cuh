@@ -34,8 +34,16 @@ int ensure_defer_capacity(vs_context* ctx, unsigned long long want);
 // Release the context's vs_join_host pipeline (streams, events, buffers).
 void free_host_pipe(vs_context* ctx);
 int launch_locate_aligned(vs_context* ctx, const vs_points* pts, const vs_polygons* polys, uint8_t* d_out);
+// Sort (left, right) pairs and wait for them; rows below max_left, max_right.
 int sort_pairs(vs_context* ctx, int32_t* d_left, int32_t* d_right, int64_t n, uint64_t max_left,
                uint64_t max_right);
+// The same without waiting (by_runs as for radix_sort_pairs).  Bit 1 of
+// d_counters[kSortErr] (which clear_sort_error zeroes) reports a wait that
+// gave up; finish_sort waits for the stream and reads it.
+int enqueue_sort_pairs(vs_context* ctx, int32_t* d_left, int32_t* d_right, int64_t n, uint64_t max_left,
+                       uint64_t max_right, bool by_runs);
+int clear_sort_error(vs_context* ctx);
+int finish_sort(vs_context* ctx);
 int build_rtree(vs_context* ctx, const vs_polygons* P, vs_index* idx);
 // y-bins for rings of at least min_vertices vertices (0: the default, < 0: none).
 int build_ring_bins(vs_context* ctx, vs_index* idx, int min_vertices);

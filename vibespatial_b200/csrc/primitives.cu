@@ -1,13 +1,13 @@
 // Exclusive scan (reduce -> scan of block sums -> downsweep) and a stable
-// LSD radix sort of (u32/u64 key, u32 value) pairs, 8 bits per pass.
+// LSD radix sort of (u32/u64 key, u32 value) items or (left, right) pairs,
+// 8 bits per pass.
 //
-// Radix sort per pass: (1) per-tile digit histograms with shared atomics,
-// written digit-major so that one exclusive scan over [digit][tile] gives
-// every (digit, tile) its global output offset; (2) a scatter that loads the
-// tile into registers, ranks each key stably with __match_any_sync (peers with
-// the same digit in a warp) plus per-warp digit counts scanned in shared
-// memory, sorts the tile by digit in shared memory and then writes each
-// digit's run contiguously (coalesced), as in one-sweep radix sorts.
+// Radix sort: one read of the keys counts every digit (rs_plan_kernel); then
+// each pass reads and writes the items once (rs_pass_kernel): a tile gets the
+// output position of its digit runs from the tiles before it while it runs (a
+// decoupled look-back over per-tile counts) instead of from a histogram pass
+// and a scan of their own.  Sorts of a few thousand items run in one block
+// (rs_small_kernel).
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -125,170 +125,593 @@ int exclusive_scan_impl(const T* in, T* out, int64_t n, T* d_total, cudaStream_t
 // ------------------------------------------------------------------------
 // Radix sort
 // ------------------------------------------------------------------------
-constexpr int kRsThreads = 256;
+constexpr int kMaxDigits = 8;
+constexpr int kRsThreads = 256;   // histogram blocks
 constexpr int kRsWarps = kRsThreads / 32;
-constexpr int kRadix = 256;
-// 16 keys per thread for 32-bit keys, 8 for 64-bit keys (keeps the tile's
-// shared-memory staging under 48 KB).
+constexpr int kPassThreads = 512;  // pass blocks: a thread a digit value at least
+constexpr int kPassWarps = kPassThreads / 32;
+
+// Which digits the passes sort by: digits that are the same in every key are
+// left out.  Slot k of the pass launches sorts by digit[k] when k < n_slots.
+// full: a pair sort by left and right (its order needs no fixing).
+struct SortPlan {
+    uint32_t n_slots;
+    uint32_t full;
+    uint32_t max_left;
+    uint32_t digit[kMaxDigits];
+};
+
+// How a pair sort orders equal left rows: by digits of right too, or by a last
+// pass over the (short) runs of equal left rows, or the plan decides.
+enum : int { kPairsFull = 0, kPairsRuns = 1, kPairsAuto = 2 };
+// Pairs a left row may have on average for the run pass to be used: with up to
+// 8 it reads a handful of neighbours, and saves the passes over right's digits
+// (half of them for 20-bit rows).
+constexpr int64_t kRunMean = 8;
+constexpr int kRunMax = 1024;  // longest run the run pass orders (each item compares itself with its run)
+
+// One sort.  The items are (key, value) arrays, or (left, right) pairs whose
+// key is left << rbits | right and which carry no value.  Arrays: slot 0 reads
+// the caller's, the last slot writes them; pairs: slot 0 reads the caller's,
+// the run pass writes them.  The slots between alternate between two buffers.
 template <class K>
-struct RsTile {
-    static constexpr int kRounds = sizeof(K) == 8 ? 8 : 16;
-    static constexpr int kTile = kRsThreads * kRounds;
+struct SortArgs {
+    K* keys;            // null: pairs
+    uint32_t* vals;
+    int32_t* left;
+    int32_t* right;
+    int rbits;
+    int pairs_mode;
+    K* kbuf[2];
+    uint32_t* vbuf[2];
+    int64_t n;
+    int shift[kMaxDigits];
+    int n_digits;
+    int n_right;        // pairs: digits [0, n_right) are right's
+    uint32_t* hist;     // [n_digits][radix] counts, then exclusive sums
+    uint32_t* ticket;   // [0] histogram blocks done, [1 + slot] tiles handed out
+    SortPlan* plan;
+    unsigned long long* err;  // nullable
+    int64_t n_tiles;
 };
 
 template <class K>
-__global__ void __launch_bounds__(kRsThreads) rs_histogram_kernel(const K* __restrict__ keys, int64_t n, int shift,
-                                                                  uint32_t* __restrict__ hist, int ntiles) {
-    __shared__ uint32_t h[kRadix];
-    h[threadIdx.x] = 0;
-    __syncthreads();
-    const int64_t base = (int64_t)blockIdx.x * RsTile<K>::kTile;
-#pragma unroll 4
-    for (int r = 0; r < RsTile<K>::kRounds; ++r) {
-        const int64_t i = base + (int64_t)r * kRsThreads + threadIdx.x;
-        if (i < n) atomicAdd(&h[(unsigned)(keys[i] >> shift) & 0xffu], 1u);
-    }
-    __syncthreads();
-    hist[(int64_t)threadIdx.x * ntiles + blockIdx.x] = h[threadIdx.x];
+__device__ __forceinline__ K sort_key(const SortArgs<K>& a, const K* keys, int64_t i) {
+    if (keys) return keys[i];
+    return (K)(((uint64_t)(uint32_t)a.left[i] << a.rbits) | (uint64_t)(uint32_t)a.right[i]);
 }
 
-// Stable scatter of one tile: the tile is ranked and sorted by digit in
-// shared memory first, then written out in digit runs so that consecutive
-// threads write consecutive addresses.
-template <class K>
-__global__ void __launch_bounds__(kRsThreads) rs_scatter_kernel(const K* __restrict__ kin, const uint32_t* __restrict__ vin,
-                                                                K* __restrict__ kout, uint32_t* __restrict__ vout,
-                                                                int64_t n, int shift,
-                                                                const uint32_t* __restrict__ offsets, int ntiles) {
-    constexpr int R = RsTile<K>::kRounds;
-    constexpr int T = RsTile<K>::kTile;
-    __shared__ uint32_t gbase[kRadix];   // global start of (digit, this tile)
-    __shared__ uint32_t lstart[kRadix];  // tile-local start of digit
-    __shared__ uint32_t run[kRadix];     // keys of digit placed by earlier rounds
-    __shared__ uint32_t wcnt[kRsWarps][kRadix];
-    __shared__ uint32_t wsum[kRsWarps];
-    __shared__ K skey[T];
-    __shared__ uint32_t sval[T];
+// Every digit's histogram in one read of the keys; the last block to finish
+// turns them into exclusive sums and writes the plan.  The counters are
+// shared-memory increments.
+template <class K, int kBits>
+__global__ void __launch_bounds__(kRsThreads) rs_plan_kernel(const SortArgs<K> a) {
+    constexpr int kRadix = 1 << kBits, kPer = kRadix / kRsThreads;
+    __shared__ uint32_t h[kMaxDigits][kRadix];
+    __shared__ uint32_t s_one[kMaxDigits];
+    __shared__ uint32_t s_sum[kRsWarps];
+    __shared__ uint32_t s_max;
+    __shared__ bool s_last;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const unsigned lt_mask = (1u << lane) - 1u;
-    const int64_t tile0 = (int64_t)blockIdx.x * T;
-    const int count = (int)((n - tile0) < T ? (n - tile0) : T);
-
-    K k[R];
-    uint32_t v[R];
-    unsigned d[R];
-    lstart[tid] = 0;
-#pragma unroll
-    for (int w = 0; w < kRsWarps; ++w) wcnt[w][tid] = 0;
+    for (int i = tid; i < a.n_digits * kRadix; i += kRsThreads) (&h[0][0])[i] = 0;
+    if (tid == 0) s_max = 0;
     __syncthreads();
+    uint32_t max_left = 0;
+    for (int64_t i = (int64_t)blockIdx.x * kRsThreads + tid; i < a.n; i += (int64_t)gridDim.x * kRsThreads) {
+        const K k = sort_key(a, a.keys, i);
+        if (a.pairs_mode == kPairsAuto) max_left = max(max_left, (uint32_t)((uint64_t)k >> a.rbits));
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-        const int j = r * kRsThreads + tid;
-        d[r] = kRadix;
-        if (j < count) {
-            k[r] = kin[tile0 + j];
-            v[r] = vin[tile0 + j];
-            d[r] = (unsigned)(k[r] >> shift) & 0xffu;
-            atomicAdd(&lstart[d[r]], 1u);
-        }
+        for (int d = 0; d < kMaxDigits; ++d)
+            if (d < a.n_digits) atomicAdd(&h[d][(unsigned)(k >> a.shift[d]) & (kRadix - 1)], 1u);
     }
+    if (a.pairs_mode == kPairsAuto) atomicMax(&s_max, max_left);
     __syncthreads();
-    // exclusive scan of the tile's digit counts (256 entries, one per thread)
-    {
-        const uint32_t c = lstart[tid];
-        uint32_t inc = c;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t t = __shfl_up_sync(0xffffffffu, inc, o);
-            if (lane >= o) inc += t;
-        }
-        if (lane == 31) wsum[warp] = inc;
-        __syncthreads();
-        uint32_t wpre = 0;
-        for (int w = 0; w < warp; ++w) wpre += wsum[w];
-        lstart[tid] = wpre + inc - c;
-        gbase[tid] = offsets[(int64_t)tid * ntiles + blockIdx.x];
-        run[tid] = 0;
-    }
+    for (int i = tid; i < a.n_digits * kRadix; i += kRsThreads)
+        if (uint32_t c = (&h[0][0])[i]) atomicAdd(&a.hist[i], c);
+    if (tid == 0 && s_max) atomicMax(&a.plan->max_left, s_max);
+    __threadfence();
     __syncthreads();
+    if (tid == 0) s_last = atomicAdd(&a.ticket[0], 1u) == gridDim.x - 1;
+    if (tid < kMaxDigits) s_one[tid] = 0;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    for (int d = 0; d < a.n_digits; ++d) {
+        uint32_t c[kPer], t = 0;
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-        const unsigned dd = d[r];
-        const unsigned peers = __match_any_sync(0xffffffffu, dd);
-        const unsigned rank = __popc(peers & lt_mask);
-        if (dd < kRadix && (__ffs(peers) - 1) == lane) wcnt[warp][dd] = __popc(peers);
-        __syncthreads();
-        uint32_t acc = 0;
-#pragma unroll
-        for (int w = 0; w < kRsWarps; ++w) {
-            const uint32_t c = wcnt[w][tid];
-            wcnt[w][tid] = acc;
-            acc += c;
+        for (int u = 0; u < kPer; ++u) {
+            c[u] = __ldcg(&a.hist[d * kRadix + tid * kPer + u]);
+            if ((int64_t)c[u] == a.n) s_one[d] = 1;  // every key has this digit
+            t += c[u];
         }
+        const uint32_t inc = warp_inclusive_scan(t);
+        if (lane == 31) s_sum[warp] = inc;
         __syncthreads();
-        if (dd < kRadix) {
-            const uint32_t pos = lstart[dd] + run[dd] + wcnt[warp][dd] + rank;
-            skey[pos] = k[r];
-            sval[pos] = v[r];
-        }
-        __syncthreads();
-        run[tid] += acc;
+        uint32_t before = inc - t;
+        for (int w = 0; w < warp; ++w) before += s_sum[w];
 #pragma unroll
-        for (int w = 0; w < kRsWarps; ++w) wcnt[w][tid] = 0;
+        for (int u = 0; u < kPer; ++u) {
+            a.hist[d * kRadix + tid * kPer + u] = before;
+            before += c[u];
+        }
         __syncthreads();
     }
-    for (int j = tid; j < count; j += kRsThreads) {
-        const K key = skey[j];
-        const unsigned dd = (unsigned)(key >> shift) & 0xffu;
-        const uint32_t pos = gbase[dd] + (uint32_t)j - lstart[dd];
-        kout[pos] = key;
-        vout[pos] = sval[j];
+    if (tid == 0) {
+        const bool pairs = a.keys == nullptr;
+        const bool full = a.pairs_mode == kPairsFull ||
+                          (a.pairs_mode == kPairsAuto && a.n > kRunMean * ((int64_t)__ldcg(&a.plan->max_left) + 1));
+        uint32_t k = 0;
+        for (int d = full ? 0 : a.n_right; d < a.n_digits; ++d)
+            if (!s_one[d]) a.plan->digit[k++] = (uint32_t)d;
+        // pairs go through a buffer at least once; one slot on arrays would read and write them at once
+        if (pairs && k == 0) a.plan->digit[k++] = (uint32_t)(a.n_digits - 1);
+        if (!pairs && k == 1) a.plan->digit[k++] = a.plan->digit[0];
+        a.plan->full = full ? 1u : 0u;
+        a.plan->n_slots = k;
     }
 }
 
-template <class K>
-int radix_sort_impl(K* keys, uint32_t* vals, int64_t n, int begin_bit, int end_bit, cudaStream_t s) {
-    if (n <= 1) return VS_OK;
-    if (n > 0xffffffffLL) {
-        set_error("radix sort supports at most 2^32-1 items (got %lld)", (long long)n);
-        return VS_E_ARG;
+// Lanes whose digit equals this lane's: a ballot a bit.  (__match_any_sync
+// steps through the distinct digits one after another: a pass over 10M pairs
+// took half as long again with it.)
+template <int kBits>
+__device__ __forceinline__ unsigned same_digit(unsigned d) {
+    unsigned peers = 0xffffffffu;
+#pragma unroll
+    for (int b = 0; b < kBits; ++b) {
+        const bool on = (d >> b) & 1u;
+        const unsigned m = __ballot_sync(0xffffffffu, on);
+        peers &= on ? m : ~m;
     }
+    return peers;
+}
+
+// Stable ranks of R rounds of 32 keys of a warp among the warp's keys of the
+// same digit: rank[r] counts the warp's earlier ones; cnt (the warp's own
+// counters, zeroed) ends as the warp's digit counts.
+template <class K, int kBits, int R>
+__device__ __forceinline__ void warp_rank(const K (&k)[R], int shift, uint32_t* cnt, uint32_t (&rank)[R]) {
+    const unsigned lt = (1u << (threadIdx.x & 31)) - 1u;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const unsigned d = (unsigned)(k[r] >> shift) & ((1u << kBits) - 1u);
+        const unsigned peers = same_digit<kBits>(d);
+        const uint32_t before = cnt[d];
+        __syncwarp();
+        rank[r] = before + __popc(peers & lt);
+        if ((peers & lt) == 0u) cnt[d] = before + __popc(peers);
+        __syncwarp();
+    }
+}
+
+// A tile state is one word, so relaxed accesses carry it whole.
+__device__ __forceinline__ uint32_t load_state(const uint32_t* p) {
+    uint32_t v;
+    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ unsigned long long load_state(const unsigned long long* p) {
+    unsigned long long v;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void store_state(uint32_t* p, uint32_t v) {
+    asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+__device__ __forceinline__ void store_state(unsigned long long* p, unsigned long long v) {
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+
+constexpr int kWaitLimit = 1 << 20;  // polls of earlier tiles before a pass gives up
+// Earlier tiles whose states a tile reads at once: the tiles of a pass's first
+// wave start together and have only counts, no sums, to read from one another.
+constexpr int kLookBack = 8;
+
+template <class K, bool kVals, int kBits, int R>
+struct PassShared {
+    static constexpr int kRadix = 1 << kBits;
+    static constexpr int T = kPassThreads * R;
+    uint32_t wcnt[kPassWarps][kRadix];
+    uint32_t start[kRadix];  // tile-local start of a digit
+    unsigned long long off[kRadix];  // output position of a digit's run minus its tile-local start
+    uint32_t sum[kPassWarps];
+    uint32_t tile;
+    alignas(16) K key[T];
+    uint32_t val[kVals ? T : 1];
+};
+
+// One slot of the sort: the tiles are taken in order (a ticket), so every tile
+// before a running one is running or done.  A tile ranks its keys (warp by
+// warp, no block barrier in between), publishes its digit counts, stages the
+// keys in digit order in shared memory, sums the counts of the tiles before
+// it (each publishes its counts, then its inclusive sums, as value << 2 |
+// state in one word: S), and writes the digit runs.  Keys are read and
+// written once a pass.  A wait that runs out sets bit 1 of *err; positions
+// stay inside the output whatever was read.
+//
+// Bound by instruction issue (the ranks: a ballot a bit) at two blocks an SM.
+// 12.2M pairs with 26 and 20 bits of rows: 94 us the first pass, which need
+// not be stable, 117 us each of the two others (9-bit digits), 440 us the whole
+// sort with the plan and the run pass; a histogram, a scan and a scatter for
+// each of six 8-bit digits took 1160 us.
+template <class K, bool kVals, class S, int kBits, int R, bool kStable>
+__global__ void __launch_bounds__(kPassThreads) rs_pass_kernel(const SortArgs<K> a, int slot, S* __restrict__ status) {
+    using Shared = PassShared<K, kVals, kBits, R>;
+    constexpr int T = Shared::T, kRadix = Shared::kRadix;
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    Shared& sm = *reinterpret_cast<Shared*>(s_raw);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int n_slots = (int)a.plan->n_slots;
+    if (slot >= n_slots) return;
+    const int digit = (int)a.plan->digit[slot];
+    const int shift = a.shift[digit];
+    const K* kin = slot == 0 ? a.keys : a.kbuf[(slot - 1) & 1];
+    const uint32_t* vin = slot == 0 ? a.vals : a.vbuf[(slot - 1) & 1];
+    if (tid == 0) sm.tile = atomicAdd(&a.ticket[1 + slot], 1u);
+    constexpr int kCounters = kStable ? kPassWarps : 1;  // sets of digit counters: a warp's own, or the block's
+    for (int i = tid; i < kCounters * kRadix / 4; i += kPassThreads)
+        reinterpret_cast<uint4*>(&sm.wcnt[0][0])[i] = make_uint4(0, 0, 0, 0);
+    __syncthreads();
+    const int64_t tile = sm.tile;
+    const int64_t tile0 = tile * T;
+    const int count = (int)(a.n - tile0 < T ? a.n - tile0 : T);
+    const int at = warp * 32 * R + lane;
+    K k[R];
+    uint32_t v[R], rank[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int j = at + r * 32;
+        k[r] = ~(K)0;  // past the end: the last digit, ranked behind the tile's own keys
+        v[r] = 0;
+        if (j < count) {
+            k[r] = sort_key(a, kin, tile0 + j);
+            if (kVals) v[r] = vin[tile0 + j];
+        }
+    }
+    if constexpr (kStable) {
+        warp_rank<K, kBits, R>(k, shift, sm.wcnt[warp], rank);
+    } else {
+#pragma unroll
+        for (int r = 0; r < R; ++r) rank[r] = 0;
+#pragma unroll
+        for (int r = 0; r < R; ++r)  // (a key past the end is not counted and not placed)
+            if (at + r * 32 < count) rank[r] = atomicAdd(&sm.wcnt[0][(unsigned)(k[r] >> shift) & (unsigned)(kRadix - 1)], 1u);
+    }
+    __syncthreads();
+    // thread t < radix owns digit t: per-warp starts, the tile's count, its scan
+    uint32_t total = 0, own = 0, before = 0;
+    S* st = status + tile * kRadix + tid;
+    if (tid < kRadix) {
+#pragma unroll
+        for (int w = 0; w < kCounters; ++w) {
+            const uint32_t c = sm.wcnt[w][tid];
+            sm.wcnt[w][tid] = total;
+            total += c;
+        }
+        own = total - (kStable && tid == kRadix - 1 ? (uint32_t)(T - count) : 0u);
+        if (tile > 0) store_state(st, ((S)own << 2) | (S)1);
+        const uint32_t inc = warp_inclusive_scan(total);
+        if (lane == 31) sm.sum[warp] = inc;
+        before = inc - total;
+    }
+    __syncthreads();
+    if (tid < kRadix) {
+        for (int w = 0; w < warp; ++w) before += sm.sum[w];
+        sm.start[tid] = before;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const unsigned d = (unsigned)(k[r] >> shift) & (unsigned)(kRadix - 1);
+        if (!kStable && at + r * 32 >= count) break;
+        const uint32_t pos = sm.start[d] + (kStable ? sm.wcnt[warp][d] : 0u) + rank[r];
+        sm.key[pos] = k[r];
+        if (kVals) sm.val[pos] = v[r];
+    }
+    if (tid < kRadix) {
+        S sum = 0;
+        int polls = 0;
+        for (int64_t t = tile - 1; t >= 0;) {
+            // kLookBack states at once: the loads' latencies overlap
+            S w[kLookBack];
+#pragma unroll
+            for (int j = 0; j < kLookBack; ++j) w[j] = t >= j ? load_state(status + (t - j) * kRadix + tid) : (S)2;
+            bool ready = true, done = false;
+#pragma unroll
+            for (int j = 0; j < kLookBack; ++j) {
+                ready = ready && (w[j] & 3) != 0;
+                if (ready && !done) {
+                    sum += w[j] >> 2;
+                    done = (w[j] & 3) == 2;
+                    --t;
+                }
+            }
+            if (done) break;
+            if (!ready) {
+                // wait for the one state that is missing, without flooding L2
+                while ((load_state(status + t * kRadix + tid) & 3) == 0 && ++polls < kWaitLimit) __nanosleep(40);
+                if (polls >= kWaitLimit) {
+                    if (a.err) atomicOr(a.err, 2ull);
+                    break;
+                }
+            }
+        }
+        store_state(st, ((sum + (S)own) << 2) | (S)2);
+        sm.off[tid] = (unsigned long long)a.hist[digit * kRadix + tid] + sum - before;
+    }
+    __syncthreads();
+    const bool arrays_last = a.keys && slot == n_slots - 1;
+    K* kout = arrays_last ? a.keys : a.kbuf[slot & 1];
+    uint32_t* vout = arrays_last ? a.vals : a.vbuf[slot & 1];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int j = tid + r * kPassThreads;
+        if (j >= count) break;
+        const K key = sm.key[j];
+        const unsigned long long pos = sm.off[(unsigned)(key >> shift) & (unsigned)(kRadix - 1)] + (unsigned)j;
+        if (pos >= (unsigned long long)a.n) continue;  // only after a wait that gave up
+        kout[pos] = key;
+        if (kVals) vout[pos] = sm.val[j];
+    }
+}
+
+// The pairs, sorted by left, back to the caller's arrays; in a run of equal
+// left rows each pair goes to the place its right row gives it (the number of
+// smaller ones in the run, equal ones in their order).  A run longer than
+// kRunMax is left as it is and reported (bit 2 of *err): such pairs are sorted
+// by right's digits instead.
+constexpr int kRunThreads = 256, kRunItems = 8, kRunTile = kRunThreads * kRunItems, kRunHalo = 64;
+
+__global__ void __launch_bounds__(kRunThreads) rs_runs_kernel(const SortArgs<uint64_t> a) {
+    // a tile with kRunHalo neighbours on both sides
+    constexpr int kHeld = kRunTile + 2 * kRunHalo;
+    __shared__ uint32_t s_left[kHeld], s_right[kHeld];
+    const uint64_t* __restrict__ key = a.kbuf[(a.plan->n_slots - 1) & 1];
+    const uint64_t rmask = (1ull << a.rbits) - 1ull;
+    const bool full = a.plan->full != 0;
+    const int64_t tile0 = (int64_t)blockIdx.x * kRunTile;
+    const int64_t held0 = tile0 - kRunHalo;  // the pair s_left[0] holds
+    for (int j = threadIdx.x; j < kHeld; j += kRunThreads) {
+        const int64_t i = held0 + j;
+        if (i < 0 || i >= a.n) continue;
+        const uint64_t k = key[i];
+        s_left[j] = (uint32_t)(k >> a.rbits);
+        s_right[j] = (uint32_t)(k & rmask);
+    }
+    __syncthreads();
+    const int j_lo = held0 < 0 ? (int)-held0 : 0;
+    const int j_hi = a.n - held0 < kHeld ? (int)(a.n - held0) : kHeld;
+    bool too_long = false;
+#pragma unroll
+    for (int u = 0; u < kRunItems; ++u) {
+        const int j0 = u * kRunThreads + (int)threadIdx.x + kRunHalo;
+        if (j0 >= j_hi) break;
+        const uint32_t l = s_left[j0], r = s_right[j0];
+        int64_t pos = held0 + j0;
+        if (!full) {
+            int move = 0;  // larger ones before move behind, smaller ones behind move before
+            int j = j0 - 1;
+            for (; j >= j_lo && s_left[j] == l; --j) move -= s_right[j] > r ? 1 : 0;
+            int len = j0 - j;
+            if (j < j_lo) {  // the run leaves what is held: on in global memory
+                for (int64_t i = held0 + j; i >= 0 && len <= kRunMax && (uint32_t)(key[i] >> a.rbits) == l; --i, ++len)
+                    move -= (uint32_t)(key[i] & rmask) > r ? 1 : 0;
+            }
+            j = j0 + 1;
+            for (; j < j_hi && s_left[j] == l; ++j) move += s_right[j] < r ? 1 : 0;
+            len += j - j0 - 1;
+            if (j >= j_hi) {
+                for (int64_t i = held0 + j; i < a.n && len <= kRunMax && (uint32_t)(key[i] >> a.rbits) == l; ++i, ++len)
+                    move += (uint32_t)(key[i] & rmask) < r ? 1 : 0;
+            }
+            if (len > kRunMax) too_long = true;
+            else pos += move;
+        }
+        a.left[pos] = (int32_t)l;
+        a.right[pos] = (int32_t)r;
+    }
+    if (too_long && a.err) atomicOr(a.err, 4ull);
+}
+
+// A sort of at most kSmallSort items in one block: every pass in shared
+// memory, one launch instead of two plus one a digit.
+constexpr int kRadix = 256;
+constexpr int kSmallThreads = 1024;
+constexpr int kSmallRounds = 8;
+constexpr int kSmallWarps = kSmallThreads / 32;
+constexpr int64_t kSmallSort = (int64_t)kSmallThreads * kSmallRounds;
+
+template <class K, bool kVals, int R>
+__global__ void __launch_bounds__(kSmallThreads) rs_small_kernel(const SortArgs<K> a) {
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    K* s_key = reinterpret_cast<K*>(s_raw);
+    uint32_t* s_val = reinterpret_cast<uint32_t*>(s_key + kSmallThreads * R);
+    uint32_t* wcnt = s_val + (kVals ? kSmallThreads * R : 0);
+    __shared__ uint32_t s_part[4][kRadix];
+    __shared__ uint32_t s_start[kRadix];
+    __shared__ uint32_t s_sum[kRadix / 32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int n = (int)a.n;
+    const int at = warp * 32 * R + lane;
+    K k[R];
+    uint32_t v[R], rank[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int j = at + r * 32;
+        k[r] = ~(K)0;  // past the end: ranked behind every item
+        v[r] = 0;
+        if (j < n) {
+            k[r] = sort_key(a, a.keys, j);
+            if (kVals) v[r] = a.vals[j];
+        }
+    }
+    for (int digit = 0; digit < a.n_digits; ++digit) {
+        const int shift = a.shift[digit];
+        for (int i = tid; i < kSmallWarps * kRadix; i += kSmallThreads) wcnt[i] = 0;
+        __syncthreads();
+        warp_rank<K, 8, R>(k, shift, wcnt + warp * kRadix, rank);
+        __syncthreads();
+        // digit tid % 256, warps [8 q, 8 q + 8): counts to starts within the quarter
+        const int q = tid >> 8, d0 = tid & (kRadix - 1);
+        uint32_t total = 0;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) {
+            uint32_t* c = &wcnt[(q * 8 + w) * kRadix + d0];
+            const uint32_t x = *c;
+            *c = total;
+            total += x;
+        }
+        s_part[q][d0] = total;
+        __syncthreads();
+        if (tid < kRadix) {
+            uint32_t t = 0;
+#pragma unroll
+            for (int w = 0; w < 4; ++w) {
+                const uint32_t x = s_part[w][tid];
+                s_part[w][tid] = t;
+                t += x;
+            }
+            const uint32_t inc = warp_inclusive_scan(t);
+            if (lane == 31) s_sum[warp] = inc;
+            s_start[tid] = inc - t;
+        }
+        __syncthreads();
+        if (tid < kRadix) {
+            uint32_t before = 0;
+            for (int w = 0; w < warp; ++w) before += s_sum[w];
+            s_start[tid] += before;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const unsigned d = (unsigned)(k[r] >> shift) & 0xffu;
+            const uint32_t pos = s_start[d] + s_part[warp >> 3][d] + wcnt[warp * kRadix + d] + rank[r];
+            s_key[pos] = k[r];
+            if (kVals) s_val[pos] = v[r];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            k[r] = s_key[at + r * 32];
+            if (kVals) v[r] = s_val[at + r * 32];
+        }
+    }
+    const uint32_t rmask = (uint32_t)((1ull << a.rbits) - 1ull);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int j = at + r * 32;
+        if (j >= n) continue;
+        if (a.keys) {
+            a.keys[j] = k[r];
+            if (kVals) a.vals[j] = v[r];
+        } else {
+            a.left[j] = (int32_t)((uint64_t)k[r] >> a.rbits);
+            a.right[j] = (int32_t)((uint32_t)k[r] & rmask);
+        }
+    }
+}
+
+template <class K, bool kVals, int R>
+int launch_small_sort(const SortArgs<K>& a, cudaStream_t s) {
+    constexpr size_t smem = (size_t)kSmallThreads * R * (sizeof(K) + (kVals ? sizeof(uint32_t) : 0)) +
+                            (size_t)kSmallWarps * kRadix * sizeof(uint32_t);
+    auto* kernel = rs_small_kernel<K, kVals, R>;
+    VS_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kernel<<<1, kSmallThreads, smem, s>>>(a);
+    VS_LAUNCHED("rs_small", s);
+    return VS_OK;
+}
+
+template <class K, bool kVals, class S, int kBits, int R>
+int run_passes(SortArgs<K>& a, cudaStream_t s) {
+    constexpr int kRadix = 1 << kBits;
+    constexpr int64_t T = (int64_t)kPassThreads * R;
+    a.n_tiles = (a.n + T - 1) / T;
+    const bool pairs = a.keys == nullptr;
+    int slots = pairs && a.pairs_mode == kPairsRuns ? a.n_digits - a.n_right : a.n_digits;
+    if (!pairs && slots < 2) slots = 2;
+    // one zeroed block: tickets, plan, histograms, the slots' tile states
+    constexpr size_t kHead = 64 * sizeof(uint32_t);
+    const size_t hist_b = (size_t)a.n_digits * kRadix * sizeof(uint32_t);
+    const size_t status_b = (size_t)a.n_tiles * kRadix * sizeof(S);
+    Scratch<char> state;
+    Scratch<K> k0, k1;
+    Scratch<uint32_t> v0, v1;
+    const bool two = slots > (pairs ? 1 : 2);
+    VS_TRY(state.alloc(kHead + hist_b + (size_t)slots * status_b, s));
+    VS_TRY(k0.alloc((size_t)a.n, s));
+    if (two) VS_TRY(k1.alloc((size_t)a.n, s));
+    if (kVals) {
+        VS_TRY(v0.alloc((size_t)a.n, s));
+        if (two) VS_TRY(v1.alloc((size_t)a.n, s));
+    }
+    a.kbuf[0] = k0.p;
+    a.kbuf[1] = k1.p;
+    a.vbuf[0] = v0.p;
+    a.vbuf[1] = v1.p;
+    a.ticket = reinterpret_cast<uint32_t*>(state.p);
+    a.plan = reinterpret_cast<SortPlan*>(a.ticket + 16);
+    a.hist = a.ticket + 64;
+    S* status = reinterpret_cast<S*>(state.p + kHead + hist_b);
+    VS_CUDA_TRY(cudaMemsetAsync(state.p, 0, kHead + hist_b + (size_t)slots * status_b, s));
+    rs_plan_kernel<K, kBits><<<grid_for((a.n + 15) / 16, kRsThreads, 8), kRsThreads, 0, s>>>(a);
+    VS_LAUNCHED("rs_plan", s);
+    constexpr size_t smem = sizeof(PassShared<K, kVals, kBits, R>);
+    for (int k = 0; k < slots; ++k) {
+        // the order the pairs come in does not matter, so their first pass need not keep it
+        auto* kernel = k == 0 && !kVals ? rs_pass_kernel<K, kVals, S, kBits, R, kVals>
+                                        : rs_pass_kernel<K, kVals, S, kBits, R, true>;
+        VS_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        kernel<<<(unsigned)a.n_tiles, kPassThreads, smem, s>>>(a, k, status + (size_t)k * a.n_tiles * kRadix);
+        VS_LAUNCHED("rs_pass", s);
+    }
+    if constexpr (!kVals) {
+        rs_runs_kernel<<<(unsigned)((a.n + kRunTile - 1) / kRunTile), kRunThreads, 0, s>>>(a);
+        VS_LAUNCHED("rs_runs", s);
+    }
+    return VS_OK;
+}
+
+// Keys a thread of a pass holds: 8 (6 with values behind 64-bit keys); 2 up to
+// this many items, so that a small sort spreads over the SMs and its tiles
+// take less time each.
+constexpr int64_t kFewItems = (int64_t)kNumSMs * kPassThreads * 4;
+
+template <class K, bool kVals, int kBits>
+int run_sort(SortArgs<K>& a, cudaStream_t s) {
+    constexpr int R = sizeof(K) + (kVals ? 4 : 0) > 8 ? 6 : 8;
+    if (a.n <= kFewItems) return run_passes<K, kVals, uint32_t, kBits, 2>(a, s);
+    // tile states hold sums below 2^30 in 32-bit words
+    if (a.n < (1ll << 30)) return run_passes<K, kVals, uint32_t, kBits, R>(a, s);
+    return run_passes<K, kVals, unsigned long long, kBits, R>(a, s);
+}
+
+int check_count(int64_t n) {
+    if (n <= 0xffffffffLL) return VS_OK;
+    set_error("radix sort supports at most 2^32-1 items (got %lld)", (long long)n);
+    return VS_E_ARG;
+}
+
+// Digits of `bits` bits each over key bits [begin, end), the last one ending
+// at or past `end`; one that would reach past the key's top bit overlaps the
+// one before it instead, which still sorts stably.
+template <class K>
+void add_digits(SortArgs<K>& a, int begin, int end, int bits) {
+    const int max_bits = (int)(8 * sizeof(K));
+    for (int sh = begin; sh < end; sh += bits) a.shift[a.n_digits++] = sh + bits > max_bits ? max_bits - bits : sh;
+}
+
+template <class K>
+int sort_arrays(SortArgs<K>& a, int begin_bit, int end_bit, cudaStream_t s) {
+    if (a.n <= 1) return VS_OK;
+    VS_TRY(check_count(a.n));
     const int max_bits = (int)(8 * sizeof(K));
     if (end_bit <= 0 || end_bit > max_bits) end_bit = max_bits;
     if (begin_bit < 0 || begin_bit >= end_bit) begin_bit = 0;
-    const int passes = (end_bit - begin_bit + 7) / 8;
-    constexpr int T = RsTile<K>::kTile;
-    const int ntiles = (int)((n + T - 1) / T);
-    Scratch<K> kalt;
-    Scratch<uint32_t> valt, hist;
-    VS_TRY(kalt.alloc((size_t)n, s));
-    VS_TRY(valt.alloc((size_t)n, s));
-    VS_TRY(hist.alloc((size_t)kRadix * ntiles, s));
-    K* ka = keys;
-    uint32_t* va = vals;
-    K* kb = kalt.p;
-    uint32_t* vb = valt.p;
-    for (int p = 0; p < passes; ++p) {
-        // the last pass may overlap the previous one's bits: it still sorts stably
-        int shift = begin_bit + 8 * p;
-        if (shift + 8 > max_bits) shift = max_bits - 8;
-        rs_histogram_kernel<K><<<ntiles, kRsThreads, 0, s>>>(ka, n, shift, hist.p, ntiles);
-        VS_LAUNCHED("rs_histogram", s);
-        VS_TRY(exclusive_scan_u32(hist.p, hist.p, (int64_t)kRadix * ntiles, nullptr, s));
-        rs_scatter_kernel<K><<<ntiles, kRsThreads, 0, s>>>(ka, va, kb, vb, n, shift, hist.p, ntiles);
-        VS_LAUNCHED("rs_scatter", s);
-        K* tk = ka;
-        ka = kb;
-        kb = tk;
-        uint32_t* tv = va;
-        va = vb;
-        vb = tv;
-    }
-    if (ka != keys) {
-        VS_CUDA_TRY(cudaMemcpyAsync(keys, ka, (size_t)n * sizeof(K), cudaMemcpyDeviceToDevice, s));
-        VS_CUDA_TRY(cudaMemcpyAsync(vals, va, (size_t)n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
-    }
-    return VS_OK;
+    add_digits(a, begin_bit, end_bit, 8);
+    if (a.n <= 2 * kSmallThreads) return launch_small_sort<K, true, 2>(a, s);
+    if (a.n <= kSmallSort) return launch_small_sort<K, true, kSmallRounds>(a, s);
+    return run_sort<K, true, 8>(a, s);
 }
 
 }  // namespace
@@ -300,12 +723,60 @@ int exclusive_scan_u64(const uint64_t* in, uint64_t* out, int64_t n, uint64_t* d
     return exclusive_scan_impl<uint64_t>(in, out, n, d_total, s);
 }
 
-int radix_sort_u64_u32(uint64_t* keys, uint32_t* vals, int64_t n, int key_bits, cudaStream_t s, int begin_bit) {
-    return radix_sort_impl<uint64_t>(keys, vals, n, begin_bit, key_bits, s);
+int radix_sort_u64_u32(uint64_t* keys, uint32_t* vals, int64_t n, int key_bits, cudaStream_t s, int begin_bit,
+                       unsigned long long* err) {
+    SortArgs<uint64_t> a{};
+    a.keys = keys;
+    a.vals = vals;
+    a.n = n;
+    a.err = err;
+    return sort_arrays(a, begin_bit, key_bits, s);
 }
 
-int radix_sort_u32_u32(uint32_t* keys, uint32_t* vals, int64_t n, int key_bits, cudaStream_t s, int begin_bit) {
-    return radix_sort_impl<uint32_t>(keys, vals, n, begin_bit, key_bits, s);
+int radix_sort_u32_u32(uint32_t* keys, uint32_t* vals, int64_t n, int key_bits, cudaStream_t s, int begin_bit,
+                       unsigned long long* err) {
+    SortArgs<uint32_t> a{};
+    a.keys = keys;
+    a.vals = vals;
+    a.n = n;
+    a.err = err;
+    return sort_arrays(a, begin_bit, key_bits, s);
+}
+
+int radix_sort_pairs(int32_t* left, int32_t* right, int64_t n, int left_bits, int right_bits, int64_t n_left,
+                     bool by_runs, cudaStream_t s, unsigned long long* err) {
+    if (n <= 1) return VS_OK;
+    VS_TRY(check_count(n));
+    SortArgs<uint64_t> a{};
+    a.left = left;
+    a.right = right;
+    a.rbits = right_bits;
+    a.n = n;
+    a.err = err;
+    if (n <= kSmallSort) {
+        add_digits(a, 0, left_bits + right_bits, 8);
+        return n <= 2 * kSmallThreads ? launch_small_sort<uint64_t, false, 2>(a, s)
+                                      : launch_small_sort<uint64_t, false, kSmallRounds>(a, s);
+    }
+    a.pairs_mode = !by_runs ? kPairsFull : n_left <= 0 ? kPairsAuto : n > kRunMean * n_left ? kPairsFull : kPairsRuns;
+    if (a.pairs_mode == kPairsRuns) {
+        // 9-bit digits where they save a pass over left's bits
+        if ((left_bits + 8) / 9 < (left_bits + 7) / 8) {
+            add_digits(a, right_bits, right_bits + left_bits, 9);
+            return run_sort<uint64_t, false, 9>(a, s);
+        }
+        add_digits(a, right_bits, right_bits + left_bits, 8);
+        return run_sort<uint64_t, false, 8>(a, s);
+    }
+    if (a.pairs_mode == kPairsAuto) {
+        // right's digits apart from left's: the plan may drop them
+        add_digits(a, 0, right_bits, 8);
+        a.n_right = a.n_digits;
+        add_digits(a, right_bits, right_bits + left_bits, 8);
+    } else {
+        add_digits(a, 0, left_bits + right_bits, 8);
+    }
+    return run_sort<uint64_t, false, 8>(a, s);
 }
 
 }  // namespace vs

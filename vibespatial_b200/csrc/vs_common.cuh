@@ -19,8 +19,9 @@ int check_polygons(const vs_polygons* p);
 // Pinned host words of a context (read-back of the device counters and of
 // per-call extras).
 constexpr int kHostCounters = 16;
-constexpr int kDevCounters = 16;
+constexpr int kDevCounters = 17;
 constexpr int kWorkCounter = 8;
+constexpr int kSortErr = 16;  // bit 1: a bounded wait of a pair sort gave up
 
 #define VS_CUDA_TRY(expr)                                                        \
     do {                                                                         \
@@ -139,7 +140,8 @@ struct vs_context {
     // [0] pair count, [1] exact-fallback count, [2] fp32-filter decided
     // edges, [3] edges sent past the fp32 filter, [4] error flags,
     // [5] candidate (bbox) count, [6] wide learned-index windows,
-    // [7] deferred pairs, [8] work queue of the refine kernel.
+    // [7] deferred pairs, [8] work queue of the refine kernel, [16] error
+    // flags of the pair sort.
     unsigned long long* d_counters;
     // Pairs deferred to the exact pass (grown on demand).
     int2* defer_buf;
