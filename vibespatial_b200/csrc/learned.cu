@@ -18,12 +18,12 @@
 // The query passes over this index live in learned_query.cu.
 #include <cuda_runtime.h>
 #include <math.h>
+#include <stddef.h>
 #include <stdint.h>
 #include <stdio.h>
 
 #include <algorithm>
 #include <cmath>
-#include <vector>
 
 #include "emit.cuh"
 #include "exact.cuh"
@@ -41,7 +41,6 @@ constexpr int kThreads = 256;
 constexpr int kRmiP = kRmiHidden + kRmiHidden + kRmiHidden * kRmiHidden + kRmiHidden + kRmiHidden + 1;  // 1153
 constexpr int kOffW1 = 0, kOffB1 = 32, kOffW2 = 64, kOffB2 = 64 + 1024, kOffW3 = 64 + 1024 + 32,
               kOffB3 = 64 + 1024 + 64;
-constexpr int kTrainBlocks = 64;
 
 __device__ __forceinline__ void frame_q(const double* fr, double& lox, double& loy, double& sx, double& sy) {
     lox = fr[0];
@@ -372,126 +371,371 @@ __global__ void pack_leaves_kernel(int nl, const double2* __restrict__ ab, const
 }
 
 // ------------------------------------------------------------ RMI train ---
-// Training pairs: x = normalised ancestor key of stored cell i, t = i / n.
-__global__ void rmi_samples_kernel(const uint32_t* __restrict__ keys, int64_t n, int S, int anc_shift, double key_lo,
-                                   double key_scale, float* __restrict__ xs, float* __restrict__ ts) {
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < S; s += gridDim.x * blockDim.x) {
-        const int64_t i = (int64_t)((double)s * (double)n / (double)S);
-        xs[s] = __double2float_rn(((double)(keys[i] >> anc_shift) - key_lo) * key_scale);
-        ts[s] = (float)((double)i / (double)n);
-    }
-}
+// The whole training of the root MLP in one cooperative launch: samples
+// x = normalised ancestor key of stored cell i, t = i / n (S of them, evenly
+// spread over the keys), full-batch mean squared error, Adam.
+//
+// Two lanes share two samples, each taking half of the layer-2 units of both
+// (the weights come from shared memory, whose bandwidth bounds the products).
+// The block's 128 samples' activations go to shared memory, where each warp
+// forms the weight gradients of its 32 samples as a
+// 32 x 32 outer-product sum (a lane owns 4 x 8 of it).  The blocks add their
+// sums to one of three rotating gradient buffers in L2, meet at one grid
+// barrier a step, and each applies the same Adam update to its own copy of
+// the weights.  One launch a pass of gradient, reduction and update took
+// 69 us a step (64 blocks, a warp a sample, the hidden layer's products by
+// shuffles): 20.7 of the 31 ms of building a 100k-footprint index.  FP32
+// throughout, two products an instruction (fma.rn.f32x2).
+constexpr int kTrainThreads = 128;
+constexpr int kTrainWarps = kTrainThreads / 32;
+constexpr int kTrainSamples = 16384;
+static_assert(kTrainSamples / kTrainThreads <= kNumSMs, "the training blocks run at once, one an SM");
+constexpr int kTrainStride = 36;  // floats a sample row: 16-byte rows whose lanes' stores miss one another's banks
+constexpr int kGradWords = 1160;  // kRmiP gradients, the loss, padding to 16 bytes
+constexpr int kLossWord = kRmiP;
+constexpr int kTrainWaitLimit = 1 << 21;
 
-// Full-batch gradient of the mean squared error over S samples.  A warp takes
-// one sample at a time with lane j owning hidden unit j; each block sums its
-// warps' gradients in shared memory and writes one partial row.
-__global__ void __launch_bounds__(kThreads) rmi_grad_kernel(const float* __restrict__ P, const float* __restrict__ xs,
-                                                            const float* __restrict__ ts, int S,
-                                                            float* __restrict__ partial, float* __restrict__ loss) {
-    __shared__ float g[kRmiP];
-    for (int i = threadIdx.x; i < kRmiP; i += blockDim.x) g[i] = 0.f;
+struct TrainArgs {
+    const uint32_t* keys;
+    int64_t n;
+    int S, anc_shift, steps, n_leaves;
+    float* grad;         // [3][kGradWords], zeroed
+    unsigned* arrived;   // zeroed
+    float* loss;
+    RmiModel* model;
+    unsigned long long* err;
+};
+
+// Shared memory of a training block.
+struct TrainShared {
+    float P[kGradWords];                      // weights (kOff*)
+    float m1[kRmiP], m2[kRmiP];               // Adam moments
+    float pad[2];
+    float h1[kTrainThreads][kTrainStride];    // layer-1 outputs
+    float d2[kTrainThreads][kTrainStride];    // layer-2 errors
+    float h2[kTrainThreads][kTrainStride];    // layer-2 outputs times the output error
+    float d1[kTrainThreads][kTrainStride];    // layer-1 errors
+    float part[kTrainWarps][kRmiP + 3];       // per-warp gradient sums
+    float x[kTrainThreads], gy[kTrainThreads], sq[kTrainThreads];
+    double knot[33];
+    double key_lo, key_scale;
+    int fail;
+};
+static_assert(sizeof(TrainShared) <= 200 * 1024, "one block an SM");
+static_assert((offsetof(TrainShared, h1) & 15) == 0, "rows are read 16 bytes at a time");
+
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+    f32x2 v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b));
+    return v;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 v;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(v) : "l"(a), "l"(b), "l"(c));
+    return v;
+}
+__device__ __forceinline__ ulonglong2 load4(const float* p) { return *reinterpret_cast<const ulonglong2*>(p); }
+
+__global__ void __launch_bounds__(kTrainThreads) rmi_train_kernel(const TrainArgs a) {
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    TrainShared& sm = *reinterpret_cast<TrainShared*>(s_raw);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    // ancestor-key range and quantile knots
+    for (int j = tid; j < 33; j += kTrainThreads) {
+        const int64_t pos = (int64_t)((double)j * (double)(a.n - 1) / 32.0);
+        sm.knot[j] = (double)(a.keys[pos] >> a.anc_shift);
+    }
+    for (int i = tid; i < kGradWords; i += kTrainThreads) sm.P[i] = 0.f;
+    for (int i = tid; i < kRmiP; i += kTrainThreads) sm.m1[i] = sm.m2[i] = 0.f;
     __syncthreads();
-    const int j = threadIdx.x & 31;
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int nwarps = (gridDim.x * blockDim.x) >> 5;
-    const float w1 = P[kOffW1 + j], b1 = P[kOffB1 + j], b2 = P[kOffB2 + j], w3 = P[kOffW3 + j], b3 = P[kOffB3];
-    float row[kRmiHidden], col[kRmiHidden], grow[kRmiHidden];
-#pragma unroll
-    for (int k = 0; k < kRmiHidden; ++k) {
-        row[k] = P[kOffW2 + j * kRmiHidden + k];
-        col[k] = P[kOffW2 + k * kRmiHidden + j];
-        grow[k] = 0.f;
+    const double key_lo = sm.knot[0];
+    const double span = sm.knot[32] - key_lo;
+    const double key_scale = span > 0 ? 1.0 / span : 0.0;
+    // Initial root: a piecewise-linear interpolant of the key CDF through the
+    // 33 quantile knots (h1_j = relu(x - c_j), W2 = I, w3_j = slope change).
+    if (tid < 32) {
+        auto slope = [&](int j) {
+            if (j < 0) return 0.0;
+            const double dx = (sm.knot[j + 1] - key_lo) * key_scale - (sm.knot[j] - key_lo) * key_scale;
+            return dx > 1e-12 ? ((double)(j + 1) / 32.0 - (double)j / 32.0) / dx : 0.0;
+        };
+        sm.P[kOffW1 + tid] = 1.0f;
+        sm.P[kOffB1 + tid] = (float)-((sm.knot[tid] - key_lo) * key_scale);
+        sm.P[kOffW2 + tid * kRmiHidden + tid] = 1.0f;
+        sm.P[kOffW3 + tid] = (float)(slope(tid) - slope(tid - 1));
     }
-    float gw1 = 0.f, gb1 = 0.f, gb2 = 0.f, gw3 = 0.f, gb3 = 0.f, l2 = 0.f;
-    const float inv = 1.0f / (float)S;
-    for (int s = warp; s < S; s += nwarps) {
-        const float x = xs[s], t = ts[s];
-        const float z1 = fmaf(w1, x, b1);
-        const float h1 = fmaxf(z1, 0.f);
-        float z2 = b2;
+    // Two neighbouring lanes share two samples; each takes half of the layer-2 units
+    const int half = tid & 1, row0 = tid - half, j0 = half * (kRmiHidden / 2);
+    bool live[2];
+    float x[2], t[2];
 #pragma unroll
-        for (int k = 0; k < kRmiHidden; ++k) z2 = fmaf(row[k], __shfl_sync(0xffffffffu, h1, k), z2);
-        const float h2 = fmaxf(z2, 0.f);
-        float y = w3 * h2;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
-        y += b3;
-        const float err = y - t;
-        const float gy = 2.f * err * inv;
-        l2 += err * err * inv;
-        gw3 += gy * h2;
-        gb3 += gy;
-        const float d2 = z2 > 0.f ? gy * w3 : 0.f;
-        gb2 += d2;
-#pragma unroll
-        for (int k = 0; k < kRmiHidden; ++k) grow[k] = fmaf(d2, __shfl_sync(0xffffffffu, h1, k), grow[k]);
-        float dh1 = 0.f;
-#pragma unroll
-        for (int i = 0; i < kRmiHidden; ++i) dh1 = fmaf(__shfl_sync(0xffffffffu, d2, i), col[i], dh1);
-        const float d1 = z1 > 0.f ? dh1 : 0.f;
-        gw1 += d1 * x;
-        gb1 += d1;
+    for (int q = 0; q < 2; ++q) {
+        const int s = blockIdx.x * kTrainThreads + row0 + q;
+        live[q] = s < a.S;
+        x[q] = t[q] = 0.f;
+        if (live[q]) {
+            const int64_t i = (int64_t)((double)s * (double)a.n / (double)a.S);
+            x[q] = __double2float_rn(((double)(a.keys[i] >> a.anc_shift) - key_lo) * key_scale);
+            t[q] = (float)((double)i / (double)a.n);
+        }
     }
-    atomicAdd(&g[kOffW1 + j], gw1);
-    atomicAdd(&g[kOffB1 + j], gb1);
-    atomicAdd(&g[kOffB2 + j], gb2);
-    atomicAdd(&g[kOffW3 + j], gw3);
-#pragma unroll
-    for (int k = 0; k < kRmiHidden; ++k) atomicAdd(&g[kOffW2 + j * kRmiHidden + k], grow[k]);
-    if (j == 0) {
-        atomicAdd(&g[kOffB3], gb3);
-        atomicAdd(loss, l2);
-    }
+    sm.x[tid] = half ? x[1] : x[0];
+    if (tid == 0) sm.fail = 0;
     __syncthreads();
-    for (int i = threadIdx.x; i < kRmiP; i += blockDim.x) partial[(int64_t)blockIdx.x * kRmiP + i] = g[i];
-}
-
-__global__ void rmi_adam_kernel(float* __restrict__ P, float* __restrict__ m1, float* __restrict__ m2,
-                                const float* __restrict__ partial, int G, int step, float lr) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= kRmiP) return;
-    float g = 0.f;
-    for (int b = 0; b < G; ++b) g += partial[(int64_t)b * kRmiP + p];
-    const float b1 = 0.9f, b2 = 0.999f;
-    const float m = b1 * m1[p] + (1.f - b1) * g;
-    const float v = b2 * m2[p] + (1.f - b2) * g * g;
-    m1[p] = m;
-    m2[p] = v;
-    const float mh = m / (1.f - powf(b1, (float)step));
-    const float vh = v / (1.f - powf(b2, (float)step));
-    P[p] -= lr * mh / (sqrtf(vh) + 1e-8f);
-}
-
-__global__ void rmi_pack_kernel(const float* __restrict__ P, RmiModel* __restrict__ m, double key_lo, double key_scale,
-                                int n_leaves, int n_keys) {
-    for (int i = threadIdx.x; i < kRmiHidden * kRmiHidden; i += blockDim.x) m->w2[i] = P[kOffW2 + i];
-    for (int i = threadIdx.x; i < kRmiHidden; i += blockDim.x) {
-        m->w1[i] = P[kOffW1 + i];
-        m->b1[i] = P[kOffB1 + i];
-        m->b2[i] = P[kOffB2 + i];
-        m->w3[i] = P[kOffW3 + i];
+    const float inv = 1.0f / (float)a.S;
+    for (int step = 1; step <= a.steps; ++step) {
+        float* grad = a.grad + (step % 3) * kGradWords;
+        // forward: both samples of the pair through this lane's half of the
+        // layer-2 units, so that a weight read from shared memory serves two
+        f32x2 h1[2][kRmiHidden / 2];
+#pragma unroll
+        for (int k = 0; k < kRmiHidden; k += 2) {
+            const float w0 = sm.P[kOffW1 + k], w1 = sm.P[kOffW1 + k + 1];
+            const float c0 = sm.P[kOffB1 + k], c1 = sm.P[kOffB1 + k + 1];
+#pragma unroll
+            for (int q = 0; q < 2; ++q)
+                h1[q][k / 2] = pack2(fmaxf(fmaf(w0, x[q], c0), 0.f), fmaxf(fmaf(w1, x[q], c1), 0.f));
+        }
+        float y[2] = {0.f, 0.f};
+#pragma unroll 1
+        for (int j = j0; j < j0 + kRmiHidden / 2; j += 2) {
+            float h2[2][2];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                f32x2 za[2], zb[2];
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    za[q] = pack2(sm.P[kOffB2 + j + u], 0.f);
+                    zb[q] = 0ull;
+                }
+#pragma unroll
+                for (int k = 0; k < kRmiHidden; k += 4) {
+                    const ulonglong2 w = load4(&sm.P[kOffW2 + (j + u) * kRmiHidden + k]);
+#pragma unroll
+                    for (int q = 0; q < 2; ++q) {
+                        za[q] = fma2(w.x, h1[q][k / 2], za[q]);
+                        zb[q] = fma2(w.y, h1[q][k / 2 + 1], zb[q]);
+                    }
+                }
+                const float w3 = sm.P[kOffW3 + j + u];
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    const float2 a2 = unpack2(za[q]), b2 = unpack2(zb[q]);
+                    h2[q][u] = fmaxf((a2.x + a2.y) + (b2.x + b2.y), 0.f);
+                    y[q] = fmaf(w3, h2[q][u], y[q]);
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < 2; ++q)
+                *reinterpret_cast<float2*>(&sm.h2[row0 + q][j]) = make_float2(h2[q][0], h2[q][1]);
+        }
+        float gy[2];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            y[q] += __shfl_xor_sync(0xffffffffu, y[q], 1);
+            const float e = live[q] ? (y[q] + sm.P[kOffB3]) - t[q] : 0.f;
+            gy[q] = 2.f * e * inv;
+            if (q == half) {
+                sm.gy[tid] = gy[q];
+                sm.sq[tid] = e * e * inv;
+            }
+        }
+        // backward
+        f32x2 dh[2][kRmiHidden / 2];
+#pragma unroll
+        for (int k = 0; k < kRmiHidden / 2; ++k) dh[0][k] = dh[1][k] = 0ull;
+#pragma unroll
+        for (int k = 0; k < kRmiHidden / 2; k += 2)
+            *reinterpret_cast<ulonglong2*>(&sm.h1[tid][2 * k]) =
+                half ? make_ulonglong2(h1[1][k], h1[1][k + 1]) : make_ulonglong2(h1[0][k], h1[0][k + 1]);
+#pragma unroll 1
+        for (int j = j0; j < j0 + kRmiHidden / 2; j += 2) {
+            float d[2][2], g2[2][2];
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                const float2 h = *reinterpret_cast<const float2*>(&sm.h2[row0 + q][j]);
+                d[q][0] = h.x > 0.f ? gy[q] * sm.P[kOffW3 + j] : 0.f;
+                d[q][1] = h.y > 0.f ? gy[q] * sm.P[kOffW3 + j + 1] : 0.f;
+                g2[q][0] = gy[q] * h.x;
+                g2[q][1] = gy[q] * h.y;
+            }
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const f32x2 d0 = pack2(d[0][u], d[0][u]), d1 = pack2(d[1][u], d[1][u]);
+#pragma unroll
+                for (int k = 0; k < kRmiHidden; k += 4) {
+                    const ulonglong2 w = load4(&sm.P[kOffW2 + (j + u) * kRmiHidden + k]);
+                    dh[0][k / 2] = fma2(w.x, d0, dh[0][k / 2]);
+                    dh[0][k / 2 + 1] = fma2(w.y, d0, dh[0][k / 2 + 1]);
+                    dh[1][k / 2] = fma2(w.x, d1, dh[1][k / 2]);
+                    dh[1][k / 2 + 1] = fma2(w.y, d1, dh[1][k / 2 + 1]);
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                *reinterpret_cast<float2*>(&sm.d2[row0 + q][j]) = make_float2(d[q][0], d[q][1]);
+                *reinterpret_cast<float2*>(&sm.h2[row0 + q][j]) = make_float2(g2[q][0], g2[q][1]);
+            }
+        }
+        // this lane's sample: its own half of the sums plus the other lane's
+#pragma unroll
+        for (int k = 0; k < kRmiHidden / 2; k += 2) {
+            float v[4];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const float2 keep = unpack2(half ? dh[1][k + u] : dh[0][k + u]);
+                const float2 send = unpack2(half ? dh[0][k + u] : dh[1][k + u]);
+                const float2 h = unpack2(half ? h1[1][k + u] : h1[0][k + u]);
+                const float gx = keep.x + __shfl_xor_sync(0xffffffffu, send.x, 1);
+                const float gz = keep.y + __shfl_xor_sync(0xffffffffu, send.y, 1);
+                v[2 * u] = h.x > 0.f ? gx : 0.f;
+                v[2 * u + 1] = h.y > 0.f ? gz : 0.f;
+            }
+            *reinterpret_cast<float4*>(&sm.d1[tid][2 * k]) = make_float4(v[0], v[1], v[2], v[3]);
+        }
+        __syncwarp();
+        // the warp's 32 samples: W2 gradient, rows 4 jr.. x columns 8 kc..
+        {
+            const int jr = 4 * (lane >> 2), kc = 8 * (lane & 3);
+            f32x2 g[4][4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+#pragma unroll
+                for (int v = 0; v < 4; ++v) g[u][v] = 0ull;
+            float gw1 = 0.f, gb1 = 0.f, gb2 = 0.f, gw3 = 0.f, gb3 = 0.f, l2 = 0.f;
+#pragma unroll 4
+            for (int q = 0; q < 32; ++q) {
+                const int r = warp * 32 + q;
+                const float4 d = *reinterpret_cast<const float4*>(&sm.d2[r][jr]);
+                const ulonglong2 ha = load4(&sm.h1[r][kc]), hb = load4(&sm.h1[r][kc + 4]);
+                const float du[4] = {d.x, d.y, d.z, d.w};
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const f32x2 dd = pack2(du[u], du[u]);
+                    g[u][0] = fma2(ha.x, dd, g[u][0]);
+                    g[u][1] = fma2(ha.y, dd, g[u][1]);
+                    g[u][2] = fma2(hb.x, dd, g[u][2]);
+                    g[u][3] = fma2(hb.y, dd, g[u][3]);
+                }
+                const float d1 = sm.d1[r][lane];
+                gw1 = fmaf(d1, sm.x[r], gw1);
+                gb1 += d1;
+                gb2 += sm.d2[r][lane];
+                gw3 += sm.h2[r][lane];
+                gb3 += sm.gy[r];
+                l2 += sm.sq[r];
+            }
+            float* part = sm.part[warp];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+#pragma unroll
+                for (int v = 0; v < 4; ++v) {
+                    const float2 w = unpack2(g[u][v]);
+                    part[kOffW2 + (jr + u) * kRmiHidden + kc + 2 * v] = w.x;
+                    part[kOffW2 + (jr + u) * kRmiHidden + kc + 2 * v + 1] = w.y;
+                }
+            part[kOffW1 + lane] = gw1;
+            part[kOffB1 + lane] = gb1;
+            part[kOffB2 + lane] = gb2;
+            part[kOffW3 + lane] = gw3;
+            if (lane == 0) {
+                part[kOffB3] = gb3;
+                part[kLossWord] = l2;
+            }
+        }
+        __syncthreads();
+        for (int i = 4 * tid; i <= kLossWord; i += 4 * kTrainThreads) {
+            float v[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                v[u] = 0.f;
+                if (i + u <= kLossWord) {
+#pragma unroll
+                    for (int w = 0; w < kTrainWarps; ++w) v[u] += sm.part[w][i + u];
+                }
+            }
+            asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(grad + i), "f"(v[0]),
+                         "f"(v[1]), "f"(v[2]), "f"(v[3])
+                         : "memory");
+        }
+        // the buffer of the step before last is read by no block any more: zero it for the step after this one
+        float* next = a.grad + ((step + 1) % 3) * kGradWords;
+        for (int i = blockIdx.x * kTrainThreads + tid; i < kGradWords; i += gridDim.x * kTrainThreads) next[i] = 0.f;
+        __threadfence();
+        __syncthreads();
+        if (tid == 0) {
+            atomicAdd(a.arrived, 1u);
+            const unsigned want = gridDim.x * (unsigned)step;
+            int polls = 0;
+            unsigned got;
+            do {
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(got) : "l"(a.arrived) : "memory");
+            } while (got < want && ++polls < kTrainWaitLimit);
+            if (got < want) {
+                atomicOr(a.err, 2ull);
+                sm.fail = 1;
+            }
+        }
+        __syncthreads();
+        if (sm.fail) return;
+        // Adam, the same in every block
+        const float lr = 2e-3f * (step < a.steps / 2 ? 1.0f : 0.3f);
+        const float b1 = 0.9f, b2 = 0.999f;
+        const float c1 = 1.f - powf(b1, (float)step), c2 = 1.f - powf(b2, (float)step);
+        constexpr int kOwn = (kRmiP + kTrainThreads - 1) / kTrainThreads;
+        float g[kOwn];  // the loads' latencies overlap
+#pragma unroll
+        for (int u = 0; u < kOwn; ++u) {
+            const int i = tid + u * kTrainThreads;
+            g[u] = i < kRmiP ? __ldcg(grad + i) : 0.f;
+        }
+#pragma unroll
+        for (int u = 0; u < kOwn; ++u) {
+            const int i = tid + u * kTrainThreads;
+            if (i >= kRmiP) break;
+            const float m = b1 * sm.m1[i] + (1.f - b1) * g[u];
+            const float v = b2 * sm.m2[i] + (1.f - b2) * g[u] * g[u];
+            sm.m1[i] = m;
+            sm.m2[i] = v;
+            sm.P[i] -= lr * (m / c1) / (sqrtf(v / c2) + 1e-8f);
+        }
+        if (blockIdx.x == 0 && tid == 0 && step == a.steps) *a.loss = __ldcg(grad + kLossWord);
+        __syncthreads();
     }
-    if (threadIdx.x == 0) {
-        m->b3 = P[kOffB3];
+    if (blockIdx.x != 0) return;
+    RmiModel* m = a.model;
+    for (int i = tid; i < kRmiHidden * kRmiHidden; i += kTrainThreads) m->w2[i] = sm.P[kOffW2 + i];
+    if (tid < kRmiHidden) {
+        m->w1[tid] = sm.P[kOffW1 + tid];
+        m->b1[tid] = sm.P[kOffB1 + tid];
+        m->b2[tid] = sm.P[kOffB2 + tid];
+        m->w3[tid] = sm.P[kOffW3 + tid];
+    }
+    if (tid == 0) {
+        m->b3 = sm.P[kOffB3];
         m->key_lo = key_lo;
         m->key_scale = key_scale;
-        m->n_leaves = n_leaves;
-        m->n_keys = n_keys;
+        m->n_leaves = a.n_leaves;
+        m->n_keys = (int)a.n;
     }
 }
 
-// Tabulate the trained root over every ancestor key (one warp per key).
+// Tabulate the trained root over every ancestor key, a thread a key (the
+// weights are broadcast reads of shared memory; a warp a key, with the hidden
+// layer by shuffles, took 180 us for the 2^20 keys of level 10).
 __global__ void __launch_bounds__(kThreads) rmi_table_kernel(const RmiModel* __restrict__ model, int64_t n_anc,
                                                              uint16_t* __restrict__ table) {
     __shared__ RmiShared sm;
     rmi_load_shared(&sm, model);
     __syncthreads();
-    const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t c = warp; c < n_anc; c += nw) {
-        const float y = rmi_root_warp(&sm, rmi_input((uint32_t)c, &sm));
-        if ((threadIdx.x & 31) == 0) table[c] = (uint16_t)rmi_leaf(sm.n_leaves, y);
-    }
+    for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < n_anc; c += (int64_t)gridDim.x * blockDim.x)
+        table[c] = (uint16_t)rmi_leaf(sm.n_leaves, rmi_root(&sm, rmi_input((uint32_t)c, &sm)));
 }
 
 __global__ void rmi_route_kernel(const uint16_t* __restrict__ table, const uint32_t* __restrict__ keys, int64_t n,
@@ -639,67 +883,38 @@ int train_rmi(vs_context* ctx, vs_index* idx, int steps) {
     cudaStream_t s = ctx->stream;
     const int64_t n = li.n_cells;
     const int anc_shift = 2 * (li.level - li.root_level);
-    // ancestor-key range and quantile knots (33 keys read back)
-    std::vector<uint32_t> q(33);
-    for (int j = 0; j <= 32; ++j) {
-        const int64_t pos = (int64_t)((double)j * (double)(n - 1) / 32.0);
-        VS_CUDA_TRY(cudaMemcpyAsync(&q[j], li.cell_keys + pos, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-    }
-    VS_CUDA_TRY(cudaStreamSynchronize(s));
-    for (auto& v : q) v >>= anc_shift;
-    const double key_lo = (double)q[0];
-    const double span = (double)q[32] - key_lo;
-    const double key_scale = span > 0 ? 1.0 / span : 0.0;
-    // Initial root: a piecewise-linear interpolant of the key CDF through the
-    // 33 quantile knots (h1_j = relu(x - c_j), W2 = I, w3_j = slope change).
-    std::vector<float> P(kRmiP, 0.f);
-    std::vector<double> c(33), yk(33);
-    for (int j = 0; j <= 32; ++j) {
-        c[j] = ((double)q[j] - key_lo) * key_scale;
-        yk[j] = (double)j / 32.0;
-    }
-    double prev_slope = 0.0;
-    for (int j = 0; j < 32; ++j) {
-        const double dx = c[j + 1] - c[j];
-        const double slope = dx > 1e-12 ? (yk[j + 1] - yk[j]) / dx : 0.0;
-        P[kOffW1 + j] = 1.0f;
-        P[kOffB1 + j] = (float)-c[j];
-        P[kOffW3 + j] = (float)(slope - prev_slope);
-        prev_slope = slope;
-        P[kOffW2 + j * kRmiHidden + j] = 1.0f;
-        P[kOffB2 + j] = 0.0f;
-    }
-    P[kOffB3] = 0.0f;
-    const int S = (int)std::min<int64_t>(n, 16384);
-    Scratch<float> dP, m1, m2, xs, ts, part, loss;
-    VS_TRY(dP.alloc(kRmiP, s));
-    VS_TRY(m1.alloc(kRmiP, s));
-    VS_TRY(m2.alloc(kRmiP, s));
-    VS_TRY(xs.alloc(S, s));
-    VS_TRY(ts.alloc(S, s));
-    VS_TRY(part.alloc((size_t)kTrainBlocks * kRmiP, s));
-    VS_TRY(loss.alloc(1, s));
-    VS_CUDA_TRY(cudaMemcpyAsync(dP.p, P.data(), kRmiP * sizeof(float), cudaMemcpyHostToDevice, s));
-    VS_CUDA_TRY(cudaMemsetAsync(m1.p, 0, kRmiP * sizeof(float), s));
-    VS_CUDA_TRY(cudaMemsetAsync(m2.p, 0, kRmiP * sizeof(float), s));
-    rmi_samples_kernel<<<div_up(S, 256), 256, 0, s>>>(li.cell_keys, n, S, anc_shift, key_lo, key_scale, xs.p, ts.p);
-    VS_CUDA_TRY(cudaGetLastError());
-    for (int step = 1; step <= steps; ++step) {
-        VS_CUDA_TRY(cudaMemsetAsync(loss.p, 0, sizeof(float), s));
-        rmi_grad_kernel<<<kTrainBlocks, kThreads, 0, s>>>(dP.p, xs.p, ts.p, S, part.p, loss.p);
-        const float lr = 2e-3f * (step < steps / 2 ? 1.0f : 0.3f);
-        rmi_adam_kernel<<<div_up(kRmiP, 256), 256, 0, s>>>(dP.p, m1.p, m2.p, part.p, kTrainBlocks, step, lr);
-    }
-    VS_CUDA_TRY(cudaGetLastError());
-    VS_CUDA_TRY(cudaMemcpyAsync(&li.rmi_final_loss, loss.p, sizeof(float), cudaMemcpyDeviceToHost, s));
     int64_t& bytes = idx->device_bytes;
     if (!li.model) VS_TRY(dalloc(&li.model, 1, bytes));
-    rmi_pack_kernel<<<1, 256, 0, s>>>(dP.p, li.model, key_lo, key_scale, li.n_leaves, (int)n);
-    VS_CUDA_TRY(cudaGetLastError());
+    Scratch<float> grad;
+    Scratch<unsigned> arrived;
+    VS_TRY(grad.alloc(3 * kGradWords + 1, s));
+    VS_TRY(arrived.alloc(1, s));
+    VS_CUDA_TRY(cudaMemsetAsync(grad.p, 0, (3 * kGradWords + 1) * sizeof(float), s));
+    VS_CUDA_TRY(cudaMemsetAsync(arrived.p, 0, sizeof(unsigned), s));
+    TrainArgs ta{};
+    ta.keys = li.cell_keys;
+    ta.n = n;
+    ta.S = (int)std::min<int64_t>(n, kTrainSamples);
+    ta.anc_shift = anc_shift;
+    ta.steps = steps;
+    ta.n_leaves = li.n_leaves;
+    ta.grad = grad.p;
+    ta.arrived = arrived.p;
+    ta.loss = grad.p + 3 * kGradWords;
+    ta.model = li.model;
+    ta.err = &ctx->d_counters[kSortErr];
+    // The blocks meet at a barrier every step: a cooperative launch, so all of them run at once.
+    VS_CUDA_TRY(cudaFuncSetAttribute(rmi_train_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)sizeof(TrainShared)));
+    void* args[] = {(void*)&ta};
+    VS_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)rmi_train_kernel, dim3(div_up(ta.S, kTrainThreads)),
+                                            dim3(kTrainThreads), args, sizeof(TrainShared), s));
+    VS_LAUNCHED("rmi_train", s);
+    VS_CUDA_TRY(cudaMemcpyAsync(&li.rmi_final_loss, ta.loss, sizeof(float), cudaMemcpyDeviceToHost, s));
     // tabulate the root over all 4^R ancestor keys
     const int64_t n_anc = 1ll << (2 * li.root_level);
     VS_TRY(dalloc(&li.root_table, (size_t)n_anc, bytes));
-    rmi_table_kernel<<<grid_for(n_anc * 32, kThreads, 8), kThreads, 0, s>>>(li.model, n_anc, li.root_table);
+    rmi_table_kernel<<<grid_for(n_anc, kThreads, 4), kThreads, 0, s>>>(li.model, n_anc, li.root_table);
     VS_CUDA_TRY(cudaGetLastError());
     return VS_OK;
 }

@@ -1,9 +1,8 @@
 // Recursive model index (RMI) evaluation.
 //
 // The root MLP (FP32, 1 -> 32 -> 32 -> 1) maps a normalised ancestor-cell key
-// to [0, 1); leaf = floor(y * n_leaves).  It is evaluated by a full warp for
-// one input (lane j owns hidden unit j) when the root table is built; queries
-// only read the table.  Leaf models predict a position from the full cell key
+// to [0, 1); leaf = floor(y * n_leaves).  It is evaluated when the root table
+// is built; queries only read the table.  Leaf models predict a position from the full cell key
 // in FP64.
 #pragma once
 #include <cuda_runtime.h>
@@ -13,11 +12,10 @@
 
 namespace vs {
 
-// Shared-memory copy of the root MLP with W2 transposed (w2t[k*32 + j] =
-// W2[j][k]) so that lane j reading column k is bank-conflict free.
+// Shared-memory copy of the root MLP.
 struct RmiShared {
     float w1[kRmiHidden], b1[kRmiHidden];
-    float w2t[kRmiHidden * kRmiHidden];
+    __align__(16) float w2[kRmiHidden * kRmiHidden];
     float b2[kRmiHidden], w3[kRmiHidden];
     float b3;
     double key_lo, key_scale;
@@ -25,10 +23,7 @@ struct RmiShared {
 };
 
 __device__ __forceinline__ void rmi_load_shared(RmiShared* s, const RmiModel* m) {
-    for (int i = threadIdx.x; i < kRmiHidden * kRmiHidden; i += blockDim.x) {
-        const int j = i / kRmiHidden, k = i % kRmiHidden;
-        s->w2t[k * kRmiHidden + j] = m->w2[i];
-    }
+    for (int i = threadIdx.x; i < kRmiHidden * kRmiHidden; i += blockDim.x) s->w2[i] = m->w2[i];
     for (int i = threadIdx.x; i < kRmiHidden; i += blockDim.x) {
         s->w1[i] = m->w1[i];
         s->b1[i] = m->b1[i];
@@ -48,18 +43,27 @@ __device__ __forceinline__ float rmi_input(uint32_t anc, const RmiShared* s) {
     return __double2float_rn(__dmul_rn((double)anc - s->key_lo, s->key_scale));
 }
 
-// Root MLP for ONE input, evaluated by the whole warp (lane j = hidden unit
-// j); the xor-butterfly sum leaves the same bits in every lane.
-__device__ __forceinline__ float rmi_root_warp(const RmiShared* s, float x) {
-    const int j = threadIdx.x & 31;
-    const float h1 = fmaxf(__fmaf_rn(s->w1[j], x, s->b1[j]), 0.0f);
-    float z2 = s->b2[j];
+// Root MLP for one input, by one thread.
+__device__ __forceinline__ float rmi_root(const RmiShared* s, float x) {
+    float h1[kRmiHidden];
 #pragma unroll
-    for (int k = 0; k < kRmiHidden; ++k) z2 = __fmaf_rn(s->w2t[k * kRmiHidden + j], __shfl_sync(0xffffffffu, h1, k), z2);
-    float t = __fmul_rn(s->w3[j], fmaxf(z2, 0.0f));
+    for (int k = 0; k < kRmiHidden; ++k) h1[k] = fmaxf(__fmaf_rn(s->w1[k], x, s->b1[k]), 0.0f);
+    float y = s->b3;
+#pragma unroll 4
+    for (int j = 0; j < kRmiHidden; ++j) {
+        float z = s->b2[j];
+        const float4* row = reinterpret_cast<const float4*>(&s->w2[j * kRmiHidden]);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) t = __fadd_rn(t, __shfl_xor_sync(0xffffffffu, t, o));
-    return __fadd_rn(t, s->b3);
+        for (int k = 0; k < kRmiHidden / 4; ++k) {
+            const float4 w = row[k];
+            z = __fmaf_rn(w.x, h1[4 * k], z);
+            z = __fmaf_rn(w.y, h1[4 * k + 1], z);
+            z = __fmaf_rn(w.z, h1[4 * k + 2], z);
+            z = __fmaf_rn(w.w, h1[4 * k + 3], z);
+        }
+        y = __fmaf_rn(s->w3[j], fmaxf(z, 0.0f), y);
+    }
+    return y;
 }
 
 __device__ __forceinline__ int rmi_leaf(int n_leaves, float y) {
