@@ -137,6 +137,20 @@ int vs_context_create(int device, void* stream, vs_context** out) {
         uint64_t thr = ~0ull;
         cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &thr);
     }
+    // Index memory has a pool of its own (sharing the scratch's fragmented it:
+    // the large scratch blocks were then mapped anew on every call); what it
+    // keeps unused is bounded.
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    if (cudaMemPoolCreate(&ctx->index_pool, &props) == cudaSuccess) {
+        uint64_t keep = kIndexPoolKeep;
+        cudaMemPoolSetAttribute(ctx->index_pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    } else {
+        ctx->index_pool = nullptr;  // index memory then comes from the default pool
+        cudaGetLastError();
+    }
     bool ok = cudaMallocHost((void**)&ctx->h_counter, kHostCounters * sizeof(unsigned long long)) == cudaSuccess &&
               cudaMalloc((void**)&ctx->d_counters, kDevCounters * sizeof(unsigned long long)) == cudaSuccess;
     for (int k = 0; k < 5 && ok; ++k) ok = cudaEventCreate(&ctx->phase_ev[k]) == cudaSuccess;
@@ -147,6 +161,7 @@ int vs_context_create(int device, void* stream, vs_context** out) {
             if (ctx->phase_ev[k]) cudaEventDestroy(ctx->phase_ev[k]);
         if (ctx->d_counters) cudaFree(ctx->d_counters);
         if (ctx->h_counter) cudaFreeHost(ctx->h_counter);
+        if (ctx->index_pool) cudaMemPoolDestroy(ctx->index_pool);
         if (ctx->owns_stream) cudaStreamDestroy(ctx->stream);
         delete ctx;
         return VS_E_OOM;
@@ -164,6 +179,8 @@ int vs_context_destroy(vs_context* ctx) {
     cudaFree(ctx->defer_buf);
     cudaFreeHost(ctx->h_counter);
     for (int k = 0; k < 5; ++k) cudaEventDestroy(ctx->phase_ev[k]);
+    // indexes that outlive the context keep their memory: the pool goes with the last of them
+    if (ctx->index_pool) cudaMemPoolDestroy(ctx->index_pool);
     if (ctx->owns_stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
     return VS_OK;

@@ -202,20 +202,6 @@ __global__ void level_kernel(const vs_box* __restrict__ child, int64_t nchild, v
     }
 }
 
-template <class T>
-int dalloc(T** p, size_t n, int64_t& bytes) {
-    if (n == 0) n = 1;
-    cudaError_t e = cudaMalloc((void**)p, n * sizeof(T));
-    if (e != cudaSuccess) {
-        *p = nullptr;
-        set_error("cudaMalloc(%zu bytes) failed: %s", n * sizeof(T), cudaGetErrorString(e));
-        return e == cudaErrorMemoryAllocation ? VS_E_OOM : VS_E_CUDA;
-    }
-    bytes += (int64_t)(n * sizeof(T));
-    return VS_OK;
-}
-
-
 // ------------------------------------------------------------ ring bins ---
 // Pass 1, one thread per ring: is it binned (enough vertices, finite y,
 // positive height), its (y0, scale), and how many (bin, edge) entries it
@@ -318,16 +304,16 @@ int hilbert_point_keys(const double* x, const double* y, int64_t n, double minx,
 }
 
 void free_index_memory(vs_index* idx) {
-    cudaFree(idx->nodes);
-    cudaFree(idx->item_geom);
-    cudaFree(idx->geom_off);
-    cudaFree(idx->part_off);
-    cudaFree(idx->ring_off);
-    cudaFree(idx->xy);
-    cudaFree(idx->frame);
-    cudaFree(idx->ring_bin);
-    cudaFree(idx->ring_bins);
-    cudaFree(idx->bin_edges);
+    index_free(idx->nodes);
+    index_free(idx->item_geom);
+    index_free(idx->geom_off);
+    index_free(idx->part_off);
+    index_free(idx->ring_off);
+    index_free(idx->xy);
+    index_free(idx->frame);
+    index_free(idx->ring_bin);
+    index_free(idx->ring_bins);
+    index_free(idx->bin_edges);
     free_learned_index(idx);
 }
 
@@ -356,13 +342,13 @@ int build_rtree(vs_context* ctx, const vs_polygons* P, vs_index* idx) {
     }
     idx->levels = L;
     int64_t& bytes = idx->device_bytes;
-    VS_TRY(dalloc(&idx->nodes, (size_t)off, bytes));
-    VS_TRY(dalloc(&idx->item_geom, (size_t)M, bytes));
-    VS_TRY(dalloc(&idx->geom_off, (size_t)M + 1, bytes));
-    VS_TRY(dalloc(&idx->part_off, (size_t)P->n_parts + 1, bytes));
-    VS_TRY(dalloc(&idx->ring_off, (size_t)P->n_rings + 1, bytes));
-    VS_TRY(dalloc(&idx->xy, (size_t)P->n_coords, bytes));
-    VS_TRY(dalloc(&idx->frame, 4, bytes));
+    VS_TRY(dalloc(&idx->nodes, (size_t)off, bytes, ctx));
+    VS_TRY(dalloc(&idx->item_geom, (size_t)M, bytes, ctx));
+    VS_TRY(dalloc(&idx->geom_off, (size_t)M + 1, bytes, ctx));
+    VS_TRY(dalloc(&idx->part_off, (size_t)P->n_parts + 1, bytes, ctx));
+    VS_TRY(dalloc(&idx->ring_off, (size_t)P->n_rings + 1, bytes, ctx));
+    VS_TRY(dalloc(&idx->xy, (size_t)P->n_coords, bytes, ctx));
+    VS_TRY(dalloc(&idx->frame, 4, bytes, ctx));
 
     Scratch<vs_box> box;
     Scratch<uint32_t> np, nr, nc, sp, sr, sc, vals, totals;
@@ -456,9 +442,9 @@ int build_ring_bins(vs_context* ctx, vs_index* idx, int min_vertices) {
     VS_CUDA_TRY(cudaStreamSynchronize(s));
     if (tot[1] == 0) return VS_OK;  // no ring qualifies
     int64_t& bytes = idx->device_bytes;
-    VS_TRY(dalloc(&idx->ring_bin, (size_t)R, bytes));
-    VS_TRY(dalloc(&idx->ring_bins, (size_t)tot[1], bytes));
-    VS_TRY(dalloc(&idx->bin_edges, (size_t)tot[0], bytes));
+    VS_TRY(dalloc(&idx->ring_bin, (size_t)R, bytes, ctx));
+    VS_TRY(dalloc(&idx->ring_bins, (size_t)tot[1], bytes, ctx));
+    VS_TRY(dalloc(&idx->bin_edges, (size_t)tot[0], bytes, ctx));
     ring_bin_fill_kernel<<<grid_for(R, 256), 256, 0, s>>>(R, idx->ring_off, idx->xy, entry_off.p, bin_idx.p, binned.p,
                                                           yinfo.p, idx->ring_bin, idx->ring_bins, idx->bin_edges);
     VS_CUDA_TRY(cudaGetLastError());

@@ -832,19 +832,6 @@ __global__ void learned_desc_kernel(const double* __restrict__ fr, LearnedJob* _
     d->cwy = units / sy;
 }
 
-template <class T>
-int dalloc(T** p, size_t n, int64_t& bytes) {
-    if (n == 0) n = 1;
-    cudaError_t e = cudaMalloc((void**)p, n * sizeof(T));
-    if (e != cudaSuccess) {
-        *p = nullptr;
-        set_error("cudaMalloc(%zu bytes) failed: %s", n * sizeof(T), cudaGetErrorString(e));
-        return e == cudaErrorMemoryAllocation ? VS_E_OOM : VS_E_CUDA;
-    }
-    bytes += (int64_t)(n * sizeof(T));
-    return VS_OK;
-}
-
 // Registrations (E), distinct cells (n_cells) and the sum over cells of
 // their squared entry counts (sum_sq) of the slot boxes at grid level L, on
 // scratch only: the count, emit, sort and unique-flag steps of the build.
@@ -884,7 +871,7 @@ int train_rmi(vs_context* ctx, vs_index* idx, int steps) {
     const int64_t n = li.n_cells;
     const int anc_shift = 2 * (li.level - li.root_level);
     int64_t& bytes = idx->device_bytes;
-    if (!li.model) VS_TRY(dalloc(&li.model, 1, bytes));
+    if (!li.model) VS_TRY(dalloc(&li.model, 1, bytes, ctx));
     Scratch<float> grad;
     Scratch<unsigned> arrived;
     VS_TRY(grad.alloc(3 * kGradWords + 1, s));
@@ -913,7 +900,7 @@ int train_rmi(vs_context* ctx, vs_index* idx, int steps) {
     VS_CUDA_TRY(cudaMemcpyAsync(&li.rmi_final_loss, ta.loss, sizeof(float), cudaMemcpyDeviceToHost, s));
     // tabulate the root over all 4^R ancestor keys
     const int64_t n_anc = 1ll << (2 * li.root_level);
-    VS_TRY(dalloc(&li.root_table, (size_t)n_anc, bytes));
+    VS_TRY(dalloc(&li.root_table, (size_t)n_anc, bytes, ctx));
     rmi_table_kernel<<<grid_for(n_anc, kThreads, 4), kThreads, 0, s>>>(li.model, n_anc, li.root_table);
     VS_CUDA_TRY(cudaGetLastError());
     return VS_OK;
@@ -926,8 +913,8 @@ int fit_leaves(vs_context* ctx, vs_index* idx) {
     const int nl = li.n_leaves;
     const int anc_shift = 2 * (li.level - li.root_level);
     int64_t& bytes = idx->device_bytes;
-    VS_TRY(dalloc(&li.leaf_ab, (size_t)nl, bytes));
-    VS_TRY(dalloc(&li.leaf_err, (size_t)nl, bytes));
+    VS_TRY(dalloc(&li.leaf_ab, (size_t)nl, bytes, ctx));
+    VS_TRY(dalloc(&li.leaf_err, (size_t)nl, bytes, ctx));
     Scratch<uint32_t> leaf_of;
     Scratch<double> sums, cov;
     Scratch<unsigned long long> acc;
@@ -944,7 +931,7 @@ int fit_leaves(vs_context* ctx, vs_index* idx) {
     rmi_leaf_fit_kernel<<<div_up(nl, 256), 256, 0, s>>>(sums.p, cov.p, nl, li.leaf_ab, li.leaf_err);
     rmi_err_kernel<<<grid_for(n, 256), 256, 0, s>>>(li.cell_keys, leaf_of.p, n, li.leaf_ab, li.leaf_err);
     rmi_window_stats_kernel<<<grid_for(n, 256), 256, 0, s>>>(leaf_of.p, n, li.leaf_err, acc.p);
-    VS_TRY(dalloc(&li.leaves, (size_t)nl, bytes));
+    VS_TRY(dalloc(&li.leaves, (size_t)nl, bytes, ctx));
     pack_leaves_kernel<<<div_up(nl, 256), 256, 0, s>>>(nl, li.leaf_ab, li.leaf_err, li.leaves);
     VS_CUDA_TRY(cudaGetLastError());
     unsigned long long h[2];
@@ -959,23 +946,23 @@ int fit_leaves(vs_context* ctx, vs_index* idx) {
 
 void free_learned_index(vs_index* idx) {
     LearnedIndex& li = idx->learned;
-    cudaFree(li.cell_keys);
-    cudaFree(li.cell_start);
-    cudaFree(li.entries);
-    cudaFree(li.occ);
-    cudaFree(li.model);
-    cudaFree(li.root_table);
-    cudaFree(li.leaf_ab);
-    cudaFree(li.leaf_err);
-    cudaFree(li.origin);
-    cudaFree(li.err32);
-    cudaFree(li.c01);
-    cudaFree(li.ring_box32);
-    cudaFree(li.ib32);
-    cudaFree(li.xy32);
-    cudaFree(li.leaves);
-    cudaFree(li.recs);
-    cudaFree(li.desc);
+    index_free(li.cell_keys);
+    index_free(li.cell_start);
+    index_free(li.entries);
+    index_free(li.occ);
+    index_free(li.model);
+    index_free(li.root_table);
+    index_free(li.leaf_ab);
+    index_free(li.leaf_err);
+    index_free(li.origin);
+    index_free(li.err32);
+    index_free(li.c01);
+    index_free(li.ring_box32);
+    index_free(li.ib32);
+    index_free(li.xy32);
+    index_free(li.leaves);
+    index_free(li.recs);
+    index_free(li.desc);
     li = LearnedIndex{};
 }
 
@@ -1063,7 +1050,7 @@ int build_learned_index(vs_context* ctx, vs_index* idx, const vs_index_options* 
     VS_TRY(off.alloc((size_t)M, s));
     VS_TRY(keys.alloc((size_t)E, s));
     VS_TRY(flag.alloc((size_t)E, s));
-    VS_TRY(dalloc(&li.entries, (size_t)E, bytes));
+    VS_TRY(dalloc(&li.entries, (size_t)E, bytes, ctx));
     VS_TRY(exclusive_scan_u32(cnt.p, off.p, M, nullptr, s));
     cell_emit_kernel<<<grid_for(M, 256), 256, 0, s>>>(boxes, M, idx->frame, L, off.p, keys.p, li.entries);
     VS_CUDA_TRY(cudaGetLastError());
@@ -1077,8 +1064,8 @@ int build_learned_index(vs_context* ctx, vs_index* idx, const vs_index_options* 
     VS_CUDA_TRY(cudaMemcpyAsync(&nc, ncell.p, sizeof(nc), cudaMemcpyDeviceToHost, s));
     VS_CUDA_TRY(cudaStreamSynchronize(s));
     li.n_cells = nc;
-    VS_TRY(dalloc(&li.cell_keys, (size_t)nc, bytes));
-    VS_TRY(dalloc(&li.cell_start, (size_t)nc + 1, bytes));
+    VS_TRY(dalloc(&li.cell_keys, (size_t)nc, bytes, ctx));
+    VS_TRY(dalloc(&li.cell_start, (size_t)nc + 1, bytes, ctx));
     cell_compact_kernel<<<grid_for(E, 256), 256, 0, s>>>(keys.p, flag.p, (int64_t)E, li.cell_keys, li.cell_start);
     const uint32_t Eu = (uint32_t)E;
     VS_CUDA_TRY(cudaMemcpyAsync(li.cell_start + nc, &Eu, sizeof(Eu), cudaMemcpyHostToDevice, s));
@@ -1088,7 +1075,7 @@ int build_learned_index(vs_context* ctx, vs_index* idx, const vs_index_options* 
 #endif
     li.occ_level = std::min(L, VS_OCC_MAX_LEVEL);
     const int64_t occ_bits = 1ll << (2 * li.occ_level);
-    VS_TRY(dalloc(&li.occ, (size_t)((occ_bits + 31) / 32), bytes));
+    VS_TRY(dalloc(&li.occ, (size_t)((occ_bits + 31) / 32), bytes, ctx));
     VS_CUDA_TRY(cudaMemsetAsync(li.occ, 0, (size_t)((occ_bits + 31) / 32) * sizeof(uint32_t), s));
     occ_kernel<<<grid_for(nc, 256), 256, 0, s>>>(li.cell_keys, nc, 2 * (L - li.occ_level), li.occ);
     VS_CUDA_TRY(cudaGetLastError());
@@ -1132,14 +1119,14 @@ int build_learned_index(vs_context* ctx, vs_index* idx, const vs_index_options* 
     d.boxes = idx->nodes;
     d.rings = idx->ring_index();
     // 7. FP32 slot-relative vertices, per-slot ring ranges, per-entry records
-    VS_TRY(dalloc(&li.origin, (size_t)M, bytes));
-    VS_TRY(dalloc(&li.err32, (size_t)M, bytes));
-    VS_TRY(dalloc(&li.c01, (size_t)M, bytes));
-    VS_TRY(dalloc(&li.ring_box32, (size_t)std::max<int32_t>(idx->n_rings, 1), bytes));
-    VS_TRY(dalloc(&li.ib32, (size_t)M, bytes));
-    VS_TRY(dalloc(&li.xy32, (size_t)std::max<int64_t>(idx->n_coords, 1), bytes));
-    VS_TRY(dalloc(&li.recs, (size_t)E, bytes));
-    VS_TRY(dalloc(&li.desc, 1, bytes));
+    VS_TRY(dalloc(&li.origin, (size_t)M, bytes, ctx));
+    VS_TRY(dalloc(&li.err32, (size_t)M, bytes, ctx));
+    VS_TRY(dalloc(&li.c01, (size_t)M, bytes, ctx));
+    VS_TRY(dalloc(&li.ring_box32, (size_t)std::max<int32_t>(idx->n_rings, 1), bytes, ctx));
+    VS_TRY(dalloc(&li.ib32, (size_t)M, bytes, ctx));
+    VS_TRY(dalloc(&li.xy32, (size_t)std::max<int64_t>(idx->n_coords, 1), bytes, ctx));
+    VS_TRY(dalloc(&li.recs, (size_t)E, bytes, ctx));
+    VS_TRY(dalloc(&li.desc, 1, bytes, ctx));
     d.recs = li.recs;
     d.c01 = li.c01;
     d.ring_box32 = li.ring_box32;

@@ -21,6 +21,7 @@ int check_polygons(const vs_polygons* p);
 constexpr int kHostCounters = 16;
 constexpr int kDevCounters = 17;
 constexpr int kWorkCounter = 8;
+constexpr uint64_t kIndexPoolKeep = 1ull << 30;  // unused bytes the index pool keeps for the next build
 constexpr int kSortErr = 16;  // bit 1: a bounded wait of a pair sort gave up
 
 #define VS_CUDA_TRY(expr)                                                        \
@@ -150,6 +151,8 @@ struct vs_context {
     // around locate / group / refine / exact; recorded only while phase_on.
     cudaEvent_t phase_ev[5];
     bool phase_on;
+    // Pool of the indexes built with this context (null: the default pool).
+    cudaMemPool_t index_pool;
     // Streams and double buffers of vs_join_host, kept between calls.
     vs::HostPipe* host_pipe;
 };
