@@ -117,6 +117,109 @@ __device__ double facet_distance(double px, double py, const double2* __restrict
     return best;
 }
 
+// Bounds of the facet distance (the minimum segment distance over every ring)
+// of slot g from a point, in FP32 on the vertices relative to the point.
+// A relative vertex is off by at most 2^-24 of its size m, the segment
+// parameter by about 6 * 2^-24 |a| / |u|, and any parameter in [0, 1] names a
+// point of the segment, so the distance found is within 1e-6 m of the real
+// one; err doubles that and covers underflow.  The FP64 distances compared in
+// the end are within 1e-15 m of the real ones.  full: a vertex is NaN or too
+// far for FP32 squares, nothing is known (lo = 0, hi = INFINITY).
+// Vertices is const double2* or SoaVertices.
+struct FacetBounds {
+    float lo, hi, err;
+    bool full;
+};
+
+struct SoaVertices {
+    const double* x;
+    const double* y;
+    __device__ __forceinline__ double2 operator[](int c) const { return make_double2(x[c], y[c]); }
+};
+
+__device__ __forceinline__ float max_nan(float a, float b) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+
+__device__ __forceinline__ float2 relative(const double2 v, double px, double py) {
+    return make_float2(__double2float_rn(v.x - px), __double2float_rn(v.y - py));
+}
+
+// Squared distance from the origin to segment a -> b (NaN when a vertex is).
+__device__ __forceinline__ float segment_dist2(const float2 a, const float2 b) {
+    const float ux = b.x - a.x, uy = b.y - a.y;
+    const float t = __saturatef(__fdividef(-fmaf(a.x, ux, a.y * uy), fmaf(ux, ux, uy * uy)));  // 0 for a == b
+    const float ex = fmaf(t, ux, a.x), ey = fmaf(t, uy, a.y);
+    return fmaf(ex, ex, ey * ey);
+}
+
+template <class Vertices>
+__device__ __forceinline__ FacetBounds facet_bounds(double px, double py, const Vertices& xy,
+                                                    const int32_t* __restrict__ ring_off, int r0, int r1) {
+    float best = INFINITY, m = 0.f;
+    for (int ring = r0; ring < r1; ++ring) {
+        const int c0 = ring_off[ring], c1 = ring_off[ring + 1];
+        if (c1 - c0 < 2) {
+            if (c1 > c0) {  // no segment, but a NaN vertex still counts for `full`
+                const float2 v = relative(xy[c0], px, py);
+                m = max_nan(m, max_nan(fabsf(v.x), fabsf(v.y)));
+            }
+            continue;
+        }
+        float2 a = relative(xy[c0], px, py);
+        m = max_nan(m, max_nan(fabsf(a.x), fabsf(a.y)));
+        for (int c = c0 + 1; c < c1; ++c) {
+            const float2 b = relative(xy[c], px, py);
+            m = max_nan(m, max_nan(fabsf(b.x), fabsf(b.y)));
+            best = fminf(best, segment_dist2(a, b));
+            a = b;
+        }
+    }
+    FacetBounds f;
+    f.full = !(m <= 1e18f);
+    f.err = fmaf(m, 2e-6f, 1e-17f);
+    const float d = sqrtf(best);
+    f.lo = f.full ? 0.f : fmaxf(d - f.err, 0.f);
+    f.hi = f.full ? INFINITY : d + f.err;
+    return f;
+}
+
+// The exact facet distance, or a larger value when it is above hi: only the
+// segments that may be within hi (whose FP32 distance, off by at most err, is
+// within hi + err) are computed in FP64, up to 64 segments at a time so that
+// lanes whose segments lie at different places compute them together.
+template <class Vertices>
+__device__ __forceinline__ double facet_distance_bounded(double px, double py, const Vertices& xy,
+                                                         const int32_t* __restrict__ ring_off, int r0, int r1,
+                                                         float hi, float err) {
+    const float reach = hi + err;
+    const float reach2 = reach * reach * 1.000001f;
+    double best = INFINITY;
+    for (int ring = r0; ring < r1; ++ring) {
+        const int c0 = ring_off[ring], c1 = ring_off[ring + 1];
+        for (int first = c0; first + 1 < c1; first += 64) {
+            const int last = first + 64 < c1 - 1 ? first + 64 : c1 - 1;  // segments [first, last)
+            unsigned long long near = 0;
+            float2 a = relative(xy[first], px, py);
+            for (int c = first; c < last; ++c) {
+                const float2 b = relative(xy[c + 1], px, py);
+                if (segment_dist2(a, b) <= reach2) near |= 1ull << (c - first);
+                a = b;
+            }
+            while (near) {
+                const int c = first + __ffsll((long long)near) - 1;
+                near &= near - 1;
+                const double2 va = xy[c], vb = xy[c + 1];
+                const double d = point_segment_distance(px, py, va.x, va.y, vb.x, vb.y);
+                best = d < best ? d : best;
+            }
+        }
+    }
+    return best;
+}
+
 struct DistArgs {
     const double* px;
     const double* py;
@@ -179,6 +282,20 @@ __device__ __forceinline__ double descent_key(const vs_box& b, double x, double 
 __device__ __noinline__ double polygon_distance(const DistArgs& a, double x, double y, int g, unsigned& n_exact) {
     const int loc = geometry_location(x, y, a.xy, a.ring_off, a.part_off, a.geom_off, g, a.rings, n_exact);
     return loc != LOC_OUTSIDE ? 0.0 : facet_distance(x, y, a.xy, a.ring_off, a.part_off, a.geom_off, g, -1.0);
+}
+
+// The distance of a polygon on a nearest list, or something larger when it is
+// above ub: the location only where the point lies in the envelope, and in
+// FP64 only the segments within reach.  err < 0: no bounds are known.
+__device__ __noinline__ double listed_distance(const DistArgs& a, double x, double y, int g, float err, float ub,
+                                               unsigned& n_exact) {
+    if (err < 0.f) return polygon_distance(a, x, y, g, n_exact);
+    const vs_box b = a.nodes[a.level_off[0] + g];
+    if (x >= b.minx && x <= b.maxx && y >= b.miny && y <= b.maxy &&
+        geometry_location(x, y, a.xy, a.ring_off, a.part_off, a.geom_off, g, a.rings, n_exact) != LOC_OUTSIDE)
+        return 0.0;
+    return facet_distance_bounded(x, y, a.xy, a.ring_off, a.part_off[a.geom_off[g]], a.part_off[a.geom_off[g + 1]],
+                                  ub, err);
 }
 
 // Warp-packet R-tree walk of the distance joins.
@@ -444,6 +561,382 @@ __global__ void __launch_bounds__(kDistThreads) dist_join_kernel(const DistArgs 
     if (kMode != kNearestMin) wflush(out, a.sink, true);
     add_counter(a.counters, 5, n_cand);
     add_counter(a.counters, 1, n_exact + n_exact_q);
+}
+
+// ------------------------------------------------------- packet walks in FP32
+// Nearest and reverse nearest walk the tree with a packet of 32
+// Hilbert-consecutive queries a warp.  Coordinates are FP32 offsets from the
+// packet's centroid: node and item boxes rounded outward, a point widened by
+// its rounding (a query polygon is its envelope), so a box distance is never
+// overestimated.  A greedy descent to the leaf block nearest to the centroid
+// gives every lane a first bound.  Nodes then come off the stack nearest to
+// the centroid first; one is skipped when its centroid distance exceeds the
+// packet's radius plus the largest of the lanes' bounds.  The lanes test the
+// children within that reach against their own bounds: a child some lane
+// reaches is pushed, and in a leaf block each lane works through the items it
+// reaches itself, so lanes handle different items at the same time.
+constexpr int kNearList = 6;
+
+// A node box relative to (cx, cy), rounded outward: each FP64 difference is
+// within 2^-53 of itself of the real one, so it is widened by that first.
+__device__ __forceinline__ float4 relative_box(const vs_box& b, double cx, double cy) {
+    const double u = 1.2e-16;
+    const double x0 = b.minx - cx, y0 = b.miny - cy, x1 = b.maxx - cx, y1 = b.maxy - cy;
+    return make_float4(__double2float_rd(x0 - fabs(x0) * u), __double2float_rd(y0 - fabs(y0) * u),
+                       __double2float_ru(x1 + fabs(x1) * u), __double2float_ru(y1 + fabs(y1) * u));
+}
+
+// Lower bound of the distance from the centroid to a relative box.  Squares
+// past FP32 give a distance beyond every finite bound.
+__device__ __forceinline__ float centroid_low(const float4& b) {
+    const float dx = fmaxf(fmaxf(b.x, -b.z), 0.f), dy = fmaxf(fmaxf(b.y, -b.w), 0.f);
+    const float d = __fsqrt_rd(__fmaf_rd(dx, dx, __fmul_rd(dy, dy)));
+    return d < INFINITY ? d : 1e19f;
+}
+
+// Lower bound of the squared distance between two relative boxes.
+__device__ __forceinline__ float box_low2(const float4& a, const float4& b) {
+    const float dx = fmaxf(fmaxf(__fsub_rd(b.x, a.z), __fsub_rd(a.x, b.z)), 0.f);
+    const float dy = fmaxf(fmaxf(__fsub_rd(b.y, a.w), __fsub_rd(a.y, b.w)), 0.f);
+    return __fmaf_rd(dx, dx, __fmul_rd(dy, dy));
+}
+
+// Largest of non-negative floats over the warp (their bits order as unsigned).
+__device__ __forceinline__ float warp_max_nonneg(float v) {
+    return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v)));
+}
+
+// A lane of a packet: its query as a relative box, its bound, and whether it
+// takes part.
+struct PacketLane {
+    float4 q;
+    float ub;
+    bool walk;
+};
+
+// What a warp keeps in shared memory for a walk.
+struct PacketShared {
+    int2 stack[kDistStack];  // (node << 4 | level, centroid distance)
+    float4 items[kFanout];   // the node's children, relative
+};
+
+// One child box a lane of the block of node `node` at level cl + 1 (lane < 16,
+// relative; empty beyond the block and for empty boxes).
+template <class Tree>
+__device__ __forceinline__ float4 child_box(const Tree& a, const vs_box* s_nodes, int cl, int64_t c, bool in_range,
+                                            double cx, double cy) {
+    float4 rb = make_float4(INFINITY, INFINITY, -INFINITY, -INFINITY);
+    if (in_range) {
+        const vs_box b = cl >= a.stage_level ? s_nodes[a.level_off[cl] - a.level_off[a.stage_level] + c]
+                                             : a.nodes[a.level_off[cl] + c];
+        if (b.minx <= b.maxx) rb = relative_box(b, cx, cy);
+    }
+    return rb;
+}
+
+// Greedy descent to a leaf block: at every level the child nearest to the
+// centroid, ties to the nearer centre.  Leaves the block's items in sm.items;
+// returns its first slot, or -1 (nothing to descend to).  Whole warp.
+template <class Tree>
+__device__ __forceinline__ int packet_descend(const Tree& a, const vs_box* s_nodes, PacketShared& sm, double cx,
+                                              double cy) {
+    const int lane = threadIdx.x & 31;
+    int64_t node = 0;
+    for (int cl = a.levels - 2; cl >= 0; --cl) {
+        const int64_t c = node * kFanout + lane;
+        const float4 rb = child_box(a, s_nodes, cl, c, lane < kFanout && c < a.level_size[cl], cx, cy);
+        if (cl == 0) {
+            if (lane < kFanout) sm.items[lane] = rb;
+            __syncwarp();
+            return (int)(node * kFanout);
+        }
+        const float low = centroid_low(rb), ox = 0.5f * (rb.x + rb.z), oy = 0.5f * (rb.y + rb.w);
+        const float key = rb.x <= rb.z ? fminf(fmaf(low, low, fmaf(ox, ox, oy * oy)), 3e38f) : INFINITY;
+        const unsigned least = __reduce_min_sync(0xffffffffu, __float_as_uint(key));
+        if (least == __float_as_uint(INFINITY)) return -1;
+        node = node * kFanout + __ffs(__ballot_sync(0xffffffffu, __float_as_uint(key) == least)) - 1;
+    }
+    const float4 rb = child_box(a, s_nodes, 0, 0, lane == 0, cx, cy);  // a single item
+    if (lane < kFanout) sm.items[lane] = rb;
+    __syncwarp();
+    return 0;
+}
+
+// The walk.  `radius`: largest distance of a walking lane's query from the
+// centroid.  leaf(slot0, mine): the block's items are slot0 + j, bit j of
+// `mine` says that this lane reaches item j; called by the whole warp, may
+// lower the lane's bound.
+template <class Tree, class Leaf>
+__device__ __forceinline__ void packet_walk(const Tree& a, const vs_box* s_nodes, PacketShared& sm, PacketLane& pl,
+                                            double cx, double cy, float radius, Leaf leaf) {
+    const int lane = threadIdx.x & 31;
+    const int top = a.levels - 1;
+    if (!__any_sync(0xffffffffu, pl.walk)) return;
+    float reach = __fadd_ru(radius, warp_max_nonneg(pl.walk ? pl.ub : 0.f));
+    if (lane == 0) sm.stack[0] = make_int2(top, 0);
+    int sp = 1;
+    __syncwarp();
+    while (sp > 0) {
+        --sp;
+        const int2 e = sm.stack[sp];
+        __syncwarp();
+        if (__int_as_float(e.y) > reach) continue;
+        const int cl = e.x & 15;
+        const bool root = cl == top;
+        const int64_t c = root ? 0 : (int64_t)(e.x >> 4) * kFanout + (lane & 15);
+        const bool in_range = root ? lane == 0 : (lane < kFanout && c < a.level_size[cl]);
+        const float4 rb = child_box(a, s_nodes, cl, c, in_range, cx, cy);
+        const float key = rb.x <= rb.z ? centroid_low(rb) : INFINITY;
+        const unsigned m = __ballot_sync(0xffffffffu, key <= reach && key < INFINITY);
+        if (!m) continue;
+        if (lane < kFanout) sm.items[lane] = rb;
+        __syncwarp();
+        unsigned mine = 0;
+        if (pl.walk) {
+            const float ub2 = __fmul_ru(pl.ub, pl.ub);
+            for (unsigned mm = m; mm; mm &= mm - 1) {
+                const int j = __ffs(mm) - 1;
+                mine |= box_low2(pl.q, sm.items[j]) <= ub2 ? 1u << j : 0u;
+            }
+        }
+        if (cl > 0) {
+            const unsigned keep = __reduce_or_sync(0xffffffffu, mine);
+            const int add = __popc(keep);
+            if (sp + add > kDistStack) {  // cannot happen for < 2^31 items
+                if (lane == 0) atomicOr(&a.counters[4], 1ull);
+                return;
+            }
+            // nearest to the centroid on top of the stack
+            int closer = 0;
+            for (unsigned mm = keep; mm; mm &= mm - 1) {
+                const int j = __ffs(mm) - 1;
+                const float kj = __shfl_sync(0xffffffffu, key, j);
+                closer += kj < key || (kj == key && j < lane) ? 1 : 0;
+            }
+            if ((keep >> lane) & 1u)
+                sm.stack[sp + add - 1 - closer] = make_int2((int)(c << 4) | (cl - 1), __float_as_int(key));
+            sp += add;
+        } else {
+            leaf(root ? 0 : (e.x >> 4) * kFanout, mine);
+            reach = __fadd_ru(radius, warp_max_nonneg(pl.walk ? pl.ub : 0.f));
+        }
+        __syncwarp();
+    }
+}
+
+// Centroid of the finite queries of a packet (the same bits in every lane).
+__device__ __forceinline__ void packet_centroid(bool finite, double x, double y, double& cx, double& cy) {
+    const int nf = __popc(__ballot_sync(0xffffffffu, finite));
+    cx = finite ? x / nf : 0.0;
+    cy = finite ? y / nf : 0.0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        cx += __shfl_xor_sync(0xffffffffu, cx, o);
+        cy += __shfl_xor_sync(0xffffffffu, cy, o);
+    }
+}
+
+// A point as a packet lane.  False (and the lane does not walk) where its
+// offset's square would not fit FP32: the FP64 walk takes such points.
+__device__ __forceinline__ bool point_lane(bool finite, double x, double y, double cx, double cy, PacketLane& pl,
+                                           float& radius) {
+    const float qx = __double2float_rn(x - cx), qy = __double2float_rn(y - cy);
+    const float far = fmaxf(fabsf(qx), fabsf(qy));
+    const float dq = fmaf(far, 6.2e-8f, 1e-37f);
+    pl.q = make_float4(__fsub_rd(qx, dq), __fsub_rd(qy, dq), __fadd_ru(qx, dq), __fadd_ru(qy, dq));
+    pl.walk = finite && far <= 1e17f;
+    radius = warp_max_nonneg(pl.walk ? __fmul_ru(far, 1.42f) : 0.f);
+    return pl.walk;
+}
+
+__device__ __forceinline__ bool finite_coordinate(double v) { return fabs(v) <= 1e300; }
+
+// Queries left to the FP64 walks.
+struct OverList {
+    uint32_t* items;
+    uint32_t* count;
+    __device__ __forceinline__ void add(bool over, uint32_t item) const {
+        const unsigned m = __ballot_sync(0xffffffffu, over);
+        if (!m) return;
+        const int lane = threadIdx.x & 31;
+        uint32_t base = 0;
+        if (lane == 0) base = atomicAdd(count, (uint32_t)__popc(m));
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (over) items[base + __popc(m & ((1u << lane) - 1u))] = item;
+    }
+};
+
+// A lane's list of candidates: (item, bounds) columns in shared memory.
+struct NearShared {
+    int slot[kNearList][32];
+    float lo[kNearList][32];
+    float err[kNearList][32];
+};
+struct NearList {
+    NearShared& s;
+    int cnt;
+    // Add an item; false when the list is full of items the bound still allows.
+    __device__ __forceinline__ bool add(int item, float lo, float err, float ub) {
+        const int lane = threadIdx.x & 31;
+        if (cnt == kNearList) {  // drop what the bound has passed
+            int keep = 0;
+            for (int k = 0; k < kNearList; ++k)
+                if (s.lo[k][lane] <= ub) {
+                    s.slot[keep][lane] = s.slot[k][lane];
+                    s.lo[keep][lane] = s.lo[k][lane];
+                    s.err[keep][lane] = s.err[k][lane];
+                    ++keep;
+                }
+            cnt = keep;
+        }
+        if (cnt == kNearList) return false;
+        s.slot[cnt][lane] = item;
+        s.lo[cnt][lane] = lo;
+        s.err[cnt][lane] = err;
+        ++cnt;
+        return true;
+    }
+};
+
+struct NearArgs {
+    DistArgs d;
+    OverList over;  // sorted positions left to dist_join_kernel
+};
+
+// Nearest polygons of points, all ties, in one walk: a polygon a lane reaches
+// gets FP32 bounds [lo, hi] of its facet distance (facet_bounds); hi lowers
+// the lane's bound, and the polygon joins the lane's short list while lo is
+// within it.  At the end each list holds the polygons within rounding of the
+// nearest, one for nearly every point, and only those get the exact location
+// and FP64 distance.  Points whose list overflows (more than kNearList
+// polygons within rounding of the nearest) go to the two FP64 walks, which
+// compute an exact distance for every polygon met.
+__global__ void __launch_bounds__(kDistThreads, 3) near_kernel(const NearArgs na) {
+    const DistArgs& a = na.d;
+    extern __shared__ vs_box s_nodes[];
+    __shared__ int2 s_buf[kDistWarps][kWarpBuf];
+    __shared__ unsigned s_cnt[kDistWarps];
+    __shared__ PacketShared s_walk[kDistWarps];
+    __shared__ NearShared s_near[kDistWarps];
+    const int64_t stage_base = a.level_off[a.stage_level];
+    for (int k = threadIdx.x; k < a.staged; k += blockDim.x) s_nodes[k] = a.nodes[stage_base + k];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (lane == 0) s_cnt[warp] = 0;
+    __syncthreads();
+    const WarpOut out{s_buf[warp], &s_cnt[warp]};
+    const int64_t n = (int64_t)*a.n_list;
+    const float cap = __double2float_ru(a.radius);  // max_distance (INFINITY: unbounded)
+    unsigned long long n_cand = 0;
+    unsigned n_exact = 0;
+    for (;;) {
+        const int64_t b0 = warp_grab(a.work, kDistGrab);
+        if (b0 >= n) break;
+        const int64_t i = b0 + lane;
+        const bool active = i < n;
+        double x = 0.0, y = 0.0;
+        int32_t row = -1;
+        if (active) {
+            row = (int32_t)a.order[i];
+            x = a.px[row];
+            y = a.py[row];
+        }
+        const bool finite = active && finite_coordinate(x) && finite_coordinate(y);
+        double cx, cy;
+        packet_centroid(finite, x, y, cx, cy);
+        PacketLane pl;
+        float radius;
+        const bool fits = point_lane(finite, x, y, cx, cy, pl, radius);  // whole warp
+        bool over = active && !fits;
+        pl.ub = cap;
+        NearList list{s_near[warp], 0};
+        // bounds of one polygon
+        auto visit = [&](int slot) {
+            ++n_cand;
+            const FacetBounds f = facet_bounds(x, y, a.xy, a.ring_off, a.part_off[a.geom_off[slot]],
+                                               a.part_off[a.geom_off[slot + 1]]);
+            pl.ub = fminf(pl.ub, f.hi);
+            float lo = f.lo;
+            if (lo > 0.f) {
+                // inside the envelope the point may be inside the polygon: distance 0
+                const vs_box b = a.nodes[a.level_off[0] + slot];
+                if (x >= b.minx && x <= b.maxx && y >= b.miny && y <= b.maxy) lo = 0.f;
+            }
+            if (lo <= pl.ub && lo < INFINITY && !list.add(slot, lo, f.full ? -1.f : f.err, pl.ub)) {
+                over = true;
+                pl.walk = false;
+            }
+        };
+        int first = -1;  // the item a lane starts with: the nearest of the descent's block, ties to the nearer centre
+        if (__any_sync(0xffffffffu, pl.walk)) {
+            const int slot0 = packet_descend(a, s_nodes, s_walk[warp], cx, cy);
+            if (slot0 >= 0 && pl.walk) {
+                float bd = INFINITY;
+                for (int j = 0; j < kFanout; ++j) {
+                    const float4 b = s_walk[warp].items[j];
+                    const float ox = 0.5f * (b.x + b.z) - pl.q.x, oy = 0.5f * (b.y + b.w) - pl.q.y;
+                    const float d = box_low2(pl.q, b) + fmaf(ox, ox, oy * oy);
+                    if (b.x <= b.z && d < bd) {
+                        bd = d;
+                        first = slot0 + j;
+                    }
+                }
+                if (first >= 0) {
+                    if (bd <= __fmul_ru(pl.ub, pl.ub)) visit(first);
+                    else first = -1;
+                }
+            }
+            __syncwarp();
+        }
+        packet_walk(a, s_nodes, s_walk[warp], pl, cx, cy, radius, [&](int slot0, unsigned mine) {
+            while (__any_sync(0xffffffffu, mine != 0)) {
+                // the lane's next item within its bound
+                int item = -1;
+                while (mine && item < 0) {
+                    const int j = __ffs(mine) - 1;
+                    mine &= mine - 1;
+                    if (slot0 + j != first && box_low2(pl.q, s_walk[warp].items[j]) <= __fmul_ru(pl.ub, pl.ub)) item = j;
+                }
+                __syncwarp();
+                if (item >= 0) visit(slot0 + item);
+                if (over) mine = 0;
+                __syncwarp();
+            }
+        });
+        __syncwarp();
+        // the exact distances of what is left of the list
+        double best = INFINITY;
+        unsigned left = 0, ties = 0;  // list entries
+        for (int k = 0; k < list.cnt; ++k)
+            if (s_near[warp].lo[k][lane] <= pl.ub) left |= 1u << k;
+        if (!pl.walk) left = 0;
+        __syncwarp();
+        while (__any_sync(0xffffffffu, left != 0)) {
+            if (left) {
+                const int k = __ffs(left) - 1;
+                left &= left - 1;
+                const double d = listed_distance(a, x, y, s_near[warp].slot[k][lane], s_near[warp].err[k][lane],
+                                                 pl.ub, n_exact);
+                if (d < best) ties = 0;
+                best = d < best ? d : best;
+                if (d == best) ties |= 1u << k;
+            }
+            __syncwarp();
+        }
+        if (!(best <= a.radius)) best = INFINITY;
+        if (active && !over) a.best[row] = best;
+        if (!(best < INFINITY)) ties = 0;
+        while (__any_sync(0xffffffffu, ties != 0)) {
+            const bool want = ties != 0;
+            const int k = want ? __ffs(ties) - 1 : 0;
+            ties &= ties - 1;
+            wemit_sync(out, a.sink, want, row, want ? a.item_geom[s_near[warp].slot[k][lane]] : 0);
+        }
+        na.over.add(over, (uint32_t)i);
+        wflush(out, a.sink, false);
+    }
+    wflush(out, a.sink, true);
+    add_counter(a.counters, 5, n_cand);
+    add_counter(a.counters, 1, n_exact);
 }
 
 // Element-wise: row i of the points against row i of the polygons (SoA
@@ -934,6 +1427,252 @@ __global__ void __launch_bounds__(kDistThreads) poly_nearest_kernel(const PolyAr
     add_counter(a.counters, 1, n_exact);
 }
 
+// The same in one walk, as near_kernel does it for points: a lane's query is
+// its polygon's envelope and a leaf item a point, which gets FP32 bounds of its
+// facet distance.  Polygons of a packet lie apart where the points are denser
+// than they are, and a leaf block then concerns one or two lanes: the (lane,
+// point) pairs queue up and are evaluated 32 at a time by whichever lane.  A
+// point in the envelope is located exactly at once: inside, its distance is 0,
+// the smallest there is, so the pair is emitted on the spot and only other
+// points at 0 remain of interest.  The two walks above took 10.6 ms (5.7 to 22
+// with the seed) on 100k footprints x 2M points: they went into every leaf that
+// the box around all 32 polygons touched and computed exact distances there.
+struct PolyNearArgs {
+    PolyArgs d;
+    OverList over;  // polygon rows left to the two walks
+};
+
+__device__ __noinline__ bool located_in(const PolyArgs& a, double px, double py, int g, unsigned& n_exact) {
+    return geometry_location_soa(px, py, a.x, a.y, a.ring_off, a.part_off, a.geom_off, g, n_exact) != LOC_OUTSIDE;
+}
+
+// A packet's queries in shared memory.
+struct PolyPacket {
+    int32_t row[32];
+    int r0[32], r1[32];
+    unsigned ub[32];     // bound (non-negative float bits)
+    int cnt[32];         // list entries
+    int state[32];       // kPoly*
+    int2 queue[64];      // (lane, slot)
+};
+enum : int { kPolyOver = 1, kPolyZero = 2 };  // left to the two walks; a pair at distance 0 was emitted
+
+__global__ void __launch_bounds__(kDistThreads, 3) poly_near_kernel(const PolyNearArgs na) {
+    const PolyArgs& a = na.d;
+    extern __shared__ vs_box s_nodes[];
+    __shared__ int2 s_buf[kDistWarps][kWarpBuf];
+    __shared__ unsigned s_cnt[kDistWarps];
+    __shared__ PacketShared s_walk[kDistWarps];
+    __shared__ NearShared s_near[kDistWarps];
+    __shared__ PolyPacket s_poly[kDistWarps];
+    const int64_t stage_base = a.level_off[a.stage_level];
+    for (int k = threadIdx.x; k < a.staged; k += blockDim.x) s_nodes[k] = a.nodes[stage_base + k];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (lane == 0) s_cnt[warp] = 0;
+    __syncthreads();
+    const WarpOut out{s_buf[warp], &s_cnt[warp]};
+    const unsigned lt = (1u << lane) - 1u;
+    NearShared& near = s_near[warp];
+    PolyPacket& pp = s_poly[warp];
+    const int64_t n = (int64_t)*a.n_valid;
+    const float cap = __double2float_ru(a.cap);
+    const SoaVertices xy{a.x, a.y};
+    unsigned long long n_cand = 0;
+    unsigned n_exact = 0;
+    // evaluate up to 32 queued pairs, one a lane
+    auto drain = [&](int cnt) {
+        // drop what the bounds have passed from the lists, so that they have room
+        {
+            int keep = 0;
+            const float ub = __uint_as_float(pp.ub[lane]);
+            for (int k = 0; k < pp.cnt[lane]; ++k)
+                if (near.lo[k][lane] <= ub) {
+                    near.slot[keep][lane] = near.slot[k][lane];
+                    near.lo[keep][lane] = near.lo[k][lane];
+                    near.err[keep][lane] = near.err[k][lane];
+                    ++keep;
+                }
+            pp.cnt[lane] = keep;
+        }
+        __syncwarp();
+        bool use = lane < cnt, at0 = false;
+        int src = 0, slot = 0, row = 0;
+        double px = 0.0, py = 0.0;
+        FacetBounds f{INFINITY, INFINITY, 0.f, false};
+        if (use) {
+            const int2 e = pp.queue[lane];
+            src = e.x;
+            slot = e.y;
+            row = pp.row[src];
+            use = !(pp.state[src] & kPolyOver);
+        }
+        if (use) {
+            ++n_cand;
+            const vs_box pb = a.nodes[a.level_off[0] + slot];  // a leaf box is its point
+            px = pb.minx;
+            py = pb.miny;
+            const vs_box qb = a.qbox[row];
+            if (px >= qb.minx && px <= qb.maxx && py >= qb.miny && py <= qb.maxy)
+                at0 = located_in(a, px, py, row, n_exact);
+            if (at0) {
+                atomicOr(&pp.state[src], kPolyZero);
+                pp.ub[src] = 0u;
+            } else {
+                f = facet_bounds(px, py, xy, a.ring_off, pp.r0[src], pp.r1[src]);
+                if (!f.full) atomicMin(&pp.ub[src], __float_as_uint(f.hi));
+            }
+        }
+        __syncwarp();
+        if (use && at0) pp.ub[src] = 0u;  // whatever order the bounds arrived in
+        __syncwarp();
+        // the list of the pair's polygon; without room (or bounds) the polygon is left to the two walks, unless pairs
+        // of it have been emitted: its distance is then 0 and the pair is decided here
+        bool failed = false;
+        if (use && !at0 && f.lo < INFINITY && f.lo <= __uint_as_float(pp.ub[src])) {
+            const int k = f.full ? kNearList : atomicAdd(&pp.cnt[src], 1);
+            if (k < kNearList) {
+                near.slot[k][src] = slot;
+                near.lo[k][src] = f.lo;
+                near.err[k][src] = f.err;
+            } else {
+                failed = true;
+            }
+        }
+        __syncwarp();
+        pp.cnt[lane] = pp.cnt[lane] < kNearList ? pp.cnt[lane] : kNearList;
+        if (failed) {
+            if (pp.state[src] & kPolyZero) at0 = point_polygon_soa(a, px, py, row, n_exact) == 0.0;
+            else atomicOr(&pp.state[src], kPolyOver);
+        }
+        __syncwarp();
+        wemit_sync(out, a.sink, at0, row, at0 ? a.item_geom[slot] : 0);
+    };
+    for (;;) {
+        const int64_t b0 = warp_grab(a.work, kDistGrab);
+        if (b0 >= n) break;
+        const int64_t i = b0 + lane;
+        const bool active = i < n;
+        int32_t row = -1;
+        vs_box qb{0.0, 0.0, 0.0, 0.0};
+        if (active) {
+            row = (int32_t)a.order[i];
+            qb = a.qbox[row];
+            pp.r0[lane] = a.part_off[a.geom_off[row]];
+            pp.r1[lane] = a.part_off[a.geom_off[row + 1]];
+        }
+        const bool finite = active && finite_coordinate(qb.minx) && finite_coordinate(qb.miny) &&
+                            finite_coordinate(qb.maxx) && finite_coordinate(qb.maxy);
+        double cx, cy;
+        packet_centroid(finite, 0.5 * qb.minx + 0.5 * qb.maxx, 0.5 * qb.miny + 0.5 * qb.maxy, cx, cy);
+        PacketLane pl;
+        pl.q = relative_box(qb, cx, cy);
+        const float far = fmaxf(fmaxf(fabsf(pl.q.x), fabsf(pl.q.z)), fmaxf(fabsf(pl.q.y), fabsf(pl.q.w)));
+        pl.walk = finite && far <= 1e17f;  // FP32 squares of the offsets must not overflow
+        pl.ub = cap;
+        const float radius = warp_max_nonneg(pl.walk ? __fmul_ru(far, 1.42f) : 0.f);
+        pp.row[lane] = row;
+        pp.ub[lane] = __float_as_uint(cap);
+        pp.cnt[lane] = 0;
+        pp.state[lane] = active && !pl.walk ? kPolyOver : 0;
+        int nq = 0;      // warp-uniform queue length
+        int first = -1;  // the point a lane starts with
+        __syncwarp();
+        auto push = [&](bool has, int slot) {
+            const unsigned m = __ballot_sync(0xffffffffu, has);
+            if (has) pp.queue[nq + __popc(m & lt)] = make_int2(lane, slot);
+            nq += __popc(m);
+            __syncwarp();
+            if (nq >= 32) {
+                drain(32);
+                __syncwarp();
+                if (lane < nq - 32) pp.queue[lane] = pp.queue[32 + lane];
+                nq -= 32;
+                __syncwarp();
+            }
+        };
+        auto take_bounds = [&]() {
+            pl.ub = __uint_as_float(pp.ub[lane]);
+            if (pp.state[lane] & kPolyOver) pl.walk = false;
+        };
+        if (__any_sync(0xffffffffu, pl.walk)) {
+            // each lane starts with the point of the descent's block nearest to its envelope's centre
+            const int slot0 = packet_descend(a, s_nodes, s_walk[warp], cx, cy);
+            if (slot0 >= 0 && pl.walk) {
+                float bd = INFINITY;
+                for (int j = 0; j < kFanout; ++j) {
+                    const float4 p = s_walk[warp].items[j];
+                    const float ox = p.x - 0.5f * (pl.q.x + pl.q.z), oy = p.y - 0.5f * (pl.q.y + pl.q.w);
+                    const float d = fmaf(ox, ox, oy * oy);
+                    if (p.x <= p.z && d < bd) {
+                        bd = d;
+                        first = slot0 + j;
+                    }
+                }
+            }
+            __syncwarp();
+            push(first >= 0, first);
+            if (nq > 0) drain(nq);
+            nq = 0;
+            __syncwarp();
+            take_bounds();
+        }
+        packet_walk(a, s_nodes, s_walk[warp], pl, cx, cy, radius, [&](int slot0, unsigned mine) {
+            while (__any_sync(0xffffffffu, mine != 0)) {
+                int item = -1;
+                while (mine && item < 0) {
+                    const int j = __ffs(mine) - 1;
+                    mine &= mine - 1;
+                    if (slot0 + j != first && box_low2(pl.q, s_walk[warp].items[j]) <= __fmul_ru(pl.ub, pl.ub)) item = j;
+                }
+                __syncwarp();
+                push(item >= 0, slot0 + item);
+                take_bounds();
+                if (!pl.walk) mine = 0;
+            }
+        });
+        __syncwarp();
+        if (nq > 0) drain(nq);
+        __syncwarp();
+        take_bounds();
+        const bool over = (pp.state[lane] & kPolyOver) != 0;
+        // the exact distances of what is left of the lists
+        double best = (pp.state[lane] & kPolyZero) ? 0.0 : INFINITY;
+        unsigned left = 0, ties = 0;
+        for (int k = 0; k < pp.cnt[lane]; ++k)
+            if (near.lo[k][lane] <= pl.ub) left |= 1u << k;
+        if (!pl.walk) left = 0;
+        __syncwarp();
+        while (__any_sync(0xffffffffu, left != 0)) {
+            if (left) {
+                const int k = __ffs(left) - 1;
+                left &= left - 1;
+                // (a point in the envelope on this list was located outside)
+                const vs_box p = a.nodes[a.level_off[0] + near.slot[k][lane]];
+                const double d = facet_distance_bounded(p.minx, p.miny, xy, a.ring_off, pp.r0[lane], pp.r1[lane],
+                                                        pl.ub, near.err[k][lane]);
+                if (d < best) ties = 0;
+                best = d < best ? d : best;
+                if (d == best) ties |= 1u << k;
+            }
+            __syncwarp();
+        }
+        if (!(best <= a.cap)) best = INFINITY;
+        if (active && !over) a.best[row] = best;
+        if (!(best < INFINITY)) ties = 0;
+        while (__any_sync(0xffffffffu, ties != 0)) {
+            const bool want = ties != 0;
+            const int k = want ? __ffs(ties) - 1 : 0;
+            ties &= ties - 1;
+            wemit_sync(out, a.sink, want, row, want ? a.item_geom[near.slot[k][lane]] : 0);
+        }
+        na.over.add(over, (uint32_t)row);
+        wflush(out, a.sink, false);
+    }
+    wflush(out, a.sink, true);
+    add_counter(a.counters, 5, n_cand);
+    add_counter(a.counters, 1, n_exact);
+}
+
 }  // namespace
 }  // namespace vs
 
@@ -1011,7 +1750,18 @@ int vs_join_nearest(vs_context* ctx, const vs_index* idx, const vs_points* pts, 
     a.best = best.p;
     a.radius = max_distance;  // the search cap
     a.sink = PairSink{d_left, d_right, (unsigned long long)(capacity > 0 ? capacity : 0), &ctx->d_counters[0]};
-    // each point's minimum distance, then every polygon at exactly that distance
+    // one walk answers nearly every point; the rest (over_list) get each point's minimum distance, then every
+    // polygon at exactly that distance
+    Scratch<uint32_t> over, n_over;
+    VS_TRY(over.alloc((size_t)pts->n, s));
+    VS_TRY(n_over.alloc(1, s));
+    VS_CUDA_TRY(cudaMemsetAsync(n_over.p, 0, sizeof(uint32_t), s));
+    const NearArgs near{a, {over.p, n_over.p}};
+    VS_CUDA_TRY(cudaFuncSetAttribute(near_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    near_kernel<<<resident_grid(near_kernel, pts->n, kDistThreads, smem), kDistThreads, smem, s>>>(near);
+    VS_LAUNCHED("near", s);
+    a.list = over.p;
+    a.n_list = n_over.p;
     VS_TRY(launch_dist<kNearestMin>(ctx, a, smem, pts->n));
     VS_TRY(launch_dist<kNearestEmit>(ctx, a, smem, pts->n));
     const int st = finish_join(ctx, idx, pts, flags, d_left, d_right, capacity, n_pairs, stats, ev, launches0);
@@ -1125,7 +1875,18 @@ int vs_join_nearest_polygons(vs_context* ctx, const vs_index* point_index, const
     a.counters = ctx->d_counters;
     a.work = &ctx->d_counters[kWorkCounter];
     const size_t smem = (size_t)a.staged * sizeof(vs_box);
-    // each polygon's minimum distance, then every point at exactly that distance
+    // one walk answers nearly every polygon; the rest (over) get each polygon's minimum distance, then every point
+    // at exactly that distance
+    Scratch<uint32_t> over, n_over;
+    VS_TRY(over.alloc((size_t)nq, s));
+    VS_TRY(n_over.alloc(1, s));
+    VS_CUDA_TRY(cudaMemsetAsync(n_over.p, 0, sizeof(uint32_t), s));
+    const PolyNearArgs near{a, {over.p, n_over.p}};
+    VS_CUDA_TRY(cudaFuncSetAttribute(poly_near_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    poly_near_kernel<<<resident_grid(poly_near_kernel, nq, kDistThreads, smem), kDistThreads, smem, s>>>(near);
+    VS_LAUNCHED("poly_near", s);
+    a.order = over.p;
+    a.n_valid = n_over.p;
     VS_CUDA_TRY(cudaMemsetAsync(a.work, 0, sizeof(unsigned long long), s));
     VS_CUDA_TRY(cudaFuncSetAttribute(poly_nearest_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)smem));
