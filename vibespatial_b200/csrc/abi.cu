@@ -152,7 +152,13 @@ int vs_context_create(int device, void* stream, vs_context** out) {
         cudaGetLastError();
     }
     bool ok = cudaMallocHost((void**)&ctx->h_counter, kHostCounters * sizeof(unsigned long long)) == cudaSuccess &&
-              cudaMalloc((void**)&ctx->d_counters, kDevCounters * sizeof(unsigned long long)) == cudaSuccess;
+              cudaMalloc((void**)&ctx->d_counters, (kDevCounters + kDirectWords) * sizeof(unsigned long long)) ==
+                  cudaSuccess;
+    if (ok) {
+        ctx->d_direct = ctx->d_counters + kDevCounters;
+        ok = cudaMemsetAsync(ctx->d_direct, 0, kDirectWords * sizeof(unsigned long long), ctx->stream) == cudaSuccess &&
+             cudaMemsetAsync(ctx->d_direct + kDirectStart, 0xff, sizeof(unsigned long long), ctx->stream) == cudaSuccess;
+    }
     for (int k = 0; k < 5 && ok; ++k) ok = cudaEventCreate(&ctx->phase_ev[k]) == cudaSuccess;
     if (!ok) {
         cudaGetLastError();
@@ -267,6 +273,45 @@ int vs_index_free(vs_index* idx) {
     return VS_OK;
 }
 
+// A learned join of few points: one launch and one wait.
+static int direct_join(vs_context* ctx, const vs_index* idx, const vs_points* pts, int mask, bool sort, int32_t* d_left,
+                       int32_t* d_right, int64_t capacity, int64_t* n_pairs, vs_join_stats* stats) {
+    const long long launches0 = g_launches;
+    VS_TRY(launch_direct_join(ctx, idx, pts, mask, d_left, d_right, capacity, sort));
+    VS_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+    const volatile unsigned long long* c = ctx->h_counter;
+    const int64_t n = (int64_t)c[kDirectPairs];
+    const bool sorted = c[kDirectTicket] != 0;
+    *n_pairs = n;
+    if (stats) {
+        stats->exact_fallbacks = (int64_t)c[kDirectExact];
+        stats->fp32_edges = (int64_t)c[kDirectFp32];
+        stats->fp64_edges = (int64_t)c[kDirectFp64];
+        stats->candidates = (int64_t)c[kDirectCandidates];
+        stats->rmi_fallbacks = (int64_t)c[kDirectWide];
+        // (the last block's sort of few pairs is part of it)
+        stats->kernel_ms = (float)(1e-6 * (double)c[kDirectStart]);
+        stats->phase_ms[2] = stats->kernel_ms;
+        stats->kernel_launches = g_launches - launches0;
+    }
+    if (n > capacity) {
+        set_error("pair buffer holds %lld pairs, %lld required", (long long)capacity, (long long)n);
+        return VS_E_CAPACITY;
+    }
+    if (sort && !sorted && n > 1) {
+        EventPair es;
+        cudaEventRecord(es.a, ctx->stream);
+        VS_TRY(sort_pairs(ctx, d_left, d_right, n, (uint64_t)pts->n, (uint64_t)idx->n_geoms));
+        cudaEventRecord(es.b, ctx->stream);
+        if (stats) {
+            VS_CUDA_TRY(cudaEventSynchronize(es.b));
+            stats->sort_ms = es.ms();
+            stats->kernel_launches = g_launches - launches0;
+        }
+    }
+    return VS_OK;
+}
+
 int vs_join(vs_context* ctx, const vs_index* idx, const vs_points* pts, int32_t predicate, int32_t method,
             uint32_t flags, int32_t* d_left, int32_t* d_right, int64_t capacity, int64_t* n_pairs,
             vs_join_stats* stats) {
@@ -298,6 +343,10 @@ int vs_join(vs_context* ctx, const vs_index* idx, const vs_points* pts, int32_t 
     if (pts->n == 0 || idx->n_geoms == 0 || !(idx->h_frame[0] <= idx->h_frame[2])) return VS_OK;
     cudaStream_t s = ctx->stream;
     const long long launches0 = g_launches;
+    constexpr uint32_t kAblations = VS_JOIN_LEARNED_BSEARCH | VS_JOIN_LEARNED_FP64_WALK | VS_JOIN_LEARNED_NO_STAGE |
+                                    VS_JOIN_LEARNED_NO_INTERIOR;
+    if (method == VS_METHOD_LEARNED && direct_join_pays(idx, pts->n) && !(flags & kAblations))
+        return direct_join(ctx, idx, pts, mask, (flags & VS_JOIN_SORT) != 0, d_left, d_right, capacity, n_pairs, stats);
     EventPair ev;
     // Pairs the filters cannot certify go to the context's deferred buffer
     // and are resolved exactly after the join kernel; if more were deferred
@@ -334,6 +383,15 @@ int vs_join(vs_context* ctx, const vs_index* idx, const vs_points* pts, int32_t 
         want = ctx->h_counter[7];
     }
     const unsigned long long* c = ctx->h_counter;
+    // Sound pairs are sorted while the host reads the times below
+    const bool sort = (flags & VS_JOIN_SORT) && c[7] <= ctx->defer_cap && c[4] == 0 && (int64_t)c[0] <= capacity &&
+                      c[0] > 1;
+    EventPair es;
+    if (sort) {
+        cudaEventRecord(es.a, s);
+        VS_TRY(enqueue_sort_pairs(ctx, d_left, d_right, (int64_t)c[0], (uint64_t)pts->n, (uint64_t)idx->n_geoms, true));
+        cudaEventRecord(es.b, s);
+    }
     if (c[7] > ctx->defer_cap) {
         set_error("deferred-pair buffer did not converge (%llu pairs)", c[7]);
         return VS_E_STATE;
@@ -362,13 +420,9 @@ int vs_join(vs_context* ctx, const vs_index* idx, const vs_points* pts, int32_t 
         set_error("pair buffer holds %lld pairs, %lld required", (long long)capacity, (long long)n);
         return VS_E_CAPACITY;
     }
-    if (flags & VS_JOIN_SORT) {
-        EventPair es;
-        cudaEventRecord(es.a, s);
-        VS_TRY(sort_pairs(ctx, d_left, d_right, n, (uint64_t)pts->n, (uint64_t)idx->n_geoms));
-        cudaEventRecord(es.b, s);
+    if (sort) {
+        VS_TRY(finish_sort_pairs(ctx, d_left, d_right, n, (uint64_t)pts->n, (uint64_t)idx->n_geoms));
         if (stats) {
-            VS_CUDA_TRY(cudaEventSynchronize(es.b));
             stats->sort_ms = es.ms();
             stats->kernel_launches = g_launches - launches0;
         }

@@ -162,6 +162,7 @@ struct LearnedIndex {
     float rmi_train_ms = 0.f;
     float rmi_final_loss = 0.f;
     float mean_window = 0.f;
+    float mean_list = 1.f;           // mean over the entries of their cell's entry count
     int32_t max_window = 0;
 };
 

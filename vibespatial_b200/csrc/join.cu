@@ -506,14 +506,19 @@ int enqueue_sort_pairs(vs_context* ctx, int32_t* d_left, int32_t* d_right, int64
                             &ctx->d_counters[kSortErr]);
 }
 
+int finish_sort_pairs(vs_context* ctx, int32_t* d_left, int32_t* d_right, int64_t n, uint64_t max_left,
+                      uint64_t max_right) {
+    VS_TRY(finish_sort(ctx));
+    if (!(ctx->h_counter[kHostCounters - 1] & 4)) return VS_OK;
+    // a left row with very many pairs
+    VS_TRY(enqueue_sort_pairs(ctx, d_left, d_right, n, max_left, max_right, false));
+    return finish_sort(ctx);
+}
+
 int sort_pairs(vs_context* ctx, int32_t* d_left, int32_t* d_right, int64_t n, uint64_t max_left, uint64_t max_right) {
-    for (int attempt = 0; attempt < 2; ++attempt) {
-        VS_TRY(clear_sort_error(ctx));
-        VS_TRY(enqueue_sort_pairs(ctx, d_left, d_right, n, max_left, max_right, attempt == 0));
-        VS_TRY(finish_sort(ctx));
-        if (!(ctx->h_counter[kHostCounters - 1] & 4)) break;  // else: a left row with very many pairs
-    }
-    return VS_OK;
+    VS_TRY(clear_sort_error(ctx));
+    VS_TRY(enqueue_sort_pairs(ctx, d_left, d_right, n, max_left, max_right, true));
+    return finish_sort_pairs(ctx, d_left, d_right, n, max_left, max_right);
 }
 
 int clear_sort_error(vs_context* ctx) {

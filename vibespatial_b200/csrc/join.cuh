@@ -22,6 +22,23 @@ int accept_mask_for(int predicate, int* mask);
 int launch_rtree_join(vs_context* ctx, const vs_index* idx, const vs_points* pts, int accept_mask, bool brute,
                       bool bulk_leaves, int32_t* d_left, int32_t* d_right, int64_t capacity, const DeferSink& dsink,
                       int64_t row_base = 0);
+// Whether a learned join of n points runs as one direct launch (no grouping):
+// while the records it tests, n times the mean list length of a cell, stay
+// below kDirectWork.  Whole sorted calls, direct against grouped, us:
+//   1000 stars (lists of 2.5)     32k 114/189  262k 158/217  1M 280/309
+//   50k stars (30)                1k 126/488   32k 354/547   65k 607/589
+//   100k footprints, UTM (1.2)    32k 35/165   262k 109/180  1M 145/204
+//   1M footprints, Zipf (2.4)     32k 108/235  524k 235/297  1M 336/336
+//   40k with holes, parts (12)    8k 149/255   131k 290/302  262k 444/360
+constexpr int64_t kDirectPoints = 1 << 20;
+constexpr double kDirectWork = 1.5e6;
+inline bool direct_join_pays(const vs_index* idx, int64_t n) {
+    return n <= kDirectPoints && (double)n * idx->learned.mean_list <= kDirectWork;
+}
+// Enqueue it; after the stream has been waited for, ctx->h_counter holds the
+// kDirect* words (ticket: whether the pairs are sorted, start: device time in ns).
+int launch_direct_join(vs_context* ctx, const vs_index* idx, const vs_points* pts, int accept_mask, int32_t* d_left,
+                       int32_t* d_right, int64_t capacity, bool sort);
 int launch_learned_join(vs_context* ctx, const vs_index* idx, const vs_points* pts, int accept_mask,
                         int32_t* d_left, int32_t* d_right, int64_t capacity, const DeferSink& dsink,
                         int64_t row_base = 0, const LearnedShape& shape = LearnedShape{});
@@ -42,6 +59,9 @@ int sort_pairs(vs_context* ctx, int32_t* d_left, int32_t* d_right, int64_t n, ui
 // gave up; finish_sort waits for the stream and reads it.
 int enqueue_sort_pairs(vs_context* ctx, int32_t* d_left, int32_t* d_right, int64_t n, uint64_t max_left,
                        uint64_t max_right, bool by_runs);
+// Wait for an enqueued sort (by_runs), and sort by every digit what it left.
+int finish_sort_pairs(vs_context* ctx, int32_t* d_left, int32_t* d_right, int64_t n, uint64_t max_left,
+                      uint64_t max_right);
 int clear_sort_error(vs_context* ctx);
 int finish_sort(vs_context* ctx);
 int build_rtree(vs_context* ctx, const vs_polygons* P, vs_index* idx);

@@ -1060,10 +1060,15 @@ int build_learned_index(vs_context* ctx, vs_index* idx, const vs_index_options* 
     VS_TRY(ncell.alloc(1, s));
     cell_flag_kernel<<<grid_for(E, 256), 256, 0, s>>>(keys.p, (int64_t)E, flag.p);
     VS_TRY(exclusive_scan_u32(flag.p, flag.p, (int64_t)E, ncell.p, s));
+    VS_CUDA_TRY(cudaMemsetAsync(tot.p, 0, sizeof(unsigned long long), s));
+    cell_run_sq_kernel<<<grid_for(E, 256), 256, 0, s>>>(keys.p, (int64_t)E, tot.p);
     uint32_t nc = 0;
+    unsigned long long sum_sq = 0;
+    VS_CUDA_TRY(cudaMemcpyAsync(&sum_sq, tot.p, sizeof(sum_sq), cudaMemcpyDeviceToHost, s));
     VS_CUDA_TRY(cudaMemcpyAsync(&nc, ncell.p, sizeof(nc), cudaMemcpyDeviceToHost, s));
     VS_CUDA_TRY(cudaStreamSynchronize(s));
     li.n_cells = nc;
+    li.mean_list = E > 0 ? (float)((double)sum_sq / (double)E) : 1.f;
     VS_TRY(dalloc(&li.cell_keys, (size_t)nc, bytes, ctx));
     VS_TRY(dalloc(&li.cell_start, (size_t)nc + 1, bytes, ctx));
     cell_compact_kernel<<<grid_for(E, 256), 256, 0, s>>>(keys.p, flag.p, (int64_t)E, li.cell_keys, li.cell_start);

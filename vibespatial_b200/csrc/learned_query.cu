@@ -22,6 +22,8 @@
 //            the rounding-error bound is deferred to the exact pass, which
 //            walks it on the FP64 coordinates (Shewchuk's stage-A filter, then
 //            the exact expansion).
+//
+// Joins of few points skip the grouping (learned_direct_kernel).
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
@@ -254,16 +256,13 @@ __device__ __forceinline__ int geometry_location_split(float qx, float qy, float
 }
 
 // ---------------------------------------------------------------- map ---
-// Exact lookup of grid cell (gx, gy) (32-bit grid coordinates) in job J's
-// learned index: level-L cell key -> occupancy bit -> root table -> leaf
-// model -> binary search inside the leaf's error window.  Returns the cell's
+// Exact lookup of a level-L cell key in job J's learned index: occupancy bit
+// -> root table -> leaf model -> binary search inside the leaf's error window.  Returns the cell's
 // index, or -1 when no stored cell matches (no polygon box overlaps it).
 // kBsearch (an ablation): the model is skipped and the search covers every
 // stored key.
 template <bool kBsearch>
-__device__ __forceinline__ int learned_lookup(const LearnedJob& J, uint32_t gx, uint32_t gy, const uint16_t* lut,
-                                              unsigned long long& n_wide) {
-    const uint32_t cell = hilbert_key_lut(gx, gy, J.L, lut);
+__device__ __forceinline__ int learned_lookup(const LearnedJob& J, uint32_t cell, unsigned long long& n_wide) {
     const uint32_t ob = cell >> J.occ_shift;
     // the occupancy word and the root-table entry depend only on the key:
     // both loads are issued before either is tested
@@ -319,7 +318,7 @@ __device__ __forceinline__ int map_point(const LqArgs& a, int64_t i, int job, co
           y <= J.hiy))
         return -1;
     const uint32_t gx = quantize(x, J.lox, J.sx), gy = quantize(y, J.loy, J.sy);
-    const int c = learned_lookup<kBsearch>(J, gx, gy, lut, n_wide);
+    const int c = learned_lookup<kBsearch>(J, hilbert_key_lut(gx, gy, J.L, lut), n_wide);
     if (c < 0) return -1;
     const int sh = 32 - J.L;
     qx = __double2float_rn(__dsub_rn(x, cell_anchor(J.lox, J.cwx, gx >> sh)));
@@ -446,6 +445,10 @@ struct GroupedLane {
     float dq;
 };
 
+__device__ __forceinline__ float point_error(float qx, float qy) {
+    return __fmaf_ru(fmaxf(fabsf(qx), fabsf(qy)), 6.1e-8f, 1e-37f);
+}
+
 template <bool kMulti>
 __device__ __forceinline__ GroupedLane load_grouped(const LqArgs& a, int64_t j, int64_t e0) {
     GroupedLane g;
@@ -460,7 +463,7 @@ __device__ __forceinline__ GroupedLane load_grouped(const LqArgs& a, int64_t j, 
         g.lo = J.cell_start[c];
         g.len = J.cell_start[c + 1] - g.lo;
     }
-    g.dq = __fmaf_ru(fmaxf(fabsf(g.p.qx), fabsf(g.p.qy)), 6.1e-8f, 1e-37f);
+    g.dq = point_error(g.p.qx, g.p.qy);
     return g;
 }
 
@@ -469,6 +472,22 @@ __device__ __forceinline__ GroupedLane load_grouped(const LqArgs& a, int64_t j, 
 __device__ __forceinline__ bool box_filter_fp32(const float4& bx, float qx, float qy, float dq) {
     return !(__fadd_ru(qx, dq) < bx.x || __fsub_rd(qx, dq) > bx.z || __fadd_ru(qy, dq) < bx.y ||
              __fsub_rd(qy, dq) > bx.w);
+}
+
+// The point in a record's slot frame and the tolerance t of every coordinate
+// difference there: its error against the real p - origin is at most dq +
+// |off error| (in r.err with the vertex error) + the rounding of the addition.
+__device__ __forceinline__ void slot_offset(const EntryRecord& r, float qx, float qy, float dq, float& sx, float& sy,
+                                            float& t) {
+    sx = __fadd_rn(qx, r.offx);
+    sy = __fadd_rn(qy, r.offy);
+    const float es = __fmaf_ru(fmaxf(fabsf(sx), fabsf(sy)), 6.1e-8f, 1e-37f);
+    t = __fmul_ru(__fadd_ru(__fadd_ru(r.err, dq), es), 1.0001f);
+}
+
+// Strictly inside the slot's interior box, whatever the rounding: interior.
+__device__ __forceinline__ bool in_interior_box(const float4& ib, float sx, float sy, float t) {
+    return __fsub_rd(sx, t) > ib.x && __fadd_ru(sx, t) < ib.z && __fsub_rd(sy, t) > ib.y && __fadd_ru(sy, t) < ib.w;
 }
 
 __device__ __forceinline__ unsigned warp_max_u32(unsigned v) {
@@ -635,24 +654,14 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) learned_refine_kernel(co
                     r = (staged && si < run_hi - run_lo) ? st[si] : recs[g.lo + k];
                     inbox = box_filter_fp32(r.box, g.p.qx, g.p.qy, g.dq);
                 }
-                // the point in the slot's frame; its error against the real p -
-                // origin is at most dq + |off error| (in r.err with the vertex
-                // error) + the rounding of this addition (es)
                 float sx = 0.f, sy = 0.f, t = 0.f;
                 bool walk = false, direct = false;
                 if (inbox) {
                     ++n_cand;
-                    sx = __fadd_rn(g.p.qx, r.offx);
-                    sy = __fadd_rn(g.p.qy, r.offy);
-                    const float es = __fmaf_ru(fmaxf(fabsf(sx), fabsf(sy)), 6.1e-8f, 1e-37f);
-                    t = __fmul_ru(__fadd_ru(__fadd_ru(r.err, g.dq), es), 1.0001f);
+                    slot_offset(r, g.p.qx, g.p.qy, g.dq, sx, sy, t);
                     walk = true;
                     if (!a.no_interior && entry_has_interior(r)) {
-                        // strictly inside the slot's interior box, whatever the
-                        // rounding: interior, no ring walk
-                        const float4 ib = ib32[entry_slot(r)];
-                        if (__fsub_rd(sx, t) > ib.x && __fadd_ru(sx, t) < ib.z && __fsub_rd(sy, t) > ib.y &&
-                            __fadd_ru(sy, t) < ib.w) {
+                        if (in_interior_box(ib32[entry_slot(r)], sx, sy, t)) {
                             walk = false;
                             direct = (a.q.accept_mask >> LOC_INTERIOR) & 1;
                         }
@@ -685,6 +694,196 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) learned_refine_kernel(co
     add_counter(a.counters, 5, n_cand);
     add_counter(a.counters, 2, n32);
     add_counter(a.counters, 3, n64);
+}
+
+// ------------------------------------------------------------- direct ---
+// A small join in one launch: no grouping.  A point's cell is looked up and
+// its records are tested by one lane, or by 2 to 32 lanes together where the
+// points alone would leave the chip idle: FP32 box, interior box, then a
+// warp-local queue for the FP32 ring walks as in the refine pass; where a
+// decision lies within the rounding error the exact location follows at once.
+// The last block to finish reports the counters to pinned host memory, zeroes
+// them for the next call and, when the pairs are few, sorts them, so that the
+// call is one launch and one wait.
+//
+// Bound by latency: the chain of dependent index loads, then the launch and
+// the wait themselves (1003 points x 10 stars: 31 us a call; the grouped
+// passes, their counters, events and sort took 121).
+constexpr int kDirectThreads = 256;
+constexpr int kDirectSort = 512;  // pairs the last block sorts (each compared with all others)
+
+struct DirectArgs {
+    LearnedJob job;
+    const double* px;
+    const double* py;
+    const uint8_t* pvalid;
+    int64_t n;
+    int accept_mask;
+    PairSink sink;
+    unsigned long long* state;  // kDirect* words, zero between calls (start: all ones)
+    unsigned long long* host;   // pinned: the words, with start replaced by the device time in ns
+    bool sort;
+    int share;                  // 2^share lanes work on one point
+};
+
+// Ring walks of up to 32 queued pairs, one a lane, decided to the end.
+template <bool kBins>
+__device__ __forceinline__ void direct_queued(const DirectArgs& a, const WarpOut& out, const QueuedPair* qp, int nq,
+                                              int lane, unsigned& n32, unsigned& n64, unsigned& n_exact) {
+    const LearnedJob& J = a.job;
+    bool want = false;
+    int32_t row = 0, right = 0;
+    if (lane < nq) {
+        const QueuedPair e = qp[lane];
+        row = e.row;
+        const PointRef P{a.px, a.py, (int64_t)row};
+        const int2 cr = J.c01[e.slot];
+        int loc = cr.x >= 0 ? ring_location_split(e.qx, e.qy, e.t, J.xy32, cr.x, cr.y, n32, n64)
+                            : geometry_location_split<kBins>(e.qx, e.qy, e.t, J, e.slot, P, n32, n64);
+        if (loc == LOC_UNDECIDED)
+            loc = geometry_location(a.px[row], a.py[row], J.xy, J.ring_off, J.part_off, J.geom_off, e.slot, J.rings,
+                                    n_exact);
+        want = (a.accept_mask >> loc) & 1;
+        if (want) right = J.item_geom[e.slot];
+    }
+    wemit_sync(out, a.sink, want, row, right);
+}
+
+template <bool kBins>
+__global__ void __launch_bounds__(kDirectThreads) learned_direct_kernel(const DirectArgs a) {
+    __shared__ int2 s_buf[kDirectThreads / 32][kWarpBuf];
+    __shared__ unsigned s_cnt[kDirectThreads / 32];
+    __shared__ QueuedPair s_q[kDirectThreads / 32][kQueue];
+    __shared__ unsigned long long s_key[kDirectSort];
+    __shared__ bool s_last;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned long long t0 = 0;
+    if (threadIdx.x == 0) {
+        asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
+        atomicMin(&a.state[kDirectStart], t0);
+    }
+    if (lane == 0) s_cnt[warp] = 0;
+    __syncwarp();
+    const WarpOut out{s_buf[warp], &s_cnt[warp]};
+    const LearnedJob& J = a.job;
+    const int64_t gw = ((int64_t)blockIdx.x * kDirectThreads + threadIdx.x) >> 5;
+    const int64_t nw = ((int64_t)gridDim.x * kDirectThreads) >> 5;
+    const int per = 32 >> a.share;                   // points a warp takes at once
+    const uint32_t lanes = 1u << a.share;            // lanes a point has
+    const uint32_t sub = (uint32_t)lane & (lanes - 1);
+    unsigned long long n_wide = 0, n_cand = 0;
+    unsigned n32 = 0, n64 = 0, n_exact = 0;
+    QueuedPair* qp = s_q[warp];
+    const unsigned lt = (1u << lane) - 1u;
+    int nq = 0;  // warp-uniform queue length
+    for (int64_t b0 = gw * per; b0 < a.n; b0 += nw * per) {
+        const int64_t i = b0 + (lane >> a.share);
+        double x = 0.0, y = 0.0;
+        float qx = 0.f, qy = 0.f;
+        uint32_t lo = 0, len = 0;
+        if (i < a.n) {
+            x = a.px[i];
+            y = a.py[i];
+            if ((a.pvalid == nullptr || a.pvalid[i]) && J.n_cells > 0 && x >= J.lox && x <= J.hix && y >= J.loy &&
+                y <= J.hiy) {
+                const uint32_t gx = quantize(x, J.lox, J.sx), gy = quantize(y, J.loy, J.sy);
+                unsigned long long wide = 0;
+                const int c = learned_lookup<false>(J, (uint32_t)hilbert_key(gx, gy, J.L), wide);
+                n_wide += sub == 0 ? wide : 0;
+                if (c >= 0) {
+                    const int sh = 32 - J.L;
+                    qx = __double2float_rn(__dsub_rn(x, cell_anchor(J.lox, J.cwx, gx >> sh)));
+                    qy = __double2float_rn(__dsub_rn(y, cell_anchor(J.loy, J.cwy, gy >> sh)));
+                    lo = J.cell_start[c];
+                    len = J.cell_start[c + 1] - lo;
+                }
+            }
+        }
+        const float dq = point_error(qx, qy);
+        const uint32_t maxlen = warp_max_u32(len);
+        for (uint32_t k0 = 0; k0 < maxlen; k0 += lanes) {
+            const uint32_t k = k0 + sub;
+            bool want = false, walk = false;
+            float sx = 0.f, sy = 0.f, t = 0.f;
+            int32_t slot = 0;
+            if (k < len) {
+                const EntryRecord r = J.recs[lo + k];
+                if (box_filter_fp32(r.box, qx, qy, dq)) {
+                    slot = entry_slot(r);
+                    if (!a.accept_mask) {  // box candidates: the exact FP64 box
+                        const vs_box bb = J.boxes[slot];
+                        want = x >= bb.minx && x <= bb.maxx && y >= bb.miny && y <= bb.maxy;
+                        n_cand += want ? 1 : 0;
+                    } else {
+                        ++n_cand;
+                        slot_offset(r, qx, qy, dq, sx, sy, t);
+                        walk = true;
+                        if (entry_has_interior(r) && in_interior_box(J.ib32[slot], sx, sy, t)) {
+                            walk = false;
+                            want = (a.accept_mask >> LOC_INTERIOR) & 1;
+                        }
+                    }
+                }
+            }
+            wemit_sync(out, a.sink, want, (int32_t)i, want ? J.item_geom[slot] : 0);
+            const unsigned m = __ballot_sync(0xffffffffu, walk);
+            if (walk) {
+                float4* e = reinterpret_cast<float4*>(&qp[nq + __popc(m & lt)]);
+                e[0] = make_float4(sx, sy, t, __int_as_float((int32_t)i));
+                e[1] = make_float4(__int_as_float(slot), 0.f, 0.f, 0.f);
+            }
+            nq += __popc(m);
+            __syncwarp();
+            if (nq >= 32) {
+                direct_queued<kBins>(a, out, qp, 32, lane, n32, n64, n_exact);
+                __syncwarp();
+                if (lane < nq - 32) qp[lane] = qp[32 + lane];
+                nq -= 32;
+                __syncwarp();
+            }
+        }
+        wflush(out, a.sink, false);
+    }
+    if (nq > 0) direct_queued<kBins>(a, out, qp, nq, lane, n32, n64, n_exact);
+    wflush(out, a.sink, true);
+    add_counter(a.state, kDirectExact, n_exact);
+    add_counter(a.state, kDirectFp32, n32);
+    add_counter(a.state, kDirectFp64, n64);
+    add_counter(a.state, kDirectCandidates, n_cand);
+    add_counter(a.state, kDirectWide, n_wide);
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(&a.state[kDirectTicket], 1ull) == gridDim.x - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    const unsigned long long pairs = __ldcg(&a.state[kDirectPairs]);
+    const bool sorted = a.sort && pairs <= kDirectSort && pairs <= a.sink.capacity;
+    if (sorted && pairs > 1) {
+        const int m = (int)pairs;
+        for (int k = threadIdx.x; k < m; k += kDirectThreads)
+            s_key[k] = ((unsigned long long)(unsigned)__ldcg(&a.sink.out_left[k]) << 32) |
+                       (unsigned)__ldcg(&a.sink.out_right[k]);
+        __syncthreads();
+        for (int k = threadIdx.x; k < m; k += kDirectThreads) {
+            const unsigned long long key = s_key[k];
+            int pos = 0;
+            for (int j = 0; j < m; ++j) pos += s_key[j] < key ? 1 : 0;  // (a join's pairs are distinct)
+            a.sink.out_left[pos] = (int32_t)(key >> 32);
+            a.sink.out_right[pos] = (int32_t)(key & 0xffffffffull);
+        }
+    }
+    if (threadIdx.x < kDirectWords) {
+        unsigned long long v = __ldcg(&a.state[threadIdx.x]);
+        if (threadIdx.x == kDirectStart) {
+            unsigned long long t1;
+            asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t1));
+            v = t1 - v;
+        }
+        if (threadIdx.x == kDirectTicket) v = sorted ? 1 : 0;
+        a.host[threadIdx.x] = v;
+        a.state[threadIdx.x] = threadIdx.x == kDirectStart ? ~0ull : 0ull;
+    }
 }
 
 int64_t stripe_cap_for(int64_t n) {
@@ -805,6 +1004,28 @@ int enqueue_learned(cudaStream_t s, vs_context* ctx, const LearnedQuery& q, cons
     VS_CUDA_TRY(cudaMemsetAsync(sc.stripe_count, 0, (size_t)kStripes * sizeof(uint32_t), s));
     if (q.n_jobs > 1) return launch_passes<true>(s, ctx, a);
     return launch_passes<false>(s, ctx, a);
+}
+
+int launch_direct_join(vs_context* ctx, const vs_index* idx, const vs_points* pts, int accept_mask, int32_t* d_left,
+                       int32_t* d_right, int64_t capacity, bool sort) {
+    DirectArgs a{};
+    a.job = idx->learned.h_desc;
+    a.px = pts->d_x;
+    a.py = pts->d_y;
+    a.pvalid = pts->d_valid;
+    a.n = pts->n;
+    a.accept_mask = accept_mask;
+    a.state = ctx->d_direct;
+    a.host = ctx->h_counter;
+    a.sink = PairSink{d_left, d_right, (unsigned long long)(capacity > 0 ? capacity : 0), &a.state[kDirectPairs]};
+    a.sort = sort;
+    const bool bins = idx->n_split_binned_rings > 0;
+    auto* kernel = bins ? learned_direct_kernel<true> : learned_direct_kernel<false>;
+    // lanes for about four warps a scheduler
+    while (a.share < 5 && (pts->n << (a.share + 1)) <= (int64_t)kNumSMs * 512) ++a.share;
+    kernel<<<resident_grid(kernel, pts->n << a.share, kDirectThreads), kDirectThreads, 0, ctx->stream>>>(a);
+    VS_LAUNCHED("learned_direct", ctx->stream);
+    return VS_OK;
 }
 
 int launch_learned_join(vs_context* ctx, const vs_index* idx, const vs_points* pts, int accept_mask, int32_t* d_left,

@@ -21,6 +21,19 @@ int check_polygons(const vs_polygons* p);
 constexpr int kHostCounters = 16;
 constexpr int kDevCounters = 17;
 constexpr int kWorkCounter = 8;
+// Words of a context's direct-join state: 0-6 as the counters of a join, then
+// the blocks done and the start time.
+enum : int {
+    kDirectPairs = 0,
+    kDirectExact = 1,
+    kDirectFp32 = 2,
+    kDirectFp64 = 3,
+    kDirectCandidates = 5,
+    kDirectWide = 6,
+    kDirectTicket = 7,
+    kDirectStart = 8,
+    kDirectWords = 9
+};
 constexpr uint64_t kIndexPoolKeep = 1ull << 30;  // unused bytes the index pool keeps for the next build
 constexpr int kSortErr = 16;  // bit 1: a bounded wait of a pair sort gave up
 
@@ -144,6 +157,9 @@ struct vs_context {
     // [7] deferred pairs, [8] work queue of the refine kernel, [16] error
     // flags of the pair sort.
     unsigned long long* d_counters;
+    // State of the direct join (kDirect* words): zero, start all ones, between
+    // calls.
+    unsigned long long* d_direct;
     // Pairs deferred to the exact pass (grown on demand).
     int2* defer_buf;
     unsigned long long defer_cap;
