@@ -73,8 +73,8 @@ def polygon_index(ga, learned: bool = True, device: int = 0) -> "_abi.DeviceInde
 
 
 def join_pairs(points, polygons, predicate, *, method: str = "learned", device: int = 0,
-               on_device: bool = False):
-    """Sorted (point row, polygon row) pairs satisfying ``predicate`` (point on the left).
+               on_device: bool = False, sort: bool = True):
+    """(Point row, polygon row) pairs satisfying ``predicate`` (point on the left), sorted unless ``sort`` is off.
 
     Host intp arrays, or with ``on_device`` the int32 CUDA tensors the join
     wrote (no device-to-host copy).
@@ -90,7 +90,7 @@ def join_pairs(points, polygons, predicate, *, method: str = "learned", device: 
     index = polygon_index(polygons, learned=learned, device=device)
     pts, _ = device_points(points, device)
     m = _abi.METHOD_LEARNED if learned else (_abi.METHOD_BRUTE if method == "brute" else _abi.METHOD_RTREE)
-    left, right, _ = index.join(pts, code, m, sort=True)
+    left, right, _ = index.join(pts, code, m, sort=sort)
     if on_device:
         return left, right
     return left.cpu().numpy().astype(np.intp), right.cpu().numpy().astype(np.intp)

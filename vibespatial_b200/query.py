@@ -35,7 +35,7 @@ _nearest_backend = None
 _nearest_polygons_backend = None
 
 
-def _pairs(points, polygons, predicate, method, on_device=False):
+def _pairs(points, polygons, predicate, method, on_device=False, sort=True):
     if _pairs_backend is not None:
         left, right = _pairs_backend(points, polygons, predicate)
         if on_device:
@@ -46,7 +46,7 @@ def _pairs(points, polygons, predicate, method, on_device=False):
         return left, right
     from ._device import join_pairs
 
-    return join_pairs(points, polygons, predicate, method=method, on_device=on_device)
+    return join_pairs(points, polygons, predicate, method=method, on_device=on_device, sort=sort)
 
 
 def _dwithin(points, polygons, method, on_device=False, **dist):
@@ -135,7 +135,8 @@ def _query_device(tree, geometry, predicate, method):
         pred = _TREE_POINTS[predicate]
         if pred == "empty":
             return empty
-        pt, poly = _pairs(tree, geometry, pred, method, on_device=True)
+        # sorted once, by the input (polygon) rows
+        pt, poly = _pairs(tree, geometry, pred, method, on_device=True, sort=False)
         if poly.numel():
             from ._device import sort_pairs_on_device
 
