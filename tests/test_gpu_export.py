@@ -67,3 +67,36 @@ def test_export_rejects_out_of_range_pairs(ctx, vsabi):
         vsabi.join_export(ctx, l, r, 3, 2, "left", codes_l, codes_r)
     with pytest.raises(ValueError):
         vsabi.join_export(ctx, l[:2], r[:2] - 1, 3, 2, "inner", codes_l, codes_r)
+
+
+@pytest.mark.parametrize("how", ["left", "right", "outer"])
+def test_export_orders_unsorted_pairs(ctx, vsabi, how):
+    """Pairs that do not come sorted give the rows of the sorted ones, with their own source positions."""
+    import torch
+
+    rng = np.random.default_rng(5)
+    l, r = _pairs(rng, 9_000, 700, 20_000)
+    el, er, es = vs_sjoin._join_indexers(l, r, 9_000, 700, how, None)
+    mix = rng.permutation(len(l))
+    gl, gr, gs = (t.cpu().numpy() for t in vsabi.join_export(ctx, torch.from_numpy(l[mix]).cuda(),
+                                                             torch.from_numpy(r[mix]).cuda(), 9_000, 700, how))
+    np.testing.assert_array_equal(gl, el)
+    np.testing.assert_array_equal(gr, er)
+    np.testing.assert_array_equal(np.where(gs >= 0, mix[np.maximum(gs, 0)], -1), es)
+
+
+@pytest.mark.parametrize("n_pairs", [2047, 2048, 2049, 65_536, 200_003])
+def test_export_filter_tiles(ctx, vsabi, n_pairs):
+    """The one-pass attribute filter at the edges of its tiles of 2048 pairs."""
+    import torch
+
+    rng = np.random.default_rng(n_pairs)
+    l, r = _pairs(rng, 50_000, 3_000, n_pairs + n_pairs // 8)
+    l, r = l[:n_pairs], r[:n_pairs]
+    codes = (_codes(rng, 50_000, 3), _codes(rng, 3_000, 3))
+    el, er, es = vs_sjoin._join_indexers(l, r, 50_000, 3_000, "inner", codes)
+    dev = [torch.from_numpy(a).cuda() for a in (l, r, *codes)]
+    gl, gr, gs = vsabi.join_export(ctx, dev[0], dev[1], 50_000, 3_000, "inner", dev[2], dev[3])
+    np.testing.assert_array_equal(gl.cpu().numpy(), el)
+    np.testing.assert_array_equal(gr.cpu().numpy(), er)
+    np.testing.assert_array_equal(gs.cpu().numpy(), es)
