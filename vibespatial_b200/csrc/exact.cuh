@@ -313,6 +313,35 @@ __device__ __forceinline__ int geometry_location(double px, double py, const dou
     return LOC_OUTSIDE;
 }
 
+// The same with the FP32 boxes of the rings (relative to the polygon's origin
+// o; err bounds the vertices' rounding): a ring whose box lies strictly beyond
+// the point neither holds it nor crosses its +x ray an odd number of times, so
+// its walk would change nothing.
+__device__ __forceinline__ int geometry_location_boxed(double px, double py, const double2* __restrict__ xy,
+                                                       const int32_t* __restrict__ ring_off,
+                                                       const int32_t* __restrict__ part_off,
+                                                       const int32_t* __restrict__ geom_off, int g,
+                                                       const RingIndex& ri, const double2 o, float err,
+                                                       const float4* __restrict__ ring_box, unsigned& n_exact) {
+    const float sx = __double2float_rn(px - o.x), sy = __double2float_rn(py - o.y);
+    const float t = __fmul_ru(__fadd_ru(err, __fmaf_ru(fmaxf(fabsf(sx), fabsf(sy)), 6.1e-8f, 1e-37f)), 1.0001f);
+    const int p0 = geom_off[g], p1 = geom_off[g + 1];
+    for (int part = p0; part < p1; ++part) {
+        bool inside = false;
+        const int r0 = part_off[part], r1 = part_off[part + 1];
+        for (int ring = r0; ring < r1; ++ring) {
+            const float4 b = ring_box[ring];
+            if (__fadd_ru(sx, t) < b.x || __fsub_rd(sx, t) > b.z || __fadd_ru(sy, t) < b.y || __fsub_rd(sy, t) > b.w)
+                continue;
+            const int k = ring_location(px, py, xy, ring_off[ring], ring_off[ring + 1], ring, ri, n_exact);
+            if (k == LOC_BOUNDARY) return LOC_BOUNDARY;
+            if (k == LOC_INTERIOR) inside = !inside;
+        }
+        if (inside) return LOC_INTERIOR;
+    }
+    return LOC_OUTSIDE;
+}
+
 __device__ __forceinline__ int geometry_location_soa(double px, double py, const double* __restrict__ x,
                                                      const double* __restrict__ y,
                                                      const int32_t* __restrict__ ring_off,
