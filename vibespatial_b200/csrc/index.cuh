@@ -83,7 +83,8 @@ struct LearnedJob {
     double lox, loy, hix, hiy, sx, sy;
     double cwx, cwy;     // level-L cell width per axis (cell_anchor)
     int32_t L;
-    int32_t occ_shift;   // cell key >> occ_shift = occupancy bit
+    int32_t occ_shift;   // occupancy bitmap in key order: cell key >> occ_shift = bit
+    int32_t occ_rows;    // its grid level where it is in row order instead (occ_bit), else -1
     int32_t root_shift;  // cell key >> root_shift = root-table index
     uint32_t cell_base;
     int64_t n_cells;
@@ -126,6 +127,12 @@ constexpr uint32_t kLearnedNoInterior = 8u;  // every box candidate is ring-walk
 __device__ __forceinline__ double cell_anchor(double lo, double cw, uint32_t c) {
     return __fma_rn((double)c + 0.5, cw, lo);
 }
+
+// Bit of grid cell (cx, cy) in a row-order occupancy bitmap of the given level.
+// Sparse indexes (sparse_map_pays) have such a bitmap: most points miss, and
+// end there, so the bit is to be had without a Hilbert key.  Where most points
+// need their key in any case, a bitmap in key order takes fewer steps.
+__device__ __forceinline__ uint32_t occ_bit(uint32_t cx, uint32_t cy, int level) { return (cy << level) | cx; }
 
 struct LearnedIndex {
     int32_t level = 0;               // grid level L (cells of frame / 2^L per axis)

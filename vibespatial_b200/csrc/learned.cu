@@ -144,9 +144,16 @@ __global__ void cell_compact_kernel(const uint32_t* __restrict__ keys, const uin
     }
 }
 
-__global__ void occ_kernel(const uint32_t* __restrict__ cell_keys, int64_t n, int shift, uint32_t* __restrict__ occ) {
+// Occupancy of the level-`level` grid (level <= L), in key or in row order.
+__global__ void occ_kernel(const uint32_t* __restrict__ cell_keys, int64_t n, int L, int level, bool rows,
+                           uint32_t* __restrict__ occ) {
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const uint32_t b = cell_keys[i] >> shift;
+        uint32_t b = cell_keys[i] >> (2 * (L - level));
+        if (rows) {
+            uint32_t cx, cy;
+            hilbert_cell(cell_keys[i], L, cx, cy);
+            b = occ_bit(cx >> (L - level), cy >> (L - level), level);
+        }
         atomicOr(&occ[b >> 5], 1u << (b & 31));
     }
 }
@@ -1082,7 +1089,8 @@ int build_learned_index(vs_context* ctx, vs_index* idx, const vs_index_options* 
     const int64_t occ_bits = 1ll << (2 * li.occ_level);
     VS_TRY(dalloc(&li.occ, (size_t)((occ_bits + 31) / 32), bytes, ctx));
     VS_CUDA_TRY(cudaMemsetAsync(li.occ, 0, (size_t)((occ_bits + 31) / 32) * sizeof(uint32_t), s));
-    occ_kernel<<<grid_for(nc, 256), 256, 0, s>>>(li.cell_keys, nc, 2 * (L - li.occ_level), li.occ);
+    const bool occ_rows = sparse_map_pays(nc, 1ll << (2 * L));
+    occ_kernel<<<grid_for(nc, 256), 256, 0, s>>>(li.cell_keys, nc, L, li.occ_level, occ_rows, li.occ);
     VS_CUDA_TRY(cudaGetLastError());
     // 5. RMI (root tabulated over level-R ancestors)
     // leaves: 4096, or one per 64 stored keys (to the next power of two, at
@@ -1108,6 +1116,7 @@ int build_learned_index(vs_context* ctx, vs_index* idx, const vs_index_options* 
     LearnedJob d{};
     d.L = L;
     d.occ_shift = 2 * (L - li.occ_level);
+    d.occ_rows = occ_rows ? li.occ_level : -1;
     d.root_shift = 2 * (L - li.root_level);
     d.cell_base = 0;
     d.n_cells = li.n_cells;

@@ -35,10 +35,20 @@ struct LearnedQuery {
     const int64_t* job_start;
     int64_t n_cells;  // batch-wide cells
     int accept_mask;
+    bool sparse;         // every job's index is sparse (its occupancy bitmap is in row order)
     bool has_ring_bins;  // some job's index has y-binned rings long enough for the split walk
     int64_t row_base;    // added to every emitted / deferred point row (chunked joins)
     LearnedShape shape;  // launch shape and ablation switches (zero = defaults)
 };
+
+// Does the map pass that queues its hits pay for an index that stores n_cells of
+// its grid's grid_cells cells?  The share of points that hit is not known
+// before the pass; the stored share of the grid stands for it.  10M points,
+// us with and without: clustered footprints, share 0.004: 70 and 120, 0.021: 84
+// and 158, 0.073: 145 and 162, 0.15: 213 and 189; points where the footprints
+// are (most hit), share 0.010: 85 and 165, 0.037: 134 and 173, 0.082: 198 and
+// 184; a full grid (0.90): 266 and 229.
+inline bool sparse_map_pays(int64_t n_cells, int64_t grid_cells) { return n_cells < grid_cells / 16; }
 
 // Enqueue map -> scan -> place -> refine on stream s (no host
 // synchronisation; capturable).  For one job, `single` is its descriptor

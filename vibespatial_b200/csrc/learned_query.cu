@@ -4,8 +4,9 @@
 // Three passes over the points (a counting sort keyed by the learned index's
 // own positions, so no general sort is needed):
 //   map      input order: the point's job (batch) -> level-L cell key ->
-//            occupancy bit -> root table -> leaf model -> binary search inside
-//            the leaf's error window -> cell index (or none); the per-cell
+//            occupancy bit (of a sparse index: before the key) -> root table
+//            -> leaf model -> binary search inside the
+//            leaf's error window -> cell index (or none); the per-cell
 //            counts are incremented, and every matched point is appended to
 //            a striped staging region as one 16-byte CellPoint: its FP32
 //            offsets from the cell's anchor, its row and its cell
@@ -44,9 +45,10 @@ namespace {
 constexpr int kThreads = 256;
 
 // The map pass appends matched points to kStripes regions of the staging
-// array, region s taking the packets p with p % kStripes == s, so each
+// array, region s taking the units u of unit_packets() consecutive packets (or,
+// in the pass for dense indexes, the packets) with u % kStripes == s, so each
 // region's append counter sees 1/kStripes of the atomics and a region never
-// holds more than 32 * ceil(packets / kStripes) points.
+// holds more than the points of ceil(units / kStripes) units.
 constexpr int kStripes = 2048;
 
 // A (point, candidate) pair that passed the FP32 box filter, queued for the
@@ -67,6 +69,7 @@ struct LqArgs {
     LearnedJob single;  // the one job of a single join (kernel parameter space)
     CellPoint* staged;
     uint32_t* stripe_count;
+    uint32_t* map_work;        // units of the sparse map pass handed out
     int64_t stripe_cap;
     uint32_t* cell_count;
     CellPoint* grouped;
@@ -256,19 +259,31 @@ __device__ __forceinline__ int geometry_location_split(float qx, float qy, float
 }
 
 // ---------------------------------------------------------------- map ---
-// Exact lookup of a level-L cell key in job J's learned index: occupancy bit
-// -> root table -> leaf model -> binary search inside the leaf's error window.  Returns the cell's
+// May job J's index store the cell of a point at (gx, gy) (32-bit grid
+// coordinates)?  False: no stored cell matches.  The bitmap is in row order.
+__device__ __forceinline__ bool learned_occupied_rows(const LearnedJob& J, uint32_t gx, uint32_t gy) {
+    const int sh = 32 - J.occ_rows;
+    const uint32_t ob = occ_bit(gx >> sh, gy >> sh, J.occ_rows);
+    return (J.occ[ob >> 5] >> (ob & 31)) & 1u;
+}
+
+// The same for either order; cell is the point's level-L cell key.
+__device__ __forceinline__ bool learned_occupied(const LearnedJob& J, uint32_t gx, uint32_t gy, uint32_t cell) {
+    if (J.occ_rows >= 0) return learned_occupied_rows(J, gx, gy);
+    const uint32_t ob = cell >> J.occ_shift;
+    return (J.occ[ob >> 5] >> (ob & 31)) & 1u;
+}
+
+// Exact lookup of a level-L cell key in job J's learned index: root table ->
+// leaf model -> binary search inside the leaf's error window.  Returns the cell's
 // index, or -1 when no stored cell matches (no polygon box overlaps it).
 // kBsearch (an ablation): the model is skipped and the search covers every
 // stored key.
 template <bool kBsearch>
-__device__ __forceinline__ int learned_lookup(const LearnedJob& J, uint32_t cell, unsigned long long& n_wide) {
-    const uint32_t ob = cell >> J.occ_shift;
-    // the occupancy word and the root-table entry depend only on the key:
-    // both loads are issued before either is tested
-    const uint32_t occ_word = J.occ[ob >> 5];
+__device__ __forceinline__ int learned_lookup(const LearnedJob& J, uint32_t cell, unsigned long long& n_wide,
+                                              bool occupied = true) {
     const uint32_t leaf_id = kBsearch ? 0u : (uint32_t)J.root_table[cell >> J.root_shift];
-    if (!((occ_word >> (ob & 31)) & 1u)) return -1;
+    if (!occupied) return -1;  // (tested here: the two loads do not wait for one another)
     // search [l0, h0) with 32-bit indices (a cell count fits in 31 bits)
     int l0 = 0, h0 = (int)J.n_cells;
     if constexpr (!kBsearch) {
@@ -305,6 +320,55 @@ __device__ __forceinline__ int packet_job(const LearnedQuery& q, int64_t b0, int
     return j;
 }
 
+// A point that passed the occupancy test, waiting for its lookup.
+struct PendingPoint {
+    double x, y;
+    uint32_t at;   // position in its unit
+    int32_t job;
+};
+
+// The sparse map pass takes units of consecutive packets of 32 points, at most
+// eight: they let a warp fill whole lookups from sparse hits, and every unit
+// costs an increment of the one counter they are handed out from (about 1 ns,
+// measured: 10M points in units of two packets took 149 us, of eight 83 us).
+// Fewer points make smaller units, so that a warp still gets several.
+__host__ __device__ __forceinline__ int unit_packets(int64_t n) {
+    const int64_t packets = (n + 31) / 32;
+    return packets >= 8 * 32 * 1024 ? 8 : packets >= 4 * 16 * 1024 ? 4 : packets >= 2 * 16 * 1024 ? 2 : 1;
+}
+
+// Look up to 32 pending points up, count their cells and append the matched
+// ones to the unit's staging region.  Whole warp, converged.
+template <bool kMulti>
+__device__ __forceinline__ void map_pending(const LqArgs& a, const PendingPoint* pend, int cnt, int64_t unit,
+                                            int64_t unit0, const uint16_t* lut, unsigned long long& n_wide) {
+    const int lane = threadIdx.x & 31;
+    int gc = -1;
+    CellPoint p{0.f, 0.f, 0, 0u};
+    if (lane < cnt) {
+        const PendingPoint e = pend[lane];
+        const LearnedJob& J = job_desc<kMulti>(a, e.job);
+        const uint32_t gx = quantize(e.x, J.lox, J.sx), gy = quantize(e.y, J.loy, J.sy);
+        const int c = learned_lookup<false>(J, hilbert_key_lut(gx, gy, J.L, lut), n_wide);
+        if (c >= 0) {
+            const int sh = 32 - J.L;
+            gc = (int)(J.cell_base + (uint32_t)c);
+            p.qx = __double2float_rn(__dsub_rn(e.x, cell_anchor(J.lox, J.cwx, gx >> sh)));
+            p.qy = __double2float_rn(__dsub_rn(e.y, cell_anchor(J.loy, J.cwy, gy >> sh)));
+            p.row = (int32_t)(unit0 + e.at + a.q.row_base);
+            p.gcell = (uint32_t)gc;
+            atomicAdd(&a.cell_count[gc], 1u);
+        }
+    }
+    const unsigned mm = __ballot_sync(0xffffffffu, gc >= 0);
+    if (!mm) return;
+    const int64_t stripe = unit % kStripes;
+    uint32_t sb = 0;
+    if (lane == 0) sb = atomicAdd(&a.stripe_count[stripe], (uint32_t)__popc(mm));
+    sb = __shfl_sync(0xffffffffu, sb, 0);
+    if (gc >= 0) store_stream(&a.staged[stripe * a.stripe_cap + sb + __popc(mm & ((1u << lane) - 1u))], p);
+}
+
 // One point of the map pass: its batch-wide cell (-1: none) and its FP32
 // offsets from the cell's anchor (|offset| <= half a cell).
 template <bool kMulti, bool kBsearch>
@@ -318,7 +382,8 @@ __device__ __forceinline__ int map_point(const LqArgs& a, int64_t i, int job, co
           y <= J.hiy))
         return -1;
     const uint32_t gx = quantize(x, J.lox, J.sx), gy = quantize(y, J.loy, J.sy);
-    const int c = learned_lookup<kBsearch>(J, hilbert_key_lut(gx, gy, J.L, lut), n_wide);
+    const uint32_t cell = hilbert_key_lut(gx, gy, J.L, lut);
+    const int c = learned_lookup<kBsearch>(J, cell, n_wide, learned_occupied(J, gx, gy, cell));
     if (c < 0) return -1;
     const int sh = 32 - J.L;
     qx = __double2float_rn(__dsub_rn(x, cell_anchor(J.lox, J.cwx, gx >> sh)));
@@ -374,6 +439,85 @@ __global__ void __launch_bounds__(kThreads, kPackets == 1 ? 8 : 6) learned_map_k
         }
 #pragma unroll
         for (int u = 0; u < kPackets; ++u) map_emit(a, b0 + 32 * u, lane, gc[u], qx[u], qy[u]);
+    }
+    add_counter(a.counters, 6, n_wide);
+}
+
+// The map pass for sparse indexes, points in input order, a unit a warp at a
+// time: each point's occupancy bit, then, for the points whose cell may be
+// stored, queued in shared memory so that every lane has one, the cell lookup,
+// the per-cell counts and the staged CellPoints.  Two packets' coordinates and
+// bits are in flight together.
+//
+// Bound by the latency of its dependent loads (coordinates, bit): 10M points
+// against 100k footprints, whose cells are 2% of the grid, 83 us for 160 MB of
+// coordinates; with a key and a lookup per lane as the points come, 155 us.
+template <bool kMulti>
+__global__ void __launch_bounds__(kThreads, 5) learned_map_sparse_kernel(const LqArgs a) {
+    __shared__ uint16_t s_lut[kHilbertLutSize];
+    __shared__ PendingPoint s_pend[kThreads / 32][64];
+    hilbert_lut_init(s_lut);
+    __syncthreads();
+    const LearnedQuery& q = a.q;
+    unsigned long long n_wide = 0;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned lt = (1u << lane) - 1u;
+    PendingPoint* pend = s_pend[warp];
+    const int64_t unit_points = 32 * (int64_t)unit_packets(q.n);
+    constexpr int kTogether = 2;
+    // Warp-uniform loops: the whole warp reaches the ballots and shuffles together.
+    for (;;) {
+        uint32_t unit = 0;
+        if (lane == 0) unit = atomicAdd(a.map_work, 1u);
+        unit = __shfl_sync(0xffffffffu, unit, 0);
+        if (unit * unit_points >= q.n) break;
+        const int64_t unit0 = unit * unit_points;
+        const int64_t end = unit0 + unit_points < q.n ? unit0 + unit_points : q.n;
+        int np = 0;  // warp-uniform
+        for (int64_t b0 = unit0; b0 < end; b0 += 32 * kTogether) {
+            double x[kTogether], y[kTogether];
+            bool hit[kTogether];
+            int job[kTogether];
+#pragma unroll
+            for (int u = 0; u < kTogether; ++u) {
+                const int64_t i = b0 + 32 * u + lane;
+                x[u] = y[u] = 0.0;
+                hit[u] = i < end && (q.pvalid == nullptr || q.pvalid[i]);
+                if (i < end) {
+                    x[u] = __ldcs(q.px + i);
+                    y[u] = __ldcs(q.py + i);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < kTogether; ++u) {
+                const int64_t bu = b0 + 32 * u;
+                job[u] = packet_job<kMulti>(q, bu < q.n ? bu : b0, bu + lane, lane);
+                const LearnedJob& J = job_desc<kMulti>(a, job[u]);
+                hit[u] = hit[u] && J.n_cells > 0 && x[u] >= J.lox && x[u] <= J.hix && y[u] >= J.loy && y[u] <= J.hiy;
+                if (hit[u])
+                    hit[u] = learned_occupied_rows(J, quantize(x[u], J.lox, J.sx), quantize(y[u], J.loy, J.sy));
+            }
+#pragma unroll
+            for (int u = 0; u < kTogether; ++u) {
+                const unsigned m = __ballot_sync(0xffffffffu, hit[u]);
+                if (hit[u])
+                    pend[np + __popc(m & lt)] =
+                        PendingPoint{x[u], y[u], (uint32_t)(b0 - unit0) + 32 * u + lane, job[u]};
+                np += __popc(m);
+                __syncwarp();
+                if (np >= 32) {
+                    map_pending<kMulti>(a, pend, 32, unit, unit0, s_lut, n_wide);
+                    __syncwarp();
+                    if (lane < np - 32) pend[lane] = pend[32 + lane];
+                    np -= 32;
+                    __syncwarp();
+                }
+            }
+        }
+        if (np > 0) {
+            map_pending<kMulti>(a, pend, np, unit, unit0, s_lut, n_wide);
+            __syncwarp();
+        }
     }
     add_counter(a.counters, 6, n_wide);
 }
@@ -788,7 +932,8 @@ __global__ void __launch_bounds__(kDirectThreads) learned_direct_kernel(const Di
                 y <= J.hiy) {
                 const uint32_t gx = quantize(x, J.lox, J.sx), gy = quantize(y, J.loy, J.sy);
                 unsigned long long wide = 0;
-                const int c = learned_lookup<false>(J, (uint32_t)hilbert_key(gx, gy, J.L), wide);
+                const uint32_t cell = (uint32_t)hilbert_key(gx, gy, J.L);
+                const int c = learned_lookup<false>(J, cell, wide, learned_occupied(J, gx, gy, cell));
                 n_wide += sub == 0 ? wide : 0;
                 if (c >= 0) {
                     const int sh = 32 - J.L;
@@ -887,8 +1032,8 @@ __global__ void __launch_bounds__(kDirectThreads) learned_direct_kernel(const Di
 }
 
 int64_t stripe_cap_for(int64_t n) {
-    const int64_t packets = (n + 31) / 32;
-    return 32 * ((packets + kStripes - 1) / kStripes);
+    const int64_t points = 32 * (int64_t)unit_packets(n), units = (n + points - 1) / points;
+    return points * ((units + kStripes - 1) / kStripes);
 }
 
 size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
@@ -897,7 +1042,7 @@ size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 
 size_t learned_scratch_bytes(int64_t n, int64_t n_cells) {
     const int64_t cap = stripe_cap_for(n);
-    return align256(sizeof(CellPoint) * (size_t)(kStripes * cap)) + align256(sizeof(uint32_t) * kStripes) +
+    return align256(sizeof(CellPoint) * (size_t)(kStripes * cap)) + align256(sizeof(uint32_t) * (kStripes + 1)) +
            align256(sizeof(uint32_t) * (size_t)(n_cells > 0 ? n_cells : 1)) +
            align256(sizeof(CellPoint) * (size_t)(n > 0 ? n : 1)) + align256(sizeof(uint32_t));
 }
@@ -908,7 +1053,7 @@ void learned_scratch_carve(void* base, int64_t n, int64_t n_cells, LearnedScratc
     sc.staged = p;
     p += align256(sizeof(CellPoint) * (size_t)(kStripes * sc.stripe_cap));
     sc.stripe_count = (uint32_t*)p;
-    p += align256(sizeof(uint32_t) * kStripes);
+    p += align256(sizeof(uint32_t) * (kStripes + 1));
     sc.cell_count = (uint32_t*)p;
     p += align256(sizeof(uint32_t) * (size_t)(n_cells > 0 ? n_cells : 1));
     sc.grouped = p;
@@ -952,6 +1097,8 @@ int launch_passes(cudaStream_t s, vs_context* ctx, const LqArgs& a) {
     if (sh.flags & kLearnedBsearch) {
         if (two) learned_map_kernel<kMulti, true, 2><<<map_grid, kThreads, 0, s>>>(a);
         else learned_map_kernel<kMulti, true, 1><<<map_grid, kThreads, 0, s>>>(a);
+    } else if (a.q.sparse && sh.map_packets == 0) {
+        learned_map_sparse_kernel<kMulti><<<map_grid, kThreads, 0, s>>>(a);
     } else {
         if (two) learned_map_kernel<kMulti, false, 2><<<map_grid, kThreads, 0, s>>>(a);
         else learned_map_kernel<kMulti, false, 1><<<map_grid, kThreads, 0, s>>>(a);
@@ -989,6 +1136,7 @@ int enqueue_learned(cudaStream_t s, vs_context* ctx, const LearnedQuery& q, cons
     if (single) a.single = *single;
     a.staged = (CellPoint*)sc.staged;
     a.stripe_count = sc.stripe_count;
+    a.map_work = sc.stripe_count + kStripes;
     a.stripe_cap = sc.stripe_cap;
     a.cell_count = sc.cell_count;
     a.grouped = (CellPoint*)sc.grouped;
@@ -1001,7 +1149,7 @@ int enqueue_learned(cudaStream_t s, vs_context* ctx, const LearnedQuery& q, cons
     a.no_stage = (q.shape.flags & kLearnedNoStage) != 0;
     a.no_interior = (q.shape.flags & kLearnedNoInterior) != 0;
     VS_CUDA_TRY(cudaMemsetAsync(sc.cell_count, 0, (size_t)(q.n_cells > 0 ? q.n_cells : 1) * sizeof(uint32_t), s));
-    VS_CUDA_TRY(cudaMemsetAsync(sc.stripe_count, 0, (size_t)kStripes * sizeof(uint32_t), s));
+    VS_CUDA_TRY(cudaMemsetAsync(sc.stripe_count, 0, (size_t)(kStripes + 1) * sizeof(uint32_t), s));
     if (q.n_jobs > 1) return launch_passes<true>(s, ctx, a);
     return launch_passes<false>(s, ctx, a);
 }
@@ -1048,6 +1196,7 @@ int launch_learned_join(vs_context* ctx, const vs_index* idx, const vs_points* p
     q.n_cells = li.n_cells;
     q.accept_mask = accept_mask;
     q.has_ring_bins = idx->n_split_binned_rings > 0;
+    q.sparse = li.h_desc.occ_rows >= 0;
     q.row_base = row_base;
     q.shape = shape;
     const PairSink sink{d_left, d_right, (unsigned long long)(capacity > 0 ? capacity : 0), &ctx->d_counters[0]};
