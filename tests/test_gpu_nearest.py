@@ -1,0 +1,58 @@
+"""Nearest joins where the single walk's tie list (six entries a point, six a
+polygon) is full, one short or overflows into the two-walk path; and points as
+far away as the FP32 bounds reach."""
+import numpy as np
+import pytest
+
+from test_gpu_distance import _device, _oracle_polys, syn
+
+pytestmark = pytest.mark.gpu
+
+
+def _copies(k, seed):
+    """300 stars, each present k times: every nearest distance has at least k polygons."""
+    w = syn.star_join(seed=seed, n_points=3_000, n_polys=300)
+    p = w.polys
+    xs, ys, sizes = [], [], []
+    for _ in range(k):
+        for a, b in zip(p.ring_off[:-1], p.ring_off[1:]):
+            xs.append(p.x[a:b])
+            ys.append(p.y[a:b])
+            sizes.append(b - a)
+    polys = syn._rings_to_soa(np.array(sizes), np.concatenate(xs), np.concatenate(ys))
+    px = np.concatenate([w.px, [1e12, -1e30, 1e30, np.nan, np.inf]])
+    py = np.concatenate([w.py, [-3.0, 1e30, 0.5, 0.5, -np.inf]])
+    return syn.Workload(name="copies", px=px, py=py, polys=polys)
+
+
+@pytest.mark.parametrize("k", [1, 5, 6, 7, 13])
+def test_ties_around_the_list_size(ctx, vsabi, oracle, k):
+    w = _copies(k, seed=k)
+    index, pts, keep = _device(vsabi, ctx, w)
+    P = _oracle_polys(oracle, w)
+    for md in (np.inf, 0.0, 0.01):
+        el, er, ed = oracle.nearest_join(w.px, w.py, None, P, md)
+        gl, gr, gd, _ = index.nearest(pts, max_distance=md)
+        np.testing.assert_array_equal(gl.cpu().numpy(), el)
+        np.testing.assert_array_equal(gr.cpu().numpy(), er)
+        np.testing.assert_array_equal(gd.cpu().numpy().view(np.int64), ed.view(np.int64))
+
+
+@pytest.mark.parametrize("k", [1, 5, 6, 7, 13])
+def test_equal_points_around_the_list_size(ctx, vsabi, oracle, k):
+    import torch
+
+    w = _copies(1, seed=20 + k)
+    px, py = np.tile(w.px[:-5], k), np.tile(w.py[:-5], k)
+    dx, dy = torch.from_numpy(px).cuda(), torch.from_numpy(py).cuda()
+    pidx = vsabi.point_index(ctx, dx, dy)
+    p = w.polys
+    t = [torch.from_numpy(np.ascontiguousarray(getattr(p, a))).cuda()
+         for a in ("x", "y", "ring_off", "part_off", "geom_off")]
+    P = vsabi.make_polygons(*t)
+    for md in (np.inf, 0.0, 0.01):
+        el, er, ed = oracle.nearest_polygons_join(px, py, None, _oracle_polys(oracle, w), md)
+        gl, gr, gd, _ = vsabi.nearest_polygons(ctx, pidx, P, max_distance=md)
+        np.testing.assert_array_equal(gl.cpu().numpy(), el)
+        np.testing.assert_array_equal(gr.cpu().numpy(), er)
+        np.testing.assert_array_equal(gd.cpu().numpy().view(np.int64), ed.view(np.int64))

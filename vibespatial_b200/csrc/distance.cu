@@ -30,15 +30,17 @@
 // radius (rounded outward, plus a relative 2^-30 margin, so no polygon within
 // the radius can be missed); the exact test above decides every candidate.
 //
-// Nearest (all ties), two walks.  The first finds each point's minimum: a
-// greedy descent per point (at every level the child box nearest to the
-// point, then the nearest item box) gives an upper bound; the walk then
-// visits, nearest first, only what lies within each point's current minimum
-// (capped by max_distance) -- a polygon nearer than the minimum is always
-// inside that box -- and the packet's box shrinks as the minima drop.  The
-// second walk emits every polygon at exactly the minimum.
-// Candidates whose envelope is certainly farther than the bound are skipped
-// before the exact distance.
+// Nearest (all ties), one walk (near_kernel, poly_near_kernel): a greedy
+// descent per query (at every level the child box nearest to it) gives an
+// upper bound; the walk visits, nearest first, what lies within the queries'
+// current bounds (capped by max_distance), bounds every item's distance from
+// both sides in FP32 and lists the few items that may still be the nearest.
+// Exact distances are computed for the listed items only and decide.
+// Queries whose list overflows, or that FP32 cannot hold, take two exact
+// walks: the first finds the query's minimum (a polygon nearer than the
+// minimum is always inside its box), the second emits every polygon at
+// exactly the minimum.  There, candidates whose envelope is certainly farther
+// than the bound are skipped before the exact distance.
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
