@@ -383,7 +383,10 @@ __global__ void pack_leaves_kernel(int nl, const double2* __restrict__ ab, const
 // spread over the keys), full-batch mean squared error, Adam.
 //
 // Two lanes share two samples, each taking half of the layer-2 units of both
-// (the weights come from shared memory, whose bandwidth bounds the products).
+// (the weights come from shared memory, whose bandwidth bounds the products:
+// the two lanes read rows two apart of a copy whose rows start four banks
+// apart, which took a step from 9.6 to 8.6 us; four lanes a pair of samples
+// and twice the warps: 8.7).
 // The block's 128 samples' activations go to shared memory, where each warp
 // forms the weight gradients of its 32 samples as a
 // 32 x 32 outer-product sum (a lane owns 4 x 8 of it).  The blocks add their
@@ -418,6 +421,7 @@ struct TrainShared {
     float P[kGradWords];                      // weights (kOff*)
     float m1[kRmiP], m2[kRmiP];               // Adam moments
     float pad[2];
+    float w2[kRmiHidden][kTrainStride];       // the layer-2 weights again, rows apart in the banks
     float h1[kTrainThreads][kTrainStride];    // layer-1 outputs
     float d2[kTrainThreads][kTrainStride];    // layer-2 errors
     float h2[kTrainThreads][kTrainStride];    // layer-2 outputs times the output error
@@ -475,10 +479,11 @@ __global__ void __launch_bounds__(kTrainThreads) rmi_train_kernel(const TrainArg
         sm.P[kOffW1 + tid] = 1.0f;
         sm.P[kOffB1 + tid] = (float)-((sm.knot[tid] - key_lo) * key_scale);
         sm.P[kOffW2 + tid * kRmiHidden + tid] = 1.0f;
+        for (int k = 0; k < kRmiHidden; ++k) sm.w2[tid][k] = k == tid ? 1.0f : 0.f;
         sm.P[kOffW3 + tid] = (float)(slope(tid) - slope(tid - 1));
     }
     // Two neighbouring lanes share two samples; each takes half of the layer-2 units
-    const int half = tid & 1, row0 = tid - half, j0 = half * (kRmiHidden / 2);
+    const int half = tid & 1, row0 = tid - half;
     bool live[2];
     float x[2], t[2];
 #pragma unroll
@@ -502,16 +507,18 @@ __global__ void __launch_bounds__(kTrainThreads) rmi_train_kernel(const TrainArg
         // layer-2 units, so that a weight read from shared memory serves two
         f32x2 h1[2][kRmiHidden / 2];
 #pragma unroll
-        for (int k = 0; k < kRmiHidden; k += 2) {
-            const float w0 = sm.P[kOffW1 + k], w1 = sm.P[kOffW1 + k + 1];
-            const float c0 = sm.P[kOffB1 + k], c1 = sm.P[kOffB1 + k + 1];
+        for (int k = 0; k < kRmiHidden; k += 4) {
+            const float4 w = *reinterpret_cast<const float4*>(&sm.P[kOffW1 + k]);
+            const float4 c = *reinterpret_cast<const float4*>(&sm.P[kOffB1 + k]);
 #pragma unroll
-            for (int q = 0; q < 2; ++q)
-                h1[q][k / 2] = pack2(fmaxf(fmaf(w0, x[q], c0), 0.f), fmaxf(fmaf(w1, x[q], c1), 0.f));
+            for (int q = 0; q < 2; ++q) {
+                h1[q][k / 2] = pack2(fmaxf(fmaf(w.x, x[q], c.x), 0.f), fmaxf(fmaf(w.y, x[q], c.y), 0.f));
+                h1[q][k / 2 + 1] = pack2(fmaxf(fmaf(w.z, x[q], c.z), 0.f), fmaxf(fmaf(w.w, x[q], c.w), 0.f));
+            }
         }
         float y[2] = {0.f, 0.f};
 #pragma unroll 1
-        for (int j = j0; j < j0 + kRmiHidden / 2; j += 2) {
+        for (int j = 2 * half; j < kRmiHidden; j += 4) {
             float h2[2][2];
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
@@ -523,7 +530,7 @@ __global__ void __launch_bounds__(kTrainThreads) rmi_train_kernel(const TrainArg
                 }
 #pragma unroll
                 for (int k = 0; k < kRmiHidden; k += 4) {
-                    const ulonglong2 w = load4(&sm.P[kOffW2 + (j + u) * kRmiHidden + k]);
+                    const ulonglong2 w = load4(&sm.w2[j + u][k]);
 #pragma unroll
                     for (int q = 0; q < 2; ++q) {
                         za[q] = fma2(w.x, h1[q][k / 2], za[q]);
@@ -562,7 +569,7 @@ __global__ void __launch_bounds__(kTrainThreads) rmi_train_kernel(const TrainArg
             *reinterpret_cast<ulonglong2*>(&sm.h1[tid][2 * k]) =
                 half ? make_ulonglong2(h1[1][k], h1[1][k + 1]) : make_ulonglong2(h1[0][k], h1[0][k + 1]);
 #pragma unroll 1
-        for (int j = j0; j < j0 + kRmiHidden / 2; j += 2) {
+        for (int j = 2 * half; j < kRmiHidden; j += 4) {
             float d[2][2], g2[2][2];
 #pragma unroll
             for (int q = 0; q < 2; ++q) {
@@ -577,7 +584,7 @@ __global__ void __launch_bounds__(kTrainThreads) rmi_train_kernel(const TrainArg
                 const f32x2 d0 = pack2(d[0][u], d[0][u]), d1 = pack2(d[1][u], d[1][u]);
 #pragma unroll
                 for (int k = 0; k < kRmiHidden; k += 4) {
-                    const ulonglong2 w = load4(&sm.P[kOffW2 + (j + u) * kRmiHidden + k]);
+                    const ulonglong2 w = load4(&sm.w2[j + u][k]);
                     dh[0][k / 2] = fma2(w.x, d0, dh[0][k / 2]);
                     dh[0][k / 2 + 1] = fma2(w.y, d0, dh[0][k / 2 + 1]);
                     dh[1][k / 2] = fma2(w.x, d1, dh[1][k / 2]);
@@ -710,7 +717,10 @@ __global__ void __launch_bounds__(kTrainThreads) rmi_train_kernel(const TrainArg
             const float v = b2 * sm.m2[i] + (1.f - b2) * g[u] * g[u];
             sm.m1[i] = m;
             sm.m2[i] = v;
-            sm.P[i] -= lr * (m / c1) / (sqrtf(v / c2) + 1e-8f);
+            const float p = sm.P[i] - lr * (m / c1) / (sqrtf(v / c2) + 1e-8f);
+            sm.P[i] = p;
+            const int k = i - kOffW2;
+            if (k >= 0 && k < kRmiHidden * kRmiHidden) sm.w2[k / kRmiHidden][k % kRmiHidden] = p;
         }
         if (blockIdx.x == 0 && tid == 0 && step == a.steps) *a.loss = __ldcg(grad + kLossWord);
         __syncthreads();
