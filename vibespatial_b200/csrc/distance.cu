@@ -1125,8 +1125,9 @@ int finish_join(vs_context* ctx, const vs_index* idx, const vs_points* pts, uint
 // Nearest points of every polygon (all ties).  The tree is an index over the
 // points, each point a one-vertex polygon, so a level-0 box is the point
 // itself; the queries are the polygons, in the Hilbert order of their
-// envelope centres.  Same two walks as the point queries: a greedy bound, a
-// nearest-first walk that keeps each lane's minimum, then the ties.
+// envelope centres.  poly_near_kernel (below) answers most of them in one
+// walk.  The rest take the same two walks as the point queries' rest: a greedy
+// bound, a nearest-first walk that keeps each lane's minimum, then the ties.
 
 struct PolyArgs {
     const double* x;  // query polygons, original rows

@@ -1,6 +1,6 @@
 // Exclusive scan (reduce -> scan of block sums -> downsweep) and a stable
 // LSD radix sort of (u32/u64 key, u32 value) items or (left, right) pairs,
-// 8 bits per pass.
+// 8 or 9 bits per pass.
 //
 // Radix sort: one read of the keys counts every digit (rs_plan_kernel); then
 // each pass reads and writes the items once (rs_pass_kernel): a tile gets the
