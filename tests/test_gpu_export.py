@@ -100,3 +100,37 @@ def test_export_filter_tiles(ctx, vsabi, n_pairs):
     np.testing.assert_array_equal(gl.cpu().numpy(), el)
     np.testing.assert_array_equal(gr.cpu().numpy(), er)
     np.testing.assert_array_equal(gs.cpu().numpy(), es)
+
+
+def _leave_nonzero_device_memory():
+    """Small device allocations full of ones, given back: what a context's own words are then carved from."""
+    import ctypes
+
+    import torch
+
+    torch.zeros(1, device="cuda")
+    rt = ctypes.CDLL("libcudart.so.12")
+    blocks = []
+    for _ in range(64):
+        p = ctypes.c_void_p()
+        assert rt.cudaMalloc(ctypes.byref(p), ctypes.c_size_t(512)) == 0
+        assert rt.cudaMemset(p, 0xFF, ctypes.c_size_t(512)) == 0
+        blocks.append(p)
+    assert rt.cudaDeviceSynchronize() == 0
+    for p in blocks:
+        assert rt.cudaFree(p) == 0
+
+
+@pytest.mark.parametrize("n", [0, 5])
+def test_export_right_without_kept_pairs_on_a_new_context(vsabi, n):
+    """The first call of a context, with no pairs or with all of them filtered out: nothing is sorted, and no status
+    is read that nothing has set."""
+    import torch
+
+    _leave_nonzero_device_memory()
+    new = vsabi.Context(0)
+    l = torch.arange(n, dtype=torch.int32, device="cuda")
+    codes = torch.zeros(8, dtype=torch.int64, device="cuda"), torch.ones(8, dtype=torch.int64, device="cuda")
+    gl, gr, gs = vsabi.join_export(new, l, l, 8, 8, "right", *codes)
+    assert gl.tolist() == [-1] * 8 and gr.tolist() == list(range(8)) and gs.tolist() == [-1] * 8
+    new.close()

@@ -156,7 +156,8 @@ int vs_context_create(int device, void* stream, vs_context** out) {
                   cudaSuccess;
     if (ok) {
         ctx->d_direct = ctx->d_counters + kDevCounters;
-        ok = cudaMemsetAsync(ctx->d_direct, 0, kDirectWords * sizeof(unsigned long long), ctx->stream) == cudaSuccess &&
+        ok = cudaMemsetAsync(ctx->d_counters, 0, (kDevCounters + kDirectWords) * sizeof(unsigned long long),
+                             ctx->stream) == cudaSuccess &&
              cudaMemsetAsync(ctx->d_direct + kDirectStart, 0xff, sizeof(unsigned long long), ctx->stream) == cudaSuccess;
     }
     for (int k = 0; k < 5 && ok; ++k) ok = cudaEventCreate(&ctx->phase_ev[k]) == cudaSuccess;

@@ -488,10 +488,10 @@ int vs_join_export(vs_context* ctx, const int32_t* d_left, const int32_t* d_righ
             const int64_t m = h.kept;
             VS_TRY(keys.alloc((size_t)m, s));
             VS_TRY(perm.alloc((size_t)m, s));
+            VS_TRY(clear_sort_error(ctx));  // (read below, whether or not there is anything to sort)
             if (m > 0) {
                 export_keys_kernel<<<grid_of(export_keys_kernel, m), 256, 0, s>>>(drive, other, m, keys.p, perm.p);
                 VS_LAUNCHED("export_keys", s);
-                VS_TRY(clear_sort_error(ctx));
                 VS_TRY(radix_sort_u64_u32(keys.p, perm.p, m, 64, s, 0, &ctx->d_counters[kSortErr]));
             }
             pairs = ExportPairs{nullptr, nullptr, keys.p, perm.p, ksrc};
