@@ -102,8 +102,9 @@ def test_export_filter_tiles(ctx, vsabi, n_pairs):
     np.testing.assert_array_equal(gs.cpu().numpy(), es)
 
 
-def _leave_nonzero_device_memory():
-    """Small device allocations full of ones, given back: what a context's own words are then carved from."""
+def _nonzero_device_memory():
+    """Small device allocations full of ones, every other one given back: the context's own words then lie in one of
+    these.  Returns what frees the rest."""
     import ctypes
 
     import torch
@@ -117,8 +118,9 @@ def _leave_nonzero_device_memory():
         assert rt.cudaMemset(p, 0xFF, ctypes.c_size_t(512)) == 0
         blocks.append(p)
     assert rt.cudaDeviceSynchronize() == 0
-    for p in blocks:
+    for p in blocks[1::2]:
         assert rt.cudaFree(p) == 0
+    return lambda: [rt.cudaFree(p) for p in blocks[::2]]
 
 
 @pytest.mark.parametrize("n", [0, 5])
@@ -127,10 +129,43 @@ def test_export_right_without_kept_pairs_on_a_new_context(vsabi, n):
     is read that nothing has set."""
     import torch
 
-    _leave_nonzero_device_memory()
+    free = _nonzero_device_memory()
     new = vsabi.Context(0)
     l = torch.arange(n, dtype=torch.int32, device="cuda")
     codes = torch.zeros(8, dtype=torch.int64, device="cuda"), torch.ones(8, dtype=torch.int64, device="cuda")
     gl, gr, gs = vsabi.join_export(new, l, l, 8, 8, "right", *codes)
     assert gl.tolist() == [-1] * 8 and gr.tolist() == list(range(8)) and gs.tolist() == [-1] * 8
     new.close()
+    free()
+
+
+def test_export_of_shuffled_pairs_over_many_tiles(ctx, vsabi):
+    """Pairs in any order: the rows of the sorted ones, in time linear in the pairs (20M left rows are 9766 tiles;
+    work that grew with pairs x tiles took over 100 times the sorted call, the sort of the pairs takes a few)."""
+    import time
+
+    import torch
+
+    n_left, n_right = 20_000_000, 1_000
+    rng = np.random.default_rng(8)
+    l, r = _pairs(rng, n_left, n_right, 2_000_000)
+    mix = rng.permutation(len(l))
+    dl, dr = torch.from_numpy(l).cuda(), torch.from_numpy(r).cuda()
+    dm = torch.from_numpy(mix).cuda()
+    ml, mr = dl[dm], dr[dm]
+
+    def timed(a, b):
+        out, best = None, 1e9
+        for _ in range(3):
+            torch.cuda.synchronize()
+            t = time.perf_counter()
+            out = vsabi.join_export(ctx, a, b, n_left, n_right, "left")
+            torch.cuda.synchronize()
+            best = min(best, time.perf_counter() - t)
+        return out, best
+
+    (sl, sr, ss), t_sorted = timed(dl, dr)
+    (gl, gr, gs), t_mixed = timed(ml, mr)
+    assert torch.equal(gl, sl) and torch.equal(gr, sr)
+    assert torch.equal(torch.where(gs >= 0, dm[gs.clamp(min=0)], gs), ss)
+    assert t_mixed < 20 * t_sorted, (t_mixed, t_sorted)
