@@ -219,7 +219,7 @@ int vs_index_build(vs_context* ctx, const vs_polygons* polys, const vs_index_opt
     idx->device = ctx->device;
     EventPair ev;
     cudaEventRecord(ev.a, ctx->stream);
-    int st = clear_sort_error(ctx);
+    int st = clear_status(ctx);
     if (st == VS_OK) st = build_rtree(ctx, polys, idx);
     if (st == VS_OK) st = build_ring_bins(ctx, idx, opts ? opts->ring_bin_min_vertices : 0);
     if (st == VS_OK && opts && (opts->method_mask & 2)) st = build_learned_index(ctx, idx, opts);
@@ -230,7 +230,7 @@ int vs_index_build(vs_context* ctx, const vs_polygons* polys, const vs_index_opt
         return st;
     }
     cudaEventRecord(ev.b, ctx->stream);
-    st = finish_sort(ctx);
+    st = finish_status(ctx);
     if (st != VS_OK) {
         cudaStreamSynchronize(ctx->stream);
         free_index_memory(idx);
@@ -468,9 +468,9 @@ int vs_radix_sort_pairs(vs_context* ctx, uint64_t* d_keys, uint32_t* d_vals, int
         return VS_E_ARG;
     }
     VS_TRY(use_device(ctx->device));
-    VS_TRY(clear_sort_error(ctx));
-    VS_TRY(radix_sort_u64_u32(d_keys, d_vals, n, key_bits, ctx->stream, 0, &ctx->d_counters[kSortErr]));
-    return finish_sort(ctx);
+    VS_TRY(radix_sort_u64_u32(d_keys, d_vals, n, key_bits, ctx->stream));
+    VS_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+    return VS_OK;
 }
 
 int vs_hilbert_keys(vs_context* ctx, const double* d_x, const double* d_y, int64_t n, double minx, double miny,

@@ -424,7 +424,7 @@ int enqueue_batch(vs_batch_plan* p, cudaStream_t s, int mask, int32_t* left, int
     const size_t smem = (size_t)(p->n_jobs + 1) * sizeof(int64_t);
     batch_key_kernel<<<resident_grid(batch_key_kernel, p->n_points, 256, smem), 256, smem, s>>>(a, p->n_points);
     VS_LAUNCHED("batch_key", s);
-    VS_TRY(radix_sort_u32_u32(p->keys, p->order, p->n_points, 32, s, p->sort_begin, a.counters + 4));
+    VS_TRY(radix_sort_u32_u32(p->keys, p->order, p->n_points, 32, s, p->sort_begin));
     // blocks per SM from the launch shape, capped at what can be resident
     const int resident = resident_grid(batch_join_kernel, (int64_t)1 << 30, kBThreads) / kNumSMs;
     const int per_sm = p->opts.blocks_per_sm < resident ? p->opts.blocks_per_sm : resident;

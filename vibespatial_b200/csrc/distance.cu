@@ -1847,7 +1847,7 @@ int vs_join_nearest_polygons(vs_context* ctx, const vs_index* point_index, const
     poly_query_key_kernel<<<resident_grid(poly_query_key_kernel, nq, 256), 256, 0, s>>>(
         *queries, point_index->frame, qbox.p, keys.p, order.p, n_valid.p);
     VS_LAUNCHED("poly_query_key", s);
-    VS_TRY(radix_sort_u32_u32(keys.p, order.p, nq, 32, s, 0, &ctx->d_counters[4]));
+    VS_TRY(radix_sort_u32_u32(keys.p, order.p, nq, 32, s));
     PolyArgs a{};
     a.x = queries->d_x;
     a.y = queries->d_y;

@@ -496,11 +496,10 @@ int vs_join_export(vs_context* ctx, const int32_t* d_left, const int32_t* d_righ
             const int64_t m = h.kept;
             VS_TRY(keys.alloc((size_t)m, s));
             VS_TRY(perm.alloc((size_t)m, s));
-            VS_TRY(clear_sort_error(ctx));  // (read below, whether or not there is anything to sort)
             if (m > 0) {
                 export_keys_kernel<<<grid_of(export_keys_kernel, m), 256, 0, s>>>(drive, other, m, keys.p, perm.p);
                 VS_LAUNCHED("export_keys", s);
-                VS_TRY(radix_sort_u64_u32(keys.p, perm.p, m, 64, s, 0, &ctx->d_counters[kSortErr]));
+                VS_TRY(radix_sort_u64_u32(keys.p, perm.p, m, 64, s));
             }
             pairs = ExportPairs{nullptr, nullptr, keys.p, perm.p, ksrc};
             VS_CUDA_TRY(cudaMemsetAsync(&state.p->unsorted, 0, sizeof(uint32_t), s));
@@ -525,7 +524,6 @@ int vs_join_export(vs_context* ctx, const int32_t* d_left, const int32_t* d_righ
             VS_LAUNCHED("export_append", s);
         }
         VS_TRY(read_state());
-        if (!sorted) VS_TRY(finish_sort(ctx));
         if (!h.unsorted) break;
         sorted = false;
     }

@@ -221,7 +221,6 @@ int vs_join_host(vs_context* ctx, const vs_index* idx, const double* h_x, const 
     int64_t total = 0;
     bool over = false;
     const long long launches0 = g_launches;
-    VS_TRY(clear_sort_error(ctx));
     VS_TRY(copy_in(0));
     for (int64_t k = 0; k < n_chunks; ++k) {
         const int b = (int)(k & 1);
@@ -233,8 +232,7 @@ int vs_join_host(vs_context* ctx, const vs_index* idx, const double* h_x, const 
         unsigned long long* c = ctx->h_counter;
         for (int attempt = 0;; ++attempt) {
             const DeferSink ds{ctx->defer_buf, ctx->defer_cap, &ctx->d_counters[7]};
-            // (the sort's error word keeps what earlier chunks set)
-            VS_CUDA_TRY(cudaMemsetAsync(ctx->d_counters, 0, kSortErr * sizeof(unsigned long long), s));
+            VS_CUDA_TRY(cudaMemsetAsync(ctx->d_counters, 0, kDevCounters * sizeof(unsigned long long), s));
             if (method == VS_METHOD_LEARNED)
                 VS_TRY(launch_learned_join(ctx, idx, &pts, mask, bf.left[b], bf.right[b], bf.cap[b], ds, first));
             else
@@ -287,7 +285,7 @@ int vs_join_host(vs_context* ctx, const vs_index* idx, const double* h_x, const 
     VS_CUDA_TRY(cudaEventRecord(st.t1, st.out));
     VS_CUDA_TRY(cudaStreamSynchronize(st.out));
     VS_CUDA_TRY(cudaStreamSynchronize(st.in));
-    VS_TRY(finish_sort(ctx));
+    VS_CUDA_TRY(cudaStreamSynchronize(s));
     *n_pairs = total;
     if (stats) {
         stats->exact_fallbacks = (int64_t)totals[1];

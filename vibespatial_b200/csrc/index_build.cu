@@ -376,7 +376,7 @@ int build_rtree(vs_context* ctx, const vs_polygons* P, vs_index* idx) {
     if (M > 0) {
         hilbert_box_key_kernel<<<grid_for(M, 256), 256, 0, s>>>(box.p, M, idx->frame, keys.p, vals.p);
         VS_CUDA_TRY(cudaGetLastError());
-        VS_TRY(radix_sort_u64_u32(keys.p, vals.p, M, 64, s, 0, &ctx->d_counters[kSortErr]));
+        VS_TRY(radix_sort_u64_u32(keys.p, vals.p, M, 64, s));
         slot_gather_kernel<<<grid_for(M, 256), 256, 0, s>>>(vals.p, M, box.p, np.p, nr.p, nc.p, idx->nodes,
                                                             idx->item_geom, sp.p, sr.p, sc.p);
         VS_CUDA_TRY(cudaGetLastError());

@@ -412,7 +412,7 @@ int prepare_queries(vs_context* ctx, const vs_index* idx, const vs_points* pts, 
     VS_LAUNCHED("point_sort_key", s);
     // Sorting by the top 24 key bits (a level-12 Hilbert cell) already makes
     // a warp's 32 points spatially coherent; the low byte is left unsorted.
-    VS_TRY(radix_sort_u32_u32(q.keys.p, q.order.p, n, 32, s, 8, &ctx->d_counters[4]));
+    VS_TRY(radix_sort_u32_u32(q.keys.p, q.order.p, n, 32, s, 8));
     return VS_OK;
 }
 
@@ -520,36 +520,36 @@ int enqueue_sort_pairs(vs_context* ctx, int32_t* d_left, int32_t* d_right, int64
     }
     const int64_t n_left = max_left < 0xffffffffull ? (int64_t)max_left : 0;
     return radix_sort_pairs(d_left, d_right, n, lbits, rbits, n_left, by_runs, ctx->stream,
-                            &ctx->d_counters[kSortErr]);
+                            &ctx->d_counters[kStatus]);
 }
 
 int finish_sort_pairs(vs_context* ctx, int32_t* d_left, int32_t* d_right, int64_t n, uint64_t max_left,
                       uint64_t max_right) {
-    VS_TRY(finish_sort(ctx));
+    VS_TRY(finish_status(ctx));
     if (!(ctx->h_counter[kHostCounters - 1] & 4)) return VS_OK;
     // a left row with very many pairs
     VS_TRY(enqueue_sort_pairs(ctx, d_left, d_right, n, max_left, max_right, false));
-    return finish_sort(ctx);
+    return finish_status(ctx);
 }
 
 int sort_pairs(vs_context* ctx, int32_t* d_left, int32_t* d_right, int64_t n, uint64_t max_left, uint64_t max_right) {
-    VS_TRY(clear_sort_error(ctx));
+    VS_TRY(clear_status(ctx));
     VS_TRY(enqueue_sort_pairs(ctx, d_left, d_right, n, max_left, max_right, true));
     return finish_sort_pairs(ctx, d_left, d_right, n, max_left, max_right);
 }
 
-int clear_sort_error(vs_context* ctx) {
-    VS_CUDA_TRY(cudaMemsetAsync(&ctx->d_counters[kSortErr], 0, sizeof(unsigned long long), ctx->stream));
+int clear_status(vs_context* ctx) {
+    VS_CUDA_TRY(cudaMemsetAsync(&ctx->d_counters[kStatus], 0, sizeof(unsigned long long), ctx->stream));
     return VS_OK;
 }
 
-int finish_sort(vs_context* ctx) {
+int finish_status(vs_context* ctx) {
     cudaStream_t s = ctx->stream;
     unsigned long long* flags = &ctx->h_counter[kHostCounters - 1];
-    VS_CUDA_TRY(cudaMemcpyAsync(flags, &ctx->d_counters[kSortErr], sizeof(*flags), cudaMemcpyDeviceToHost, s));
+    VS_CUDA_TRY(cudaMemcpyAsync(flags, &ctx->d_counters[kStatus], sizeof(*flags), cudaMemcpyDeviceToHost, s));
     VS_CUDA_TRY(cudaStreamSynchronize(s));
     if (*flags & 2) {
-        set_error("a bounded device wait (radix sort) gave up; the order is incomplete");
+        set_error("a bounded device wait (RMI training) gave up; there is no model");
         return VS_E_TIMEOUT;
     }
     return VS_OK;

@@ -54,16 +54,17 @@ int launch_locate_aligned(vs_context* ctx, const vs_points* pts, const vs_polygo
 // Sort (left, right) pairs and wait for them; rows below max_left, max_right.
 int sort_pairs(vs_context* ctx, int32_t* d_left, int32_t* d_right, int64_t n, uint64_t max_left,
                uint64_t max_right);
-// The same without waiting (by_runs as for radix_sort_pairs).  Bit 1 of
-// d_counters[kSortErr] (which clear_sort_error zeroes) reports a wait that
-// gave up; finish_sort waits for the stream and reads it.
+// The same without waiting (by_runs as for radix_sort_pairs, on
+// d_counters[kStatus], which clear_status zeroes).
 int enqueue_sort_pairs(vs_context* ctx, int32_t* d_left, int32_t* d_right, int64_t n, uint64_t max_left,
                        uint64_t max_right, bool by_runs);
 // Wait for an enqueued sort (by_runs), and sort by every digit what it left.
 int finish_sort_pairs(vs_context* ctx, int32_t* d_left, int32_t* d_right, int64_t n, uint64_t max_left,
                       uint64_t max_right);
-int clear_sort_error(vs_context* ctx);
-int finish_sort(vs_context* ctx);
+// Zero the status word; wait for the stream and read it (to the last word of
+// h_counter; VS_E_TIMEOUT for a wait that gave up).
+int clear_status(vs_context* ctx);
+int finish_status(vs_context* ctx);
 int build_rtree(vs_context* ctx, const vs_polygons* P, vs_index* idx);
 // y-bins for rings of at least min_vertices vertices (0: the default, < 0: none).
 int build_ring_bins(vs_context* ctx, vs_index* idx, int min_vertices);

@@ -853,8 +853,7 @@ __global__ void learned_desc_kernel(const double* __restrict__ fr, LearnedJob* _
 // their squared entry counts (sum_sq) of the slot boxes at grid level L, on
 // scratch only: the count, emit, sort and unique-flag steps of the build.
 int probe_level(cudaStream_t s, const vs_box* boxes, int64_t M, const double* frame, int L, uint32_t* cnt,
-                unsigned long long* tot, unsigned long long* sort_err, unsigned long long& E, uint32_t& n_cells,
-                unsigned long long& sum_sq) {
+                unsigned long long* tot, unsigned long long& E, uint32_t& n_cells, unsigned long long& sum_sq) {
     VS_CUDA_TRY(cudaMemsetAsync(tot, 0, sizeof(unsigned long long), s));
     cell_count_kernel<<<grid_for(M, 256), 256, 0, s>>>(boxes, M, frame, L, cnt, tot);
     VS_CUDA_TRY(cudaMemcpyAsync(&E, tot, sizeof(E), cudaMemcpyDeviceToHost, s));
@@ -871,7 +870,7 @@ int probe_level(cudaStream_t s, const vs_box* boxes, int64_t M, const double* fr
     VS_TRY(exclusive_scan_u32(cnt, off.p, M, nullptr, s));
     cell_emit_kernel<<<grid_for(M, 256), 256, 0, s>>>(boxes, M, frame, L, off.p, keys.p, vals.p);
     VS_CUDA_TRY(cudaGetLastError());
-    VS_TRY(radix_sort_u32_u32(keys.p, vals.p, (int64_t)E, 2 * L, s, 0, sort_err));
+    VS_TRY(radix_sort_u32_u32(keys.p, vals.p, (int64_t)E, 2 * L, s));
     cell_flag_kernel<<<grid_for((int64_t)E, 256), 256, 0, s>>>(keys.p, (int64_t)E, flag.p);
     VS_TRY(exclusive_scan_u32(flag.p, flag.p, (int64_t)E, nc.p, s));
     VS_CUDA_TRY(cudaMemsetAsync(tot, 0, sizeof(unsigned long long), s));
@@ -906,7 +905,7 @@ int train_rmi(vs_context* ctx, vs_index* idx, int steps) {
     ta.arrived = arrived.p;
     ta.loss = grad.p + 3 * kGradWords;
     ta.model = li.model;
-    ta.err = &ctx->d_counters[kSortErr];
+    ta.err = &ctx->d_counters[kStatus];
     // The blocks meet at a barrier every step: a cooperative launch, so all of them run at once.
     VS_CUDA_TRY(cudaFuncSetAttribute(rmi_train_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)sizeof(TrainShared)));
@@ -1038,13 +1037,12 @@ int build_learned_index(vs_context* ctx, vs_index* idx, const vs_index_options* 
     if (auto_level && E > 0) {
         uint32_t nc = 0;
         unsigned long long sq = 0;
-        VS_TRY(probe_level(s, boxes, M, idx->frame, L, cnt.p, tot.p, &ctx->d_counters[kSortErr], E, nc, sq));
+        VS_TRY(probe_level(s, boxes, M, idx->frame, L, cnt.p, tot.p, E, nc, sq));
         const int l_max = std::min(15, L + 3);
         while (L < l_max && nc > 0 && (double)sq > 2.5 * (double)E) {
             unsigned long long e1 = 0, sq1 = 0;
             uint32_t nc1 = 0;
-            VS_TRY(probe_level(s, boxes, M, idx->frame, L + 1, cnt.p, tot.p,
-                               &ctx->d_counters[kSortErr], e1, nc1, sq1));
+            VS_TRY(probe_level(s, boxes, M, idx->frame, L + 1, cnt.p, tot.p, e1, nc1, sq1));
             if (e1 > (unsigned long long)(16 * M + (1 << 20)) || e1 >= 0x7fffffffull) break;
             ++L;
             E = e1;
@@ -1071,7 +1069,7 @@ int build_learned_index(vs_context* ctx, vs_index* idx, const vs_index_options* 
     VS_TRY(exclusive_scan_u32(cnt.p, off.p, M, nullptr, s));
     cell_emit_kernel<<<grid_for(M, 256), 256, 0, s>>>(boxes, M, idx->frame, L, off.p, keys.p, li.entries);
     VS_CUDA_TRY(cudaGetLastError());
-    VS_TRY(radix_sort_u32_u32(keys.p, li.entries, (int64_t)E, 2 * L, s, 0, &ctx->d_counters[kSortErr]));
+    VS_TRY(radix_sort_u32_u32(keys.p, li.entries, (int64_t)E, 2 * L, s));
     // 3. unique cells + CSR
     Scratch<uint32_t> ncell;
     VS_TRY(ncell.alloc(1, s));

@@ -171,14 +171,18 @@ struct SortArgs {
     uint32_t* hist;     // [n_digits][radix] counts, then exclusive sums
     uint32_t* ticket;   // [0] histogram blocks done, [1 + slot] tiles handed out
     SortPlan* plan;
-    unsigned long long* err;  // nullable
+    unsigned long long* too_long;  // pairs by runs: gets bit 2 (nullable)
     int64_t n_tiles;
 };
 
 template <class K>
-__device__ __forceinline__ K sort_key(const SortArgs<K>& a, const K* keys, int64_t i) {
+__device__ __forceinline__ K sort_key(const K* keys, const int32_t* left, const int32_t* right, int rbits, int64_t i) {
     if (keys) return keys[i];
-    return (K)(((uint64_t)(uint32_t)a.left[i] << a.rbits) | (uint64_t)(uint32_t)a.right[i]);
+    return (K)(((uint64_t)(uint32_t)left[i] << rbits) | (uint64_t)(uint32_t)right[i]);
+}
+template <class K>
+__device__ __forceinline__ K sort_key(const SortArgs<K>& a, const K* keys, int64_t i) {
+    return sort_key(keys, a.left, a.right, a.rbits, i);
 }
 
 // Every digit's histogram in one read of the keys; the last block to finish
@@ -302,7 +306,11 @@ __device__ __forceinline__ void store_state(unsigned long long* p, unsigned long
     asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
-constexpr int kWaitLimit = 1 << 20;  // polls of earlier tiles before a pass gives up
+// Polls of earlier tiles before a tile counts their keys itself (a build may lower it to test that).
+#ifndef VS_SORT_WAIT_LIMIT
+#define VS_SORT_WAIT_LIMIT (1 << 20)
+#endif
+constexpr int kWaitLimit = VS_SORT_WAIT_LIMIT;
 // Earlier tiles whose states a tile reads at once: the tiles of a pass's first
 // wave start together and have only counts, no sums, to read from one another.
 constexpr int kLookBack = 8;
@@ -320,14 +328,26 @@ struct PassShared {
     uint32_t val[kVals ? T : 1];
 };
 
+// Keys of a digit value among the first n of a pass's input, by one thread.  A
+// tile that has waited kWaitLimit polls for an earlier one counts that tile's
+// keys, and those before it, this way: the input is complete before the pass
+// starts, so the positions are right whatever became of the wait.
+template <class K>
+__device__ __noinline__ uint32_t count_digit(const K* keys, const int32_t* left, const int32_t* right, int rbits,
+                                             int64_t n, int shift, unsigned mask, unsigned digit) {
+    uint32_t c = 0;
+    for (int64_t i = 0; i < n; ++i)
+        c += ((unsigned)(sort_key(keys, left, right, rbits, i) >> shift) & mask) == digit ? 1u : 0u;
+    return c;
+}
+
 // One slot of the sort: the tiles are taken in order (a ticket), so every tile
 // before a running one is running or done.  A tile ranks its keys (warp by
 // warp, no block barrier in between), publishes its digit counts, stages the
 // keys in digit order in shared memory, sums the counts of the tiles before
 // it (each publishes its counts, then its inclusive sums, as value << 2 |
 // state in one word: S), and writes the digit runs.  Keys are read and
-// written once a pass.  A wait that runs out sets bit 1 of *err; positions
-// stay inside the output whatever was read.
+// written once a pass.  A wait that runs out ends in a count (count_digit).
 //
 // Bound by instruction issue (the ranks: a ballot a bit) at two blocks an SM.
 // 12.2M pairs with 26 and 20 bits of rows: 94 us the first pass, which need
@@ -431,7 +451,7 @@ __global__ void __launch_bounds__(kPassThreads) rs_pass_kernel(const SortArgs<K>
                 // wait for the one state that is missing, without flooding L2
                 while ((load_state(status + t * kRadix + tid) & 3) == 0 && ++polls < kWaitLimit) __nanosleep(40);
                 if (polls >= kWaitLimit) {
-                    if (a.err) atomicOr(a.err, 2ull);
+                    sum += count_digit(kin, a.left, a.right, a.rbits, (t + 1) * T, shift, kRadix - 1u, (unsigned)tid);
                     break;
                 }
             }
@@ -449,7 +469,6 @@ __global__ void __launch_bounds__(kPassThreads) rs_pass_kernel(const SortArgs<K>
         if (j >= count) break;
         const K key = sm.key[j];
         const unsigned long long pos = sm.off[(unsigned)(key >> shift) & (unsigned)(kRadix - 1)] + (unsigned)j;
-        if (pos >= (unsigned long long)a.n) continue;  // only after a wait that gave up
         kout[pos] = key;
         if (kVals) vout[pos] = sm.val[j];
     }
@@ -458,7 +477,7 @@ __global__ void __launch_bounds__(kPassThreads) rs_pass_kernel(const SortArgs<K>
 // The pairs, sorted by left, back to the caller's arrays; in a run of equal
 // left rows each pair goes to the place its right row gives it (the number of
 // smaller ones in the run, equal ones in their order).  A run longer than
-// kRunMax is left as it is and reported (bit 2 of *err): such pairs are sorted
+// kRunMax is left as it is and reported (bit 2 of *too_long): such pairs are sorted
 // by right's digits instead.
 constexpr int kRunThreads = 256, kRunItems = 8, kRunTile = kRunThreads * kRunItems, kRunHalo = 64;
 
@@ -510,7 +529,7 @@ __global__ void __launch_bounds__(kRunThreads) rs_runs_kernel(const SortArgs<uin
         a.left[pos] = (int32_t)l;
         a.right[pos] = (int32_t)r;
     }
-    if (too_long && a.err) atomicOr(a.err, 4ull);
+    if (too_long && a.too_long) atomicOr(a.too_long, 4ull);
 }
 
 // A sort of at most kSmallSort items in one block: every pass in shared
@@ -723,28 +742,24 @@ int exclusive_scan_u64(const uint64_t* in, uint64_t* out, int64_t n, uint64_t* d
     return exclusive_scan_impl<uint64_t>(in, out, n, d_total, s);
 }
 
-int radix_sort_u64_u32(uint64_t* keys, uint32_t* vals, int64_t n, int key_bits, cudaStream_t s, int begin_bit,
-                       unsigned long long* err) {
+int radix_sort_u64_u32(uint64_t* keys, uint32_t* vals, int64_t n, int key_bits, cudaStream_t s, int begin_bit) {
     SortArgs<uint64_t> a{};
     a.keys = keys;
     a.vals = vals;
     a.n = n;
-    a.err = err;
     return sort_arrays(a, begin_bit, key_bits, s);
 }
 
-int radix_sort_u32_u32(uint32_t* keys, uint32_t* vals, int64_t n, int key_bits, cudaStream_t s, int begin_bit,
-                       unsigned long long* err) {
+int radix_sort_u32_u32(uint32_t* keys, uint32_t* vals, int64_t n, int key_bits, cudaStream_t s, int begin_bit) {
     SortArgs<uint32_t> a{};
     a.keys = keys;
     a.vals = vals;
     a.n = n;
-    a.err = err;
     return sort_arrays(a, begin_bit, key_bits, s);
 }
 
 int radix_sort_pairs(int32_t* left, int32_t* right, int64_t n, int left_bits, int right_bits, int64_t n_left,
-                     bool by_runs, cudaStream_t s, unsigned long long* err) {
+                     bool by_runs, cudaStream_t s, unsigned long long* too_long) {
     if (n <= 1) return VS_OK;
     VS_TRY(check_count(n));
     SortArgs<uint64_t> a{};
@@ -752,7 +767,7 @@ int radix_sort_pairs(int32_t* left, int32_t* right, int64_t n, int left_bits, in
     a.right = right;
     a.rbits = right_bits;
     a.n = n;
-    a.err = err;
+    a.too_long = too_long;
     if (n <= kSmallSort) {
         add_digits(a, 0, left_bits + right_bits, 8);
         return n <= 2 * kSmallThreads ? launch_small_sort<uint64_t, false, 2>(a, s)

@@ -73,20 +73,16 @@ int exclusive_scan_u32(const uint32_t* in, uint32_t* out, int64_t n, uint32_t* d
 int exclusive_scan_u64(const uint64_t* in, uint64_t* out, int64_t n, uint64_t* d_total, cudaStream_t s);
 
 // Stable LSD radix sort of (key, value) pairs by key bits [begin_bit,
-// key_bits) (8 bits per pass).  Sorted data ends in keys / vals.  Bit 1 of
-// *err (device memory) is set when a bounded wait inside a pass gave up: the
-// order is then incomplete.
-int radix_sort_u64_u32(uint64_t* keys, uint32_t* vals, int64_t n, int key_bits, cudaStream_t s, int begin_bit,
-                       unsigned long long* err);
-int radix_sort_u32_u32(uint32_t* keys, uint32_t* vals, int64_t n, int key_bits, cudaStream_t s, int begin_bit,
-                       unsigned long long* err);
+// key_bits) (8 bits per pass).  Sorted data ends in keys / vals.
+int radix_sort_u64_u32(uint64_t* keys, uint32_t* vals, int64_t n, int key_bits, cudaStream_t s, int begin_bit = 0);
+int radix_sort_u32_u32(uint32_t* keys, uint32_t* vals, int64_t n, int key_bits, cudaStream_t s, int begin_bit = 0);
 // The same for (left, right) pairs in place, by left then right: rows below
 // 2^left_bits and 2^right_bits (at most 32 each; digits that are the same in
 // every pair cost no pass).  by_runs: where left rows have few pairs each
 // (n_left rows; 0: not known) only left is sorted by digits and equal left
-// rows are ordered in their runs; bit 2 of *err then reports a run too long
-// for that, whose pairs are in left's order only.
+// rows are ordered in their runs; bit 2 of *too_long (device memory) then
+// reports a run too long for that, whose pairs are in left's order only.
 int radix_sort_pairs(int32_t* left, int32_t* right, int64_t n, int left_bits, int right_bits, int64_t n_left,
-                     bool by_runs, cudaStream_t s, unsigned long long* err);
+                     bool by_runs, cudaStream_t s, unsigned long long* too_long);
 
 }  // namespace vs

@@ -35,7 +35,7 @@ enum : int {
     kDirectWords = 9
 };
 constexpr uint64_t kIndexPoolKeep = 1ull << 30;  // unused bytes the index pool keeps for the next build
-constexpr int kSortErr = 16;  // bit 1: a bounded wait of a pair sort gave up
+constexpr int kStatus = 16;  // bit 1: a bounded wait of the RMI training gave up; bit 2: a run of pairs too long
 
 #define VS_CUDA_TRY(expr)                                                        \
     do {                                                                         \
@@ -154,8 +154,8 @@ struct vs_context {
     // [0] pair count, [1] exact-fallback count, [2] fp32-filter decided
     // edges, [3] edges sent past the fp32 filter, [4] error flags,
     // [5] candidate (bbox) count, [6] wide learned-index windows,
-    // [7] deferred pairs, [8] work queue of the refine kernel, [16] error
-    // flags of the pair sort.
+    // [7] deferred pairs, [8] work queue of the refine kernel, [16] status
+    // of a training or pair sort (kStatus).
     unsigned long long* d_counters;
     // State of the direct join (kDirect* words): zero, start all ones, between
     // calls.
