@@ -84,3 +84,26 @@ order = np.lexsort((tree[1].cpu().numpy(), tree[0].cpu().numpy()))
 assert np.array_equal(order, np.arange(len(order)))
 assert torch.equal(tree[0], cells[0]) and torch.equal(tree[1], cells[1])
 """)
+
+
+@needs_nvcc
+def test_training_that_gives_up_reports_it(tmp_path):
+    """A training whose grid barrier runs out leaves a model that the passes after it can use within their arrays; the
+    build then reports the timeout, and the context serves the next calls."""
+    lib = _library(tmp_path, {"learned": ["-DVS_TRAIN_WAIT_LIMIT=1"]})
+    _run(lib, """
+w = syn.star_join(seed=3, n_points=20_003, n_polys=20_000)  # over 16384 cells: 128 blocks
+polys = [dev(getattr(w.polys, k)) for k in ("x", "y", "ring_off", "part_off", "geom_off")]
+for _ in range(2):
+    try:
+        _abi.DeviceIndex(ctx, _abi.make_polygons(*polys), learned=True)
+        raise SystemExit("no timeout")
+    except _abi.VsError as e:
+        assert e.status == _abi.VS_E_TIMEOUT and "RMI training" in str(e), e
+tree = _abi.DeviceIndex(ctx, _abi.make_polygons(*polys))
+dx, dy = dev(w.px), dev(w.py)
+pts = _abi.make_points(dx, dy)
+left, right, _ = tree.join(pts, _abi.PRED_WITHIN, _abi.METHOD_RTREE)
+brute = tree.join(pts, _abi.PRED_WITHIN, _abi.METHOD_BRUTE)
+assert left.numel() > 0 and torch.equal(left, brute[0]) and torch.equal(right, brute[1])
+""")

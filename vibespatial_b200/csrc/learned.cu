@@ -403,7 +403,11 @@ static_assert(kTrainSamples / kTrainThreads <= kNumSMs, "the training blocks run
 constexpr int kTrainStride = 36;  // floats a sample row: 16-byte rows whose lanes' stores miss one another's banks
 constexpr int kGradWords = 1160;  // kRmiP gradients, the loss, padding to 16 bytes
 constexpr int kLossWord = kRmiP;
-constexpr int kTrainWaitLimit = 1 << 21;
+// Polls of the grid barrier before a block ends the training (a build may lower it to test that).
+#ifndef VS_TRAIN_WAIT_LIMIT
+#define VS_TRAIN_WAIT_LIMIT (1 << 21)
+#endif
+constexpr int kTrainWaitLimit = VS_TRAIN_WAIT_LIMIT;
 
 struct TrainArgs {
     const uint32_t* keys;
@@ -697,7 +701,8 @@ __global__ void __launch_bounds__(kTrainThreads) rmi_train_kernel(const TrainArg
             }
         }
         __syncthreads();
-        if (sm.fail) return;
+        // (the model is written all the same: the passes after this one read it before the host reads the status)
+        if (sm.fail) break;
         // Adam, the same in every block
         const float lr = 2e-3f * (step < a.steps / 2 ? 1.0f : 0.3f);
         const float b1 = 0.9f, b2 = 0.999f;
