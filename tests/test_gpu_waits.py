@@ -42,11 +42,12 @@ def _library(folder, defines):
 
 def _run(lib, code):
     head = (f"import sys\nsys.path.insert(0, {str(ROOT)!r})\nimport numpy as np\nimport torch\n"
-            f"from vibespatial_b200 import _abi\n_abi.load({str(lib)!r})\n"
+            f"from vibespatial_b200 import _abi\n_abi._lib = _abi.load({str(lib)!r})\n"
             "from vibespatial_b200.testing import synthetic as syn\nctx = _abi.default_context(0)\n"
             "dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()\n")
     r = subprocess.run([sys.executable, "-c", head + code], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout + r.stderr
+    print(r.stdout)
 
 
 needs_nvcc = pytest.mark.skipif(shutil.which(_build.nvcc()) is None, reason="needs nvcc")
@@ -106,4 +107,31 @@ pts = _abi.make_points(dx, dy)
 left, right, _ = tree.join(pts, _abi.PRED_WITHIN, _abi.METHOD_RTREE)
 brute = tree.join(pts, _abi.PRED_WITHIN, _abi.METHOD_BRUTE)
 assert left.numel() > 0 and torch.equal(left, brute[0]) and torch.equal(right, brute[1])
+""")
+
+
+@needs_nvcc
+@pytest.mark.parametrize("blocks", [1, 7])
+def test_training_in_fewer_blocks(tmp_path, blocks):
+    """Training blocks that take turns at the samples (a GPU that holds fewer of them) end in a model as good (its
+    gradients differ in the order of their FP32 sums only: the lookup windows within 1% of each other) and in the
+    pairs of the tree."""
+    lib = _library(tmp_path, {"learned": [f"-DVS_TRAIN_BLOCKS={blocks}"]})
+    _run(lib, f"""
+few, whole = _abi._lib, _abi.load({str(_build.LIB)!r})
+w = syn.utm_join(seed=3, n_points=400_003, n_polys=30_000)  # over 16384 cells: 128 lots of samples
+polys = [dev(getattr(w.polys, k)) for k in ("x", "y", "ring_off", "part_off", "geom_off")]
+dx, dy = dev(w.px), dev(w.py)
+pts = _abi.make_points(dx, dy)
+index = _abi.DeviceIndex(ctx, _abi.make_polygons(*polys), learned=True)
+for flags in (0, _abi.JOIN_LEARNED_NO_STAGE):
+    left, right, _ = index.join(pts, _abi.PRED_WITHIN, _abi.METHOD_LEARNED, flags=flags)
+    tree = index.join(pts, _abi.PRED_WITHIN, _abi.METHOD_RTREE)
+    assert left.numel() > 0 and torch.equal(left, tree[0]) and torch.equal(right, tree[1])
+window = index.info()["rmi_mean_window"]
+index.close()
+_abi._lib = whole
+expected = _abi.DeviceIndex(_abi.Context(0), _abi.make_polygons(*polys), learned=True).info()["rmi_mean_window"]
+print("windows", window, expected)
+assert expected > 4 and abs(window - expected) < 0.01 * expected, (window, expected)
 """)

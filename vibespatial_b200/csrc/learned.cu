@@ -399,7 +399,7 @@ __global__ void pack_leaves_kernel(int nl, const double2* __restrict__ ab, const
 constexpr int kTrainThreads = 128;
 constexpr int kTrainWarps = kTrainThreads / 32;
 constexpr int kTrainSamples = 16384;
-static_assert(kTrainSamples / kTrainThreads <= kNumSMs, "the training blocks run at once, one an SM");
+static_assert(kTrainSamples / kTrainThreads <= kNumSMs, "on a whole GPU every training block has an SM to itself");
 constexpr int kTrainStride = 36;  // floats a sample row: 16-byte rows whose lanes' stores miss one another's banks
 constexpr int kGradWords = 1160;  // kRmiP gradients, the loss, padding to 16 bytes
 constexpr int kLossWord = kRmiP;
@@ -436,7 +436,7 @@ struct TrainShared {
     double key_lo, key_scale;
     int fail;
 };
-static_assert(sizeof(TrainShared) <= 200 * 1024, "one block an SM");
+static_assert(sizeof(TrainShared) <= 200 * 1024, "a training block fits an SM");
 static_assert((offsetof(TrainShared, h1) & 15) == 0, "rows are read 16 bytes at a time");
 
 typedef unsigned long long f32x2;
@@ -457,6 +457,8 @@ __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
 }
 __device__ __forceinline__ ulonglong2 load4(const float* p) { return *reinterpret_cast<const ulonglong2*>(p); }
 
+// kSeveral: a block has more samples than it holds, and reads them again every step.
+template <bool kSeveral>
 __global__ void __launch_bounds__(kTrainThreads) rmi_train_kernel(const TrainArgs a) {
     extern __shared__ __align__(16) unsigned char s_raw[];
     TrainShared& sm = *reinterpret_cast<TrainShared*>(s_raw);
@@ -490,197 +492,205 @@ __global__ void __launch_bounds__(kTrainThreads) rmi_train_kernel(const TrainArg
     const int half = tid & 1, row0 = tid - half;
     bool live[2];
     float x[2], t[2];
+    auto take = [&](int chunk) {
 #pragma unroll
-    for (int q = 0; q < 2; ++q) {
-        const int s = blockIdx.x * kTrainThreads + row0 + q;
-        live[q] = s < a.S;
-        x[q] = t[q] = 0.f;
-        if (live[q]) {
-            const int64_t i = (int64_t)((double)s * (double)a.n / (double)a.S);
-            x[q] = __double2float_rn(((double)(a.keys[i] >> a.anc_shift) - key_lo) * key_scale);
-            t[q] = (float)((double)i / (double)a.n);
+        for (int q = 0; q < 2; ++q) {
+            const int s = chunk * kTrainThreads + row0 + q;
+            live[q] = s < a.S;
+            x[q] = t[q] = 0.f;
+            if (live[q]) {
+                const int64_t i = (int64_t)((double)s * (double)a.n / (double)a.S);
+                x[q] = __double2float_rn(((double)(a.keys[i] >> a.anc_shift) - key_lo) * key_scale);
+                t[q] = (float)((double)i / (double)a.n);
+            }
         }
-    }
-    sm.x[tid] = half ? x[1] : x[0];
+        sm.x[tid] = half ? x[1] : x[0];
+    };
+    const int chunks = kSeveral ? (a.S + kTrainThreads - 1) / kTrainThreads : (int)blockIdx.x + 1;
+    take(blockIdx.x);
     if (tid == 0) sm.fail = 0;
     __syncthreads();
     const float inv = 1.0f / (float)a.S;
     for (int step = 1; step <= a.steps; ++step) {
         float* grad = a.grad + (step % 3) * kGradWords;
-        // forward: both samples of the pair through this lane's half of the
-        // layer-2 units, so that a weight read from shared memory serves two
-        f32x2 h1[2][kRmiHidden / 2];
+        for (int chunk = blockIdx.x; chunk < chunks; chunk += gridDim.x) {
+            if (kSeveral) take(chunk);
+            // forward: both samples of the pair through this lane's half of the
+            // layer-2 units, so that a weight read from shared memory serves two
+            f32x2 h1[2][kRmiHidden / 2];
 #pragma unroll
-        for (int k = 0; k < kRmiHidden; k += 4) {
-            const float4 w = *reinterpret_cast<const float4*>(&sm.P[kOffW1 + k]);
-            const float4 c = *reinterpret_cast<const float4*>(&sm.P[kOffB1 + k]);
-#pragma unroll
-            for (int q = 0; q < 2; ++q) {
-                h1[q][k / 2] = pack2(fmaxf(fmaf(w.x, x[q], c.x), 0.f), fmaxf(fmaf(w.y, x[q], c.y), 0.f));
-                h1[q][k / 2 + 1] = pack2(fmaxf(fmaf(w.z, x[q], c.z), 0.f), fmaxf(fmaf(w.w, x[q], c.w), 0.f));
-            }
-        }
-        float y[2] = {0.f, 0.f};
-#pragma unroll 1
-        for (int j = 2 * half; j < kRmiHidden; j += 4) {
-            float h2[2][2];
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                f32x2 za[2], zb[2];
+            for (int k = 0; k < kRmiHidden; k += 4) {
+                const float4 w = *reinterpret_cast<const float4*>(&sm.P[kOffW1 + k]);
+                const float4 c = *reinterpret_cast<const float4*>(&sm.P[kOffB1 + k]);
 #pragma unroll
                 for (int q = 0; q < 2; ++q) {
-                    za[q] = pack2(sm.P[kOffB2 + j + u], 0.f);
-                    zb[q] = 0ull;
+                    h1[q][k / 2] = pack2(fmaxf(fmaf(w.x, x[q], c.x), 0.f), fmaxf(fmaf(w.y, x[q], c.y), 0.f));
+                    h1[q][k / 2 + 1] = pack2(fmaxf(fmaf(w.z, x[q], c.z), 0.f), fmaxf(fmaf(w.w, x[q], c.w), 0.f));
                 }
+            }
+            float y[2] = {0.f, 0.f};
+#pragma unroll 1
+            for (int j = 2 * half; j < kRmiHidden; j += 4) {
+                float h2[2][2];
 #pragma unroll
-                for (int k = 0; k < kRmiHidden; k += 4) {
-                    const ulonglong2 w = load4(&sm.w2[j + u][k]);
+                for (int u = 0; u < 2; ++u) {
+                    f32x2 za[2], zb[2];
 #pragma unroll
                     for (int q = 0; q < 2; ++q) {
-                        za[q] = fma2(w.x, h1[q][k / 2], za[q]);
-                        zb[q] = fma2(w.y, h1[q][k / 2 + 1], zb[q]);
+                        za[q] = pack2(sm.P[kOffB2 + j + u], 0.f);
+                        zb[q] = 0ull;
+                    }
+#pragma unroll
+                    for (int k = 0; k < kRmiHidden; k += 4) {
+                        const ulonglong2 w = load4(&sm.w2[j + u][k]);
+#pragma unroll
+                        for (int q = 0; q < 2; ++q) {
+                            za[q] = fma2(w.x, h1[q][k / 2], za[q]);
+                            zb[q] = fma2(w.y, h1[q][k / 2 + 1], zb[q]);
+                        }
+                    }
+                    const float w3 = sm.P[kOffW3 + j + u];
+#pragma unroll
+                    for (int q = 0; q < 2; ++q) {
+                        const float2 a2 = unpack2(za[q]), b2 = unpack2(zb[q]);
+                        h2[q][u] = fmaxf((a2.x + a2.y) + (b2.x + b2.y), 0.f);
+                        y[q] = fmaf(w3, h2[q][u], y[q]);
                     }
                 }
-                const float w3 = sm.P[kOffW3 + j + u];
+#pragma unroll
+                for (int q = 0; q < 2; ++q)
+                    *reinterpret_cast<float2*>(&sm.h2[row0 + q][j]) = make_float2(h2[q][0], h2[q][1]);
+            }
+            float gy[2];
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                y[q] += __shfl_xor_sync(0xffffffffu, y[q], 1);
+                const float e = live[q] ? (y[q] + sm.P[kOffB3]) - t[q] : 0.f;
+                gy[q] = 2.f * e * inv;
+                if (q == half) {
+                    sm.gy[tid] = gy[q];
+                    sm.sq[tid] = e * e * inv;
+                }
+            }
+            // backward
+            f32x2 dh[2][kRmiHidden / 2];
+#pragma unroll
+            for (int k = 0; k < kRmiHidden / 2; ++k) dh[0][k] = dh[1][k] = 0ull;
+#pragma unroll
+            for (int k = 0; k < kRmiHidden / 2; k += 2)
+                *reinterpret_cast<ulonglong2*>(&sm.h1[tid][2 * k]) =
+                    half ? make_ulonglong2(h1[1][k], h1[1][k + 1]) : make_ulonglong2(h1[0][k], h1[0][k + 1]);
+#pragma unroll 1
+            for (int j = 2 * half; j < kRmiHidden; j += 4) {
+                float d[2][2], g2[2][2];
 #pragma unroll
                 for (int q = 0; q < 2; ++q) {
-                    const float2 a2 = unpack2(za[q]), b2 = unpack2(zb[q]);
-                    h2[q][u] = fmaxf((a2.x + a2.y) + (b2.x + b2.y), 0.f);
-                    y[q] = fmaf(w3, h2[q][u], y[q]);
+                    const float2 h = *reinterpret_cast<const float2*>(&sm.h2[row0 + q][j]);
+                    d[q][0] = h.x > 0.f ? gy[q] * sm.P[kOffW3 + j] : 0.f;
+                    d[q][1] = h.y > 0.f ? gy[q] * sm.P[kOffW3 + j + 1] : 0.f;
+                    g2[q][0] = gy[q] * h.x;
+                    g2[q][1] = gy[q] * h.y;
+                }
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    const f32x2 d0 = pack2(d[0][u], d[0][u]), d1 = pack2(d[1][u], d[1][u]);
+#pragma unroll
+                    for (int k = 0; k < kRmiHidden; k += 4) {
+                        const ulonglong2 w = load4(&sm.w2[j + u][k]);
+                        dh[0][k / 2] = fma2(w.x, d0, dh[0][k / 2]);
+                        dh[0][k / 2 + 1] = fma2(w.y, d0, dh[0][k / 2 + 1]);
+                        dh[1][k / 2] = fma2(w.x, d1, dh[1][k / 2]);
+                        dh[1][k / 2 + 1] = fma2(w.y, d1, dh[1][k / 2 + 1]);
+                    }
+                }
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    *reinterpret_cast<float2*>(&sm.d2[row0 + q][j]) = make_float2(d[q][0], d[q][1]);
+                    *reinterpret_cast<float2*>(&sm.h2[row0 + q][j]) = make_float2(g2[q][0], g2[q][1]);
                 }
             }
+            // this lane's sample: its own half of the sums plus the other lane's
 #pragma unroll
-            for (int q = 0; q < 2; ++q)
-                *reinterpret_cast<float2*>(&sm.h2[row0 + q][j]) = make_float2(h2[q][0], h2[q][1]);
-        }
-        float gy[2];
+            for (int k = 0; k < kRmiHidden / 2; k += 2) {
+                float v[4];
 #pragma unroll
-        for (int q = 0; q < 2; ++q) {
-            y[q] += __shfl_xor_sync(0xffffffffu, y[q], 1);
-            const float e = live[q] ? (y[q] + sm.P[kOffB3]) - t[q] : 0.f;
-            gy[q] = 2.f * e * inv;
-            if (q == half) {
-                sm.gy[tid] = gy[q];
-                sm.sq[tid] = e * e * inv;
-            }
-        }
-        // backward
-        f32x2 dh[2][kRmiHidden / 2];
-#pragma unroll
-        for (int k = 0; k < kRmiHidden / 2; ++k) dh[0][k] = dh[1][k] = 0ull;
-#pragma unroll
-        for (int k = 0; k < kRmiHidden / 2; k += 2)
-            *reinterpret_cast<ulonglong2*>(&sm.h1[tid][2 * k]) =
-                half ? make_ulonglong2(h1[1][k], h1[1][k + 1]) : make_ulonglong2(h1[0][k], h1[0][k + 1]);
-#pragma unroll 1
-        for (int j = 2 * half; j < kRmiHidden; j += 4) {
-            float d[2][2], g2[2][2];
-#pragma unroll
-            for (int q = 0; q < 2; ++q) {
-                const float2 h = *reinterpret_cast<const float2*>(&sm.h2[row0 + q][j]);
-                d[q][0] = h.x > 0.f ? gy[q] * sm.P[kOffW3 + j] : 0.f;
-                d[q][1] = h.y > 0.f ? gy[q] * sm.P[kOffW3 + j + 1] : 0.f;
-                g2[q][0] = gy[q] * h.x;
-                g2[q][1] = gy[q] * h.y;
-            }
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                const f32x2 d0 = pack2(d[0][u], d[0][u]), d1 = pack2(d[1][u], d[1][u]);
-#pragma unroll
-                for (int k = 0; k < kRmiHidden; k += 4) {
-                    const ulonglong2 w = load4(&sm.w2[j + u][k]);
-                    dh[0][k / 2] = fma2(w.x, d0, dh[0][k / 2]);
-                    dh[0][k / 2 + 1] = fma2(w.y, d0, dh[0][k / 2 + 1]);
-                    dh[1][k / 2] = fma2(w.x, d1, dh[1][k / 2]);
-                    dh[1][k / 2 + 1] = fma2(w.y, d1, dh[1][k / 2 + 1]);
+                for (int u = 0; u < 2; ++u) {
+                    const float2 keep = unpack2(half ? dh[1][k + u] : dh[0][k + u]);
+                    const float2 send = unpack2(half ? dh[0][k + u] : dh[1][k + u]);
+                    const float2 h = unpack2(half ? h1[1][k + u] : h1[0][k + u]);
+                    const float gx = keep.x + __shfl_xor_sync(0xffffffffu, send.x, 1);
+                    const float gz = keep.y + __shfl_xor_sync(0xffffffffu, send.y, 1);
+                    v[2 * u] = h.x > 0.f ? gx : 0.f;
+                    v[2 * u + 1] = h.y > 0.f ? gz : 0.f;
                 }
+                *reinterpret_cast<float4*>(&sm.d1[tid][2 * k]) = make_float4(v[0], v[1], v[2], v[3]);
             }
+            __syncwarp();
+            // the warp's 32 samples: W2 gradient, rows 4 jr.. x columns 8 kc..
+            {
+                const int jr = 4 * (lane >> 2), kc = 8 * (lane & 3);
+                f32x2 g[4][4];
 #pragma unroll
-            for (int q = 0; q < 2; ++q) {
-                *reinterpret_cast<float2*>(&sm.d2[row0 + q][j]) = make_float2(d[q][0], d[q][1]);
-                *reinterpret_cast<float2*>(&sm.h2[row0 + q][j]) = make_float2(g2[q][0], g2[q][1]);
-            }
-        }
-        // this lane's sample: its own half of the sums plus the other lane's
+                for (int u = 0; u < 4; ++u)
 #pragma unroll
-        for (int k = 0; k < kRmiHidden / 2; k += 2) {
-            float v[4];
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                const float2 keep = unpack2(half ? dh[1][k + u] : dh[0][k + u]);
-                const float2 send = unpack2(half ? dh[0][k + u] : dh[1][k + u]);
-                const float2 h = unpack2(half ? h1[1][k + u] : h1[0][k + u]);
-                const float gx = keep.x + __shfl_xor_sync(0xffffffffu, send.x, 1);
-                const float gz = keep.y + __shfl_xor_sync(0xffffffffu, send.y, 1);
-                v[2 * u] = h.x > 0.f ? gx : 0.f;
-                v[2 * u + 1] = h.y > 0.f ? gz : 0.f;
-            }
-            *reinterpret_cast<float4*>(&sm.d1[tid][2 * k]) = make_float4(v[0], v[1], v[2], v[3]);
-        }
-        __syncwarp();
-        // the warp's 32 samples: W2 gradient, rows 4 jr.. x columns 8 kc..
-        {
-            const int jr = 4 * (lane >> 2), kc = 8 * (lane & 3);
-            f32x2 g[4][4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-#pragma unroll
-                for (int v = 0; v < 4; ++v) g[u][v] = 0ull;
-            float gw1 = 0.f, gb1 = 0.f, gb2 = 0.f, gw3 = 0.f, gb3 = 0.f, l2 = 0.f;
+                    for (int v = 0; v < 4; ++v) g[u][v] = 0ull;
+                float gw1 = 0.f, gb1 = 0.f, gb2 = 0.f, gw3 = 0.f, gb3 = 0.f, l2 = 0.f;
 #pragma unroll 4
-            for (int q = 0; q < 32; ++q) {
-                const int r = warp * 32 + q;
-                const float4 d = *reinterpret_cast<const float4*>(&sm.d2[r][jr]);
-                const ulonglong2 ha = load4(&sm.h1[r][kc]), hb = load4(&sm.h1[r][kc + 4]);
-                const float du[4] = {d.x, d.y, d.z, d.w};
+                for (int q = 0; q < 32; ++q) {
+                    const int r = warp * 32 + q;
+                    const float4 d = *reinterpret_cast<const float4*>(&sm.d2[r][jr]);
+                    const ulonglong2 ha = load4(&sm.h1[r][kc]), hb = load4(&sm.h1[r][kc + 4]);
+                    const float du[4] = {d.x, d.y, d.z, d.w};
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        const f32x2 dd = pack2(du[u], du[u]);
+                        g[u][0] = fma2(ha.x, dd, g[u][0]);
+                        g[u][1] = fma2(ha.y, dd, g[u][1]);
+                        g[u][2] = fma2(hb.x, dd, g[u][2]);
+                        g[u][3] = fma2(hb.y, dd, g[u][3]);
+                    }
+                    const float d1 = sm.d1[r][lane];
+                    gw1 = fmaf(d1, sm.x[r], gw1);
+                    gb1 += d1;
+                    gb2 += sm.d2[r][lane];
+                    gw3 += sm.h2[r][lane];
+                    gb3 += sm.gy[r];
+                    l2 += sm.sq[r];
+                }
+                float* part = sm.part[warp];
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+#pragma unroll
+                    for (int v = 0; v < 4; ++v) {
+                        const float2 w = unpack2(g[u][v]);
+                        part[kOffW2 + (jr + u) * kRmiHidden + kc + 2 * v] = w.x;
+                        part[kOffW2 + (jr + u) * kRmiHidden + kc + 2 * v + 1] = w.y;
+                    }
+                part[kOffW1 + lane] = gw1;
+                part[kOffB1 + lane] = gb1;
+                part[kOffB2 + lane] = gb2;
+                part[kOffW3 + lane] = gw3;
+                if (lane == 0) {
+                    part[kOffB3] = gb3;
+                    part[kLossWord] = l2;
+                }
+            }
+            __syncthreads();
+            for (int i = 4 * tid; i <= kLossWord; i += 4 * kTrainThreads) {
+                float v[4];
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
-                    const f32x2 dd = pack2(du[u], du[u]);
-                    g[u][0] = fma2(ha.x, dd, g[u][0]);
-                    g[u][1] = fma2(ha.y, dd, g[u][1]);
-                    g[u][2] = fma2(hb.x, dd, g[u][2]);
-                    g[u][3] = fma2(hb.y, dd, g[u][3]);
+                    v[u] = 0.f;
+                    if (i + u <= kLossWord) {
+#pragma unroll
+                        for (int w = 0; w < kTrainWarps; ++w) v[u] += sm.part[w][i + u];
+                    }
                 }
-                const float d1 = sm.d1[r][lane];
-                gw1 = fmaf(d1, sm.x[r], gw1);
-                gb1 += d1;
-                gb2 += sm.d2[r][lane];
-                gw3 += sm.h2[r][lane];
-                gb3 += sm.gy[r];
-                l2 += sm.sq[r];
+                asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(grad + i), "f"(v[0]),
+                             "f"(v[1]), "f"(v[2]), "f"(v[3])
+                             : "memory");
             }
-            float* part = sm.part[warp];
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-#pragma unroll
-                for (int v = 0; v < 4; ++v) {
-                    const float2 w = unpack2(g[u][v]);
-                    part[kOffW2 + (jr + u) * kRmiHidden + kc + 2 * v] = w.x;
-                    part[kOffW2 + (jr + u) * kRmiHidden + kc + 2 * v + 1] = w.y;
-                }
-            part[kOffW1 + lane] = gw1;
-            part[kOffB1 + lane] = gb1;
-            part[kOffB2 + lane] = gb2;
-            part[kOffW3 + lane] = gw3;
-            if (lane == 0) {
-                part[kOffB3] = gb3;
-                part[kLossWord] = l2;
-            }
-        }
-        __syncthreads();
-        for (int i = 4 * tid; i <= kLossWord; i += 4 * kTrainThreads) {
-            float v[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                v[u] = 0.f;
-                if (i + u <= kLossWord) {
-#pragma unroll
-                    for (int w = 0; w < kTrainWarps; ++w) v[u] += sm.part[w][i + u];
-                }
-            }
-            asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(grad + i), "f"(v[0]),
-                         "f"(v[1]), "f"(v[2]), "f"(v[3])
-                         : "memory");
+            if (kSeveral) __syncthreads();  // (part and x are written again)
         }
         // the buffer of the step before last is read by no block any more: zero it for the step after this one
         float* next = a.grad + ((step + 1) % 3) * kGradWords;
@@ -911,12 +921,24 @@ int train_rmi(vs_context* ctx, vs_index* idx, int steps) {
     ta.loss = grad.p + 3 * kGradWords;
     ta.model = li.model;
     ta.err = &ctx->d_counters[kStatus];
-    // The blocks meet at a barrier every step: a cooperative launch, so all of them run at once.
-    VS_CUDA_TRY(cudaFuncSetAttribute(rmi_train_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)sizeof(TrainShared)));
+    // The blocks meet at a barrier every step: a cooperative launch, so all of them run at once.  A device (or a share
+    // of one) that cannot hold a block for every 128 samples gets fewer, which take turns at them.
     void* args[] = {(void*)&ta};
-    VS_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)rmi_train_kernel, dim3(div_up(ta.S, kTrainThreads)),
-                                            dim3(kTrainThreads), args, sizeof(TrainShared), s));
+    int grid = (int)div_up(ta.S, kTrainThreads);
+#ifdef VS_TRAIN_BLOCKS  // (a build may lower it to test that)
+    grid = std::min(grid, VS_TRAIN_BLOCKS);
+#endif
+    for (;; grid = (grid + 1) / 2) {
+        const auto* kernel = (const void*)(grid * kTrainThreads < ta.S ? rmi_train_kernel<true> : rmi_train_kernel<false>);
+        VS_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TrainShared)));
+        const cudaError_t e = cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(kTrainThreads), args,
+                                                          sizeof(TrainShared), s);
+        if (e != cudaErrorCooperativeLaunchTooLarge || grid == 1) {
+            VS_CUDA_TRY(e);
+            break;
+        }
+        cudaGetLastError();
+    }
     VS_LAUNCHED("rmi_train", s);
     VS_CUDA_TRY(cudaMemcpyAsync(&li.rmi_final_loss, ta.loss, sizeof(float), cudaMemcpyDeviceToHost, s));
     // tabulate the root over all 4^R ancestor keys
