@@ -401,7 +401,8 @@ int vs_row_counts(vs_context* ctx, const int32_t* d_rows, const uint8_t* d_mask,
 
 /* d_sums[r] = sum of d_values[d_cols[k]] over the pairs k with d_rows[k] == r,
  * added in pair order (so equal to numpy's bincount(rows, weights=...)); the
- * rows must ascend (VS_E_ARG otherwise), as a join's sorted pairs do. */
+ * rows must ascend (VS_E_ARG otherwise, d_sums untouched), as a join's sorted
+ * pairs do. */
 int vs_row_sums(vs_context* ctx, const int32_t* d_rows, const int32_t* d_cols, int64_t n_pairs, int64_t n_rows,
                 const double* d_values, int64_t n_values, double* d_sums);
 

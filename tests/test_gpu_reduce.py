@@ -76,3 +76,21 @@ def test_row_range_errors(vsabi, ctx):
         vsabi.row_counts(ctx, _dev(rows), 5)
     with pytest.raises(ValueError, match="outside"):
         vsabi.row_counts(ctx, _dev(np.array([-1], np.int32)), 5)
+
+
+@pytest.mark.parametrize("n_rows", [3, 1000])  # a warp a row, a thread a row
+@pytest.mark.parametrize("rows", ["descending", "below", "above"])
+def test_row_sums_leaves_its_output_alone_on_bad_rows(vsabi, ctx, n_rows, rows):
+    import torch
+
+    r = np.sort(np.random.default_rng(6).integers(0, n_rows, 1500)).astype(np.int32)
+    if rows == "descending":
+        r = r[::-1].copy()
+    else:
+        r[0 if rows == "below" else -1] = -1 if rows == "below" else n_rows
+    dr, dc, dv = _dev(r), _dev(np.zeros(len(r), np.int32)), _dev(np.ones(4))
+    out = torch.full((n_rows,), -7.0, dtype=torch.float64, device="cuda")
+    with pytest.raises(ValueError):
+        vsabi.check(vsabi.load().vs_row_sums(ctx.handle, dr.data_ptr(), dc.data_ptr(), len(r), n_rows, dv.data_ptr(), 4,
+                                             out.data_ptr()))
+    assert bool((out == -7.0).all())

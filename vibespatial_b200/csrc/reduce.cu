@@ -57,6 +57,7 @@ __global__ void descent_kernel(const int32_t* __restrict__ rows, int64_t n, unsi
 __global__ void row_sum_kernel(const uint64_t* __restrict__ off, int64_t n_rows, const int32_t* __restrict__ cols,
                                const double* __restrict__ values, int64_t n_values, double* __restrict__ sums,
                                unsigned* __restrict__ bad) {
+    if (*bad & 3u) return;  // rows out of range or out of order: sums is left as it was
     for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n_rows; r += (int64_t)gridDim.x * blockDim.x) {
         double acc = 0.0;
         for (uint64_t k = off[r]; k < off[r + 1]; ++k) {
@@ -78,6 +79,7 @@ __global__ void __launch_bounds__(kRThreads) row_sum_warp_kernel(const uint64_t*
                                                                  const int32_t* __restrict__ cols,
                                                                  const double* __restrict__ values, int64_t n_values,
                                                                  double* __restrict__ sums, unsigned* __restrict__ bad) {
+    if (*bad & 3u) return;  // rows out of range or out of order: sums is left as it was
     const int lane = threadIdx.x & 31;
     const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
     for (int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < n_rows; r += nw) {
@@ -237,7 +239,7 @@ extern "C" int vs_row_sums(vs_context* ctx, const int32_t* d_rows, const int32_t
     }
     VS_TRY(exclusive_scan_u64(reinterpret_cast<uint64_t*>(off.p), reinterpret_cast<uint64_t*>(off.p), n_rows,
                               reinterpret_cast<uint64_t*>(off.p) + n_rows, s));
-    // (the offsets stay within the pairs whatever the rows are: only rows in range are counted)
+    // (the host reads what the passes above say of the rows after the sums: these look themselves)
     if (n_pairs >= kWarpRowPairs * n_rows) {
         row_sum_warp_kernel<<<grid_for(n_rows * 32, kRThreads), kRThreads, 0, s>>>(
             reinterpret_cast<const uint64_t*>(off.p), n_rows, d_cols, d_values, n_values, d_sums, bad.p);
