@@ -320,7 +320,9 @@ typedef struct vs_batch_options {
                                              48-register one */
     int32_t learned_grab;     /* learned: grouped points a refine warp takes per grab (0 = 32; rounded up to 32s) */
     uint32_t learned_flags;   /* learned: VS_JOIN_LEARNED_BSEARCH | _FP64_WALK | _NO_STAGE | _NO_INTERIOR (ablations) */
-    int32_t learned_map_packets; /* learned: 32-point packets a map warp looks up together, 1 or 2 (0 = 1) */
+    int32_t learned_map_packets; /* learned: 32-point packets a map warp looks up together, 1 or 2 (0 = 1); of no
+                                    effect where the indexes' own shape decides the map pass (from 2^21 points on
+                                    indexes that store few of their grid's cells) */
 } vs_batch_options;
 
 /* At most 4096 jobs and 2^31-1 points in total. */

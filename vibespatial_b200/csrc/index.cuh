@@ -114,7 +114,8 @@ struct LearnedShape {
     int32_t refine_blocks_per_sm;  // refine pass blocks per SM (0 = as many as fit)
     int32_t grab;                  // grouped points a refine warp takes per work grab (0 = 32; multiple of 32)
     uint32_t flags;                // kLearnedBsearch | kLearnedFp64Walk | kLearnedNoStage | kLearnedNoInterior
-    int32_t map_packets;           // 32-point packets a map warp looks up together (1 or 2; 0 = 1)
+    int32_t map_packets;           // 32-point packets a map warp looks up together (1 or 2; 0 = 1); not used
+                                   // by the map pass of sparse indexes (kSparseMapPoints)
 };
 constexpr uint32_t kLearnedBsearch = 1u;   // cell lookup by binary search over all cell keys (no RMI)
 constexpr uint32_t kLearnedFp64Walk = 2u;  // ring walks in FP64 (no FP32 edge stage)

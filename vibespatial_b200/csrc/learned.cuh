@@ -49,6 +49,13 @@ struct LearnedQuery {
 // are (most hit), share 0.010: 85 and 165, 0.037: 134 and 173, 0.082: 198 and
 // 184; a full grid (0.90): 266 and 229.
 inline bool sparse_map_pays(int64_t n_cells, int64_t grid_cells) { return n_cells < grid_cells / 16; }
+// Points from which it pays there: below, units large enough for whole lookups
+// are too few to go round, and smaller ones wait for their counter.  One join
+// over an index of 20k footprints (share 0.005), us with and without: 0.3M
+// points 55 and 48, 1M 71 and 61, 2M 75 and 75, 2.5M 73 and 83, 5M 100 and 120,
+// 12M 151 and 210; of 3k (0.0006): 1M 63 and 51, 2M 67 and 61, 2.5M 63 and 67;
+// of 100k (0.02): 1M 117 and 106, 2M 135 and 132, 2.5M 134 and 143.
+constexpr int64_t kSparseMapPoints = 1 << 21;
 
 // Enqueue map -> scan -> place -> refine on stream s (no host
 // synchronisation; capturable).  For one job, `single` is its descriptor

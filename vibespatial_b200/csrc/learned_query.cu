@@ -331,10 +331,10 @@ struct PendingPoint {
 // eight: they let a warp fill whole lookups from sparse hits, and every unit
 // costs an increment of the one counter they are handed out from (about 1 ns,
 // measured: 10M points in units of two packets took 149 us, of eight 83 us).
-// Fewer points make smaller units, so that a warp still gets several.
+// Fewer points make smaller units, so that a warp still gets several.  (Below
+// kSparseMapPoints a unit is a packet: only the other pass runs there.)
 __host__ __device__ __forceinline__ int unit_packets(int64_t n) {
-    const int64_t packets = (n + 31) / 32;
-    return packets >= 8 * 32 * 1024 ? 8 : packets >= 4 * 16 * 1024 ? 4 : packets >= 2 * 16 * 1024 ? 2 : 1;
+    return n >= 4 * kSparseMapPoints ? 8 : n >= kSparseMapPoints ? 4 : 1;
 }
 
 // Look up to 32 pending points up, count their cells and append the matched
@@ -1097,7 +1097,7 @@ int launch_passes(cudaStream_t s, vs_context* ctx, const LqArgs& a) {
     if (sh.flags & kLearnedBsearch) {
         if (two) learned_map_kernel<kMulti, true, 2><<<map_grid, kThreads, 0, s>>>(a);
         else learned_map_kernel<kMulti, true, 1><<<map_grid, kThreads, 0, s>>>(a);
-    } else if (a.q.sparse && sh.map_packets == 0) {
+    } else if (a.q.sparse && n >= kSparseMapPoints) {
         learned_map_sparse_kernel<kMulti><<<map_grid, kThreads, 0, s>>>(a);
     } else {
         if (two) learned_map_kernel<kMulti, false, 2><<<map_grid, kThreads, 0, s>>>(a);
