@@ -56,3 +56,56 @@ def test_equal_points_around_the_list_size(ctx, vsabi, oracle, k):
         np.testing.assert_array_equal(gl.cpu().numpy(), el)
         np.testing.assert_array_equal(gr.cpu().numpy(), er)
         np.testing.assert_array_equal(gd.cpu().numpy().view(np.int64), ed.view(np.int64))
+
+
+def _time(f):
+    import time
+
+    import torch
+
+    f()
+    best = 1e9
+    for _ in range(5):
+        torch.cuda.synchronize()
+        t = time.perf_counter()
+        f()
+        torch.cuda.synchronize()
+        best = min(best, time.perf_counter() - t)
+    return best
+
+
+@pytest.mark.parametrize("k", [5, 6, 7, 12])
+@pytest.mark.parametrize("side", ["points", "polygons"])
+def test_time_grows_with_the_copies(ctx, vsabi, side, k):
+    """Every polygon (point) k times: k times the pairs, for at most five times as much time a pair as without copies,
+    also where the single walk leaves some or all queries to the exact walks (a mixture of far-apart queries in their
+    packets took 39 times as long for 6 copies of the polygons, 310 for 5 of the points)."""
+    import torch
+
+    w = syn.utm_join(seed=3, n_points=150_000, n_polys=5_000)
+    q = w.polys
+
+    def run(copies):
+        sizes = np.diff(q.ring_off)
+        if side == "polygons":
+            sizes = np.tile(sizes, copies)
+            xs, ys, px, py = np.tile(q.x, copies), np.tile(q.y, copies), w.px, w.py
+        else:
+            xs, ys, px, py = q.x, q.y, np.tile(w.px[:50_000], copies), np.tile(w.py[:50_000], copies)
+        polys = syn._rings_to_soa(sizes, xs, ys)
+        t = [torch.from_numpy(np.ascontiguousarray(getattr(polys, a))).cuda()
+             for a in ("x", "y", "ring_off", "part_off", "geom_off")]
+        P = vsabi.make_polygons(*t)
+        dx, dy = torch.from_numpy(px).cuda(), torch.from_numpy(py).cuda()
+        if side == "polygons":
+            index, pts = vsabi.DeviceIndex(ctx, P), vsabi.make_points(dx, dy)
+            return index.nearest(pts)[0].numel(), _time(lambda: index.nearest(pts, sort=False))
+        index = vsabi.point_index(ctx, dx, dy)
+        return (vsabi.nearest_polygons(ctx, index, P)[0].numel(),
+                _time(lambda: vsabi.nearest_polygons(ctx, index, P, sort=False)))
+
+    pairs_one, one = run(1)
+    pairs, many = run(k)
+    assert pairs == k * pairs_one
+    print(side, k, one, many, many / one)
+    assert many < 5 * k * one, (one, many)

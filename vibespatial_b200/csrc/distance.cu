@@ -226,8 +226,9 @@ struct DistArgs {
     const double* px;
     const double* py;
     const uint32_t* order;   // sorted position -> point row
-    const uint32_t* list;    // positions to visit (nullable: every position below *n_list)
-    const uint32_t* n_list;
+    const uint32_t* n_valid; // dwithin: sorted positions
+    const uint2* packets;    // nearest: packets left to the exact walks (OverPackets)
+    const uint32_t* n_packets;
     const vs_box* nodes;
     int64_t level_off[kMaxLevels];
     int64_t level_size[kMaxLevels];
@@ -243,8 +244,8 @@ struct DistArgs {
     const double* dist_pt;    // dwithin: per point row (nullable)
     const double* dist_geom;  // dwithin: per polygon row (nullable)
     double dist_scalar;       // dwithin: the distance, or the largest per-polygon one
-    double radius;            // nearest, min pass: the search radius of this pass
-    double* best;             // nearest: per point row minimum distance
+    double radius;            // nearest: the search cap
+    double* best;             // nearest: per point row minimum distance (min pass: an upper bound of it at first)
     PairSink sink;
     unsigned long long* counters;
     unsigned long long* work;
@@ -303,10 +304,11 @@ __device__ __noinline__ double listed_distance(const DistArgs& a, double x, doub
 // Warp-packet R-tree walk of the distance joins.
 //   kDwithin      per lane radius d (per point / per polygon / scalar); emits
 //                 the pairs within it
-//   kNearestMin   per lane minimum distance: each lane's greedy descent
-//                 (level by level the child box nearest to its point, ties
-//                 broken by the box centre, then the nearest item box) gives
-//                 it an upper bound; the walk then
+//   kNearestMin   per lane minimum distance: it starts from the upper bound
+//                 in best[row], or where that is no better than the cap, from
+//                 a greedy descent (level by level the child box nearest to
+//                 its point, ties broken by the box centre, then the nearest
+//                 item box); the walk then
 //                 visits, nearest to the packet's centroid first, what lies
 //                 within each lane's current minimum (capped by max_distance
 //                 in a.radius), the packet's box shrinking as the minima
@@ -358,23 +360,26 @@ __global__ void __launch_bounds__(kDistThreads) dist_join_kernel(const DistArgs 
     };
     const unsigned lt = (1u << lane) - 1u;
     const int top = a.levels - 1;
-    const int64_t n = (int64_t)*a.n_list;
+    const int64_t n = kMode == kDwithin ? (int64_t)*a.n_valid : kDistGrab * (int64_t)*a.n_packets;
     unsigned long long n_cand = 0;
     unsigned n_exact = 0;
     for (;;) {
         const int64_t b0 = warp_grab(a.work, kDistGrab);
         if (b0 >= n) break;
-        const int64_t i = b0 + lane;
+        int64_t i = b0 + lane;
         bool active = i < n;
+        if (kMode != kDwithin) {
+            const uint2 packet = a.packets[b0 / kDistGrab];
+            i = (int64_t)packet.x + lane;
+            active = (packet.y >> lane) & 1u;
+        }
         double x = 0.0, y = 0.0, q = 0.0;
         int32_t row = -1;
         if (active) {
-            const uint32_t pos = a.list ? a.list[i] : (uint32_t)i;
-            row = (int32_t)a.order[pos];
+            row = (int32_t)a.order[i];
             x = a.px[row];
             y = a.py[row];
             if (kMode == kDwithin) q = a.dist_pt ? a.dist_pt[row] : a.dist_scalar;
-            else if (kMode == kNearestMin) q = a.radius;  // the cap (max_distance or INFINITY)
             else q = a.best[row];
             // a negative or NaN radius matches nothing; nearest emits only finite minima
             active = q >= 0.0 && (kMode != kNearestEmit || q < INFINITY);
@@ -396,7 +401,7 @@ __global__ void __launch_bounds__(kDistThreads) dist_join_kernel(const DistArgs 
             // every lane descends on its own: at each level the child box nearest to
             // its point, then the exact distance to the nearest item box of the
             // leaf block reached -- an upper bound of the lane's minimum
-            if (active) {
+            if (active && !(q < a.radius)) {
                 int64_t node = 0;
                 bool ok = true;
                 for (int cl = top - 1; cl >= 1 && ok; --cl) {
@@ -521,7 +526,7 @@ __global__ void __launch_bounds__(kDistThreads) dist_join_kernel(const DistArgs 
                             // a polygon whose envelope is farther than the bound (with a
                             // margin above the rounding of both distances) can neither
                             // lower the minimum nor tie it
-                            const double bound = kMode == kNearestMin ? my_best : q;
+                            const double bound = kMode == kNearestMin ? fmin(my_best, q) : q;
                             // (a minimum of 0 cannot drop further: the min walk skips the rest)
                             if ((kMode != kNearestMin || my_best > 0.0) &&
                                 !(envelope_distance(ib, x, y) > bound * (1.0 + 0x1p-40))) {
@@ -753,18 +758,17 @@ __device__ __forceinline__ bool point_lane(bool finite, double x, double y, doub
 
 __device__ __forceinline__ bool finite_coordinate(double v) { return fabs(v) <= 1e300; }
 
-// Queries left to the FP64 walks.
-struct OverList {
-    uint32_t* items;
+// Queries left to the FP64 walks, as packets (sorted position of the first,
+// mask of the lanes): those of one packet lie together.  (Lists of single
+// queries put neighbours of several packets into one, whose box then holds all
+// that lies between them: 300k points on 3000 footprints, each present five
+// times, of which a few in every packet are left, took 7.1 ms.)
+struct OverPackets {
+    uint2* items;
     uint32_t* count;
-    __device__ __forceinline__ void add(bool over, uint32_t item) const {
+    __device__ __forceinline__ void add(bool over, int64_t first) const {
         const unsigned m = __ballot_sync(0xffffffffu, over);
-        if (!m) return;
-        const int lane = threadIdx.x & 31;
-        uint32_t base = 0;
-        if (lane == 0) base = atomicAdd(count, (uint32_t)__popc(m));
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if (over) items[base + __popc(m & ((1u << lane) - 1u))] = item;
+        if (m && (threadIdx.x & 31) == 0) items[atomicAdd(count, 1u)] = make_uint2((uint32_t)first, m);
     }
 };
 
@@ -802,7 +806,7 @@ struct NearList {
 
 struct NearArgs {
     DistArgs d;
-    OverList over;  // sorted positions left to dist_join_kernel
+    OverPackets over;  // left to dist_join_kernel
 };
 
 // Nearest polygons of points, all ties, in one walk: a polygon a lane reaches
@@ -826,7 +830,7 @@ __global__ void __launch_bounds__(kDistThreads, 3) near_kernel(const NearArgs na
     if (lane == 0) s_cnt[warp] = 0;
     __syncthreads();
     const WarpOut out{s_buf[warp], &s_cnt[warp]};
-    const int64_t n = (int64_t)*a.n_list;
+    const int64_t n = (int64_t)*a.n_valid;
     const float cap = __double2float_ru(a.radius);  // max_distance (INFINITY: unbounded)
     unsigned long long n_cand = 0;
     unsigned n_exact = 0;
@@ -925,7 +929,7 @@ __global__ void __launch_bounds__(kDistThreads, 3) near_kernel(const NearArgs na
             __syncwarp();
         }
         if (!(best <= a.radius)) best = INFINITY;
-        if (active && !over) a.best[row] = best;
+        if (active) a.best[row] = over ? fmin((double)pl.ub, a.radius) : best;
         if (!(best < INFINITY)) ties = 0;
         while (__any_sync(0xffffffffu, ties != 0)) {
             const bool want = ties != 0;
@@ -933,7 +937,7 @@ __global__ void __launch_bounds__(kDistThreads, 3) near_kernel(const NearArgs na
             ties &= ties - 1;
             wemit_sync(out, a.sink, want, row, want ? a.item_geom[s_near[warp].slot[k][lane]] : 0);
         }
-        na.over.add(over, (uint32_t)i);
+        na.over.add(over, b0);
         wflush(out, a.sink, false);
     }
     wflush(out, a.sink, true);
@@ -1138,6 +1142,8 @@ struct PolyArgs {
     const vs_box* qbox;         // envelopes (inverted for null / empty rows)
     const uint32_t* order;      // query rows, valid ones first
     const uint32_t* n_valid;
+    const uint2* packets;       // left to the exact walks (OverPackets)
+    const uint32_t* n_packets;
     const vs_box* nodes;        // the point index
     int64_t level_off[kMaxLevels];
     int64_t level_size[kMaxLevels];
@@ -1146,7 +1152,7 @@ struct PolyArgs {
     int staged;
     const int32_t* item_geom;   // slot -> point row
     double cap;                 // max_distance (INFINITY: unbounded)
-    double* best;               // per query row
+    double* best;               // per query row (min pass: an upper bound of it at first)
     PairSink sink;
     unsigned long long* counters;
     unsigned long long* work;
@@ -1229,7 +1235,7 @@ __global__ void __launch_bounds__(kDistThreads) poly_nearest_kernel(const PolyAr
     const WarpOut out{s_buf[warp], &s_cnt[warp]};
     const unsigned lt = (1u << lane) - 1u;
     const int top = a.levels - 1;
-    const int64_t n = (int64_t)*a.n_valid;
+    const int64_t n = kDistGrab * (int64_t)*a.n_packets;
     unsigned long long n_cand = 0;
     unsigned n_exact = 0;
     // tie walk: candidate points queue up here (point, the polygon's minimum,
@@ -1250,15 +1256,15 @@ __global__ void __launch_bounds__(kDistThreads) poly_nearest_kernel(const PolyAr
     for (;;) {
         const int64_t b0 = warp_grab(a.work, kDistGrab);
         if (b0 >= n) break;
-        const int64_t i = b0 + lane;
-        bool active = i < n;
+        const uint2 packet = a.packets[b0 / kDistGrab];
+        bool active = (packet.y >> lane) & 1u;
         int32_t row = -1;
         vs_box qb{INFINITY, INFINITY, -INFINITY, -INFINITY};
         double q = 0.0;
         if (active) {
-            row = (int32_t)a.order[i];
+            row = (int32_t)a.order[(int64_t)packet.x + lane];
             qb = a.qbox[row];
-            q = kEmit ? a.best[row] : a.cap;
+            q = a.best[row];
             active = q >= 0.0 && (!kEmit || q < INFINITY);
         }
         const double mx = 0.5 * (qb.minx + qb.maxx), my = 0.5 * (qb.miny + qb.maxy);
@@ -1272,7 +1278,7 @@ __global__ void __launch_bounds__(kDistThreads) poly_nearest_kernel(const PolyAr
             cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
         }
         const double cx = cnt ? sx / cnt : 0.0, cy = cnt ? sy / cnt : 0.0;
-        if (!kEmit && active) {
+        if (!kEmit && active && !(q < a.cap)) {
             // greedy descent towards the envelope centre, then the nearest point of the block
             int64_t node = 0;
             bool ok = true;
@@ -1388,7 +1394,7 @@ __global__ void __launch_bounds__(kDistThreads) poly_nearest_kernel(const PolyAr
                     bool queue = false;
                     if (active && ib.minx <= lx1 && ib.maxx >= lx0 && ib.miny <= ly1 && ib.maxy >= ly0) {
                         ++n_cand;
-                        const double bound = kEmit ? q : my_best;
+                        const double bound = kEmit ? q : fmin(my_best, q);
                         // (a minimum of 0 cannot drop further: the min walk skips the rest)
                         if ((kEmit || my_best > 0.0) &&
                             !(envelope_distance(qb, ib.minx, ib.miny) > bound * (1.0 + 0x1p-40))) {
@@ -1442,7 +1448,7 @@ __global__ void __launch_bounds__(kDistThreads) poly_nearest_kernel(const PolyAr
 // the box around all 32 polygons touched and computed exact distances there.
 struct PolyNearArgs {
     PolyArgs d;
-    OverList over;  // polygon rows left to the two walks
+    OverPackets over;  // left to the two walks
 };
 
 __device__ __noinline__ bool located_in(const PolyArgs& a, double px, double py, int g, unsigned& n_exact) {
@@ -1660,7 +1666,7 @@ __global__ void __launch_bounds__(kDistThreads, 3) poly_near_kernel(const PolyNe
             __syncwarp();
         }
         if (!(best <= a.cap)) best = INFINITY;
-        if (active && !over) a.best[row] = best;
+        if (active) a.best[row] = over ? fmin((double)pl.ub, a.cap) : best;
         if (!(best < INFINITY)) ties = 0;
         while (__any_sync(0xffffffffu, ties != 0)) {
             const bool want = ties != 0;
@@ -1668,7 +1674,7 @@ __global__ void __launch_bounds__(kDistThreads, 3) poly_near_kernel(const PolyNe
             ties &= ties - 1;
             wemit_sync(out, a.sink, want, row, want ? a.item_geom[near.slot[k][lane]] : 0);
         }
-        na.over.add(over, (uint32_t)row);
+        na.over.add(over, b0);
         wflush(out, a.sink, false);
     }
     wflush(out, a.sink, true);
@@ -1717,7 +1723,7 @@ int vs_join_dwithin(vs_context* ctx, const vs_index* idx, const vs_points* pts, 
     VS_TRY(prepare_queries(ctx, idx, pts, q, true));
     size_t smem = 0;
     DistArgs a = dist_args(ctx, idx, pts, q, &smem);
-    a.n_list = q.n_valid.p;
+    a.n_valid = q.n_valid.p;
     a.dist_pt = d_point_distance;
     a.dist_geom = d_geom_distance;
     a.dist_scalar = distance;
@@ -1749,22 +1755,23 @@ int vs_join_nearest(vs_context* ctx, const vs_index* idx, const vs_points* pts, 
     VS_TRY(best.alloc((size_t)pts->n, s));
     size_t smem = 0;
     DistArgs a = dist_args(ctx, idx, pts, q, &smem);
-    a.n_list = q.n_valid.p;
+    a.n_valid = q.n_valid.p;
     a.best = best.p;
     a.radius = max_distance;  // the search cap
     a.sink = PairSink{d_left, d_right, (unsigned long long)(capacity > 0 ? capacity : 0), &ctx->d_counters[0]};
-    // one walk answers nearly every point; the rest (over_list) get each point's minimum distance, then every
-    // polygon at exactly that distance
-    Scratch<uint32_t> over, n_over;
-    VS_TRY(over.alloc((size_t)pts->n, s));
+    // one walk answers nearly every point; the rest (over) get each point's minimum distance, then every polygon at
+    // exactly that distance
+    Scratch<uint2> over;
+    Scratch<uint32_t> n_over;
+    VS_TRY(over.alloc((size_t)(pts->n / kDistGrab + 1), s));
     VS_TRY(n_over.alloc(1, s));
     VS_CUDA_TRY(cudaMemsetAsync(n_over.p, 0, sizeof(uint32_t), s));
     const NearArgs near{a, {over.p, n_over.p}};
     VS_CUDA_TRY(cudaFuncSetAttribute(near_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     near_kernel<<<resident_grid(near_kernel, pts->n, kDistThreads, smem), kDistThreads, smem, s>>>(near);
     VS_LAUNCHED("near", s);
-    a.list = over.p;
-    a.n_list = n_over.p;
+    a.packets = over.p;
+    a.n_packets = n_over.p;
     VS_TRY(launch_dist<kNearestMin>(ctx, a, smem, pts->n));
     VS_TRY(launch_dist<kNearestEmit>(ctx, a, smem, pts->n));
     const int st = finish_join(ctx, idx, pts, flags, d_left, d_right, capacity, n_pairs, stats, ev, launches0);
@@ -1880,16 +1887,17 @@ int vs_join_nearest_polygons(vs_context* ctx, const vs_index* point_index, const
     const size_t smem = (size_t)a.staged * sizeof(vs_box);
     // one walk answers nearly every polygon; the rest (over) get each polygon's minimum distance, then every point
     // at exactly that distance
-    Scratch<uint32_t> over, n_over;
-    VS_TRY(over.alloc((size_t)nq, s));
+    Scratch<uint2> over;
+    Scratch<uint32_t> n_over;
+    VS_TRY(over.alloc((size_t)(nq / kDistGrab + 1), s));
     VS_TRY(n_over.alloc(1, s));
     VS_CUDA_TRY(cudaMemsetAsync(n_over.p, 0, sizeof(uint32_t), s));
     const PolyNearArgs near{a, {over.p, n_over.p}};
     VS_CUDA_TRY(cudaFuncSetAttribute(poly_near_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     poly_near_kernel<<<resident_grid(poly_near_kernel, nq, kDistThreads, smem), kDistThreads, smem, s>>>(near);
     VS_LAUNCHED("poly_near", s);
-    a.order = over.p;
-    a.n_valid = n_over.p;
+    a.packets = over.p;
+    a.n_packets = n_over.p;
     VS_CUDA_TRY(cudaMemsetAsync(a.work, 0, sizeof(unsigned long long), s));
     VS_CUDA_TRY(cudaFuncSetAttribute(poly_nearest_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)smem));
