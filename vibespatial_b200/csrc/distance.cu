@@ -1490,20 +1490,6 @@ __global__ void __launch_bounds__(kDistThreads, 3) poly_near_kernel(const PolyNe
     unsigned n_exact = 0;
     // evaluate up to 32 queued pairs, one a lane
     auto drain = [&](int cnt) {
-        // drop what the bounds have passed from the lists, so that they have room
-        {
-            int keep = 0;
-            const float ub = __uint_as_float(pp.ub[lane]);
-            for (int k = 0; k < pp.cnt[lane]; ++k)
-                if (near.lo[k][lane] <= ub) {
-                    near.slot[keep][lane] = near.slot[k][lane];
-                    near.lo[keep][lane] = near.lo[k][lane];
-                    near.err[keep][lane] = near.err[k][lane];
-                    ++keep;
-                }
-            pp.cnt[lane] = keep;
-        }
-        __syncwarp();
         bool use = lane < cnt, at0 = false;
         int src = 0, slot = 0, row = 0;
         double px = 0.0, py = 0.0;
@@ -1533,6 +1519,20 @@ __global__ void __launch_bounds__(kDistThreads, 3) poly_near_kernel(const PolyNe
         }
         __syncwarp();
         if (use && at0) pp.ub[src] = 0u;  // whatever order the bounds arrived in
+        __syncwarp();
+        // drop what the bounds have passed from the lists (these pairs lowered them), so that they have room
+        {
+            int keep = 0;
+            const float ub = __uint_as_float(pp.ub[lane]);
+            for (int k = 0; k < pp.cnt[lane]; ++k)
+                if (near.lo[k][lane] <= ub) {
+                    near.slot[keep][lane] = near.slot[k][lane];
+                    near.lo[keep][lane] = near.lo[k][lane];
+                    near.err[keep][lane] = near.err[k][lane];
+                    ++keep;
+                }
+            pp.cnt[lane] = keep;
+        }
         __syncwarp();
         // the list of the pair's polygon; without room (or bounds) the polygon is left to the two walks, unless pairs
         // of it have been emitted: its distance is then 0 and the pair is decided here
