@@ -109,3 +109,50 @@ def test_time_grows_with_the_copies(ctx, vsabi, side, k):
     assert pairs == k * pairs_one
     print(side, k, one, many, many / one)
     assert many < 5 * k * one, (one, many)
+
+
+def _crowd(seed):
+    """3000 stars, about 20 over any place and some of them twice; points anywhere, on vertices, beside edges (an ulp
+    off, where a distance may round to 0) and outside them all."""
+    rng = np.random.default_rng(seed)
+    p = syn.star_polygons(rng, 3_000, 0.0, 250.0)
+    k = rng.choice(3_000, 400, replace=False)
+    xs, ys, sizes = [p.x], [p.y], [np.diff(p.ring_off)]
+    for g in k:
+        xs.append(p.x[p.ring_off[g]:p.ring_off[g + 1]])
+        ys.append(p.y[p.ring_off[g]:p.ring_off[g + 1]])
+        sizes.append([p.ring_off[g + 1] - p.ring_off[g]])
+    polys = syn._rings_to_soa(np.concatenate(sizes), np.concatenate(xs), np.concatenate(ys))
+    v = rng.integers(0, len(p.x) - 1, 600)
+    mid_x, mid_y = 0.5 * (p.x[v] + p.x[v + 1]), 0.5 * (p.y[v] + p.y[v + 1])
+    px = np.concatenate([rng.uniform(-40, 290, 1500), p.x[v], np.nextafter(p.x[v], 1e9), mid_x, np.nextafter(mid_x, 0)])
+    py = np.concatenate([rng.uniform(-40, 290, 1500), p.y[v], p.y[v], mid_y, mid_y])
+    return syn.Workload(name="crowd", px=px, py=py, polys=polys)
+
+
+@pytest.mark.parametrize("max_distance", [np.inf, 0.0, 0.5])
+def test_points_under_many_polygons(ctx, vsabi, oracle, max_distance):
+    w = _crowd(11)
+    index, pts, keep = _device(vsabi, ctx, w)
+    el, er, ed = oracle.nearest_join(w.px, w.py, None, _oracle_polys(oracle, w), max_distance)
+    gl, gr, gd, _ = index.nearest(pts, max_distance=max_distance)
+    np.testing.assert_array_equal(gl.cpu().numpy(), el)
+    np.testing.assert_array_equal(gr.cpu().numpy(), er)
+    np.testing.assert_array_equal(gd.cpu().numpy().view(np.int64), ed.view(np.int64))
+
+
+@pytest.mark.parametrize("max_distance", [np.inf, 0.0, 0.5])
+def test_polygons_over_many_points(ctx, vsabi, oracle, max_distance):
+    import torch
+
+    w = _crowd(12)
+    px, py = np.concatenate([w.px, w.px[::3]]), np.concatenate([w.py, w.py[::3]])
+    dx, dy = torch.from_numpy(px).cuda(), torch.from_numpy(py).cuda()
+    pidx = vsabi.point_index(ctx, dx, dy)
+    t = [torch.from_numpy(np.ascontiguousarray(getattr(w.polys, a))).cuda()
+         for a in ("x", "y", "ring_off", "part_off", "geom_off")]
+    el, er, ed = oracle.nearest_polygons_join(px, py, None, _oracle_polys(oracle, w), max_distance)
+    gl, gr, gd, _ = vsabi.nearest_polygons(ctx, pidx, vsabi.make_polygons(*t), max_distance=max_distance)
+    np.testing.assert_array_equal(gl.cpu().numpy(), el)
+    np.testing.assert_array_equal(gr.cpu().numpy(), er)
+    np.testing.assert_array_equal(gd.cpu().numpy().view(np.int64), ed.view(np.int64))

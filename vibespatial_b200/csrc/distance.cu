@@ -35,9 +35,10 @@
 // upper bound; the walk visits, nearest first, what lies within the queries'
 // current bounds (capped by max_distance), bounds every item's distance from
 // both sides in FP32 and lists the few items that may still be the nearest.
-// Exact distances are computed for the listed items only and decide.
-// Queries whose list overflows, or that FP32 cannot hold, take two exact
-// walks: the first finds the query's minimum (a polygon nearer than the
+// Exact distances are computed for the listed items only and decide.  Points
+// under many envelopes repeat the walk and locate each polygon as it is met.
+// Queries that end with more items within rounding of the nearest than the
+// list holds, or that FP32 cannot hold, take two exact walks: the first finds the query's minimum (a polygon nearer than the
 // minimum is always inside its box), the second emits every polygon at
 // exactly the minimum.  There, candidates whose envelope is certainly farther
 // than the bound are skipped before the exact distance.
@@ -287,16 +288,27 @@ __device__ __noinline__ double polygon_distance(const DistArgs& a, double x, dou
     return loc != LOC_OUTSIDE ? 0.0 : facet_distance(x, y, a.xy, a.ring_off, a.part_off, a.geom_off, g, -1.0);
 }
 
+// Is the point in polygon g (inside or on it)?
+__device__ __noinline__ bool point_in(const DistArgs& a, double x, double y, int g, unsigned& n_exact) {
+    const vs_box b = a.nodes[a.level_off[0] + g];
+    return x >= b.minx && x <= b.maxx && y >= b.miny && y <= b.maxy &&
+           geometry_location(x, y, a.xy, a.ring_off, a.part_off, a.geom_off, g, a.rings, n_exact) != LOC_OUTSIDE;
+}
+
 // The distance of a polygon on a nearest list, or something larger when it is
-// above ub: the location only where the point lies in the envelope, and in
-// FP64 only the segments within reach.  err < 0: no bounds are known.
+// above ub: the location only where the point lies in the envelope (kLocated:
+// it is known to be outside), and in FP64 only the segments within reach.
+// err < 0: no bounds are known.
+template <bool kLocated>
 __device__ __noinline__ double listed_distance(const DistArgs& a, double x, double y, int g, float err, float ub,
                                                unsigned& n_exact) {
     if (err < 0.f) return polygon_distance(a, x, y, g, n_exact);
-    const vs_box b = a.nodes[a.level_off[0] + g];
-    if (x >= b.minx && x <= b.maxx && y >= b.miny && y <= b.maxy &&
-        geometry_location(x, y, a.xy, a.ring_off, a.part_off, a.geom_off, g, a.rings, n_exact) != LOC_OUTSIDE)
-        return 0.0;
+    if (!kLocated) {
+        const vs_box b = a.nodes[a.level_off[0] + g];
+        if (x >= b.minx && x <= b.maxx && y >= b.miny && y <= b.maxy &&
+            geometry_location(x, y, a.xy, a.ring_off, a.part_off, a.geom_off, g, a.rings, n_exact) != LOC_OUTSIDE)
+            return 0.0;
+    }
     return facet_distance_bounded(x, y, a.xy, a.ring_off, a.part_off[a.geom_off[g]], a.part_off[a.geom_off[g + 1]],
                                   ub, err);
 }
@@ -806,17 +818,29 @@ struct NearList {
 
 struct NearArgs {
     DistArgs d;
-    OverPackets over;  // left to dist_join_kernel
+    OverPackets crowded;  // left to the pass that locates at once
+    OverPackets over;     // left to dist_join_kernel
 };
 
 // Nearest polygons of points, all ties, in one walk: a polygon a lane reaches
 // gets FP32 bounds [lo, hi] of its facet distance (facet_bounds); hi lowers
-// the lane's bound, and the polygon joins the lane's short list while lo is
-// within it.  At the end each list holds the polygons within rounding of the
-// nearest, one for nearly every point, and only those get the exact location
-// and FP64 distance.  Points whose list overflows (more than kNearList
-// polygons within rounding of the nearest) go to the two FP64 walks, which
-// compute an exact distance for every polygon met.
+// the lane's bound, and the polygon joins the lane's short list while lo, or 0
+// where the point lies in its envelope, is within it.  At the end each list
+// holds the polygons within rounding of the nearest, one for nearly every
+// point, and only those get the exact location and FP64 distance.
+//
+// Points in more than kNearList envelopes go to a second pass (kCrowded), which
+// locates a polygon exactly as soon as the point is found in its envelope:
+// inside, the distance is 0, the smallest there is, so the pair is emitted on
+// the spot and only other polygons at 0 remain of interest.  500k points on
+// 50k stars, 30 envelopes a point: 16.3 ms when such points went to the FP64
+// walks.  Locating at once in the first pass too, where a lane or two a warp
+// have something to locate, took disjoint footprints from 2.59 to 2.81 ms.
+//
+// Points that end with more than kNearList polygons within rounding of the
+// nearest go to the two FP64 walks, which compute an exact distance for every
+// polygon met.
+template <bool kCrowded>
 __global__ void __launch_bounds__(kDistThreads, 3) near_kernel(const NearArgs na) {
     const DistArgs& a = na.d;
     extern __shared__ vs_box s_nodes[];
@@ -830,19 +854,23 @@ __global__ void __launch_bounds__(kDistThreads, 3) near_kernel(const NearArgs na
     if (lane == 0) s_cnt[warp] = 0;
     __syncthreads();
     const WarpOut out{s_buf[warp], &s_cnt[warp]};
-    const int64_t n = (int64_t)*a.n_valid;
+    const int64_t n = kCrowded ? kDistGrab * (int64_t)*na.crowded.count : (int64_t)*a.n_valid;
     const float cap = __double2float_ru(a.radius);  // max_distance (INFINITY: unbounded)
     unsigned long long n_cand = 0;
     unsigned n_exact = 0;
     for (;;) {
-        const int64_t b0 = warp_grab(a.work, kDistGrab);
+        int64_t b0 = warp_grab(a.work, kDistGrab);
         if (b0 >= n) break;
-        const int64_t i = b0 + lane;
-        const bool active = i < n;
+        bool active = b0 + lane < n;
+        if (kCrowded) {
+            const uint2 packet = na.crowded.items[b0 / kDistGrab];
+            b0 = packet.x;
+            active = (packet.y >> lane) & 1u;
+        }
         double x = 0.0, y = 0.0;
         int32_t row = -1;
         if (active) {
-            row = (int32_t)a.order[i];
+            row = (int32_t)a.order[b0 + lane];
             x = a.px[row];
             y = a.py[row];
         }
@@ -852,28 +880,45 @@ __global__ void __launch_bounds__(kDistThreads, 3) near_kernel(const NearArgs na
         PacketLane pl;
         float radius;
         const bool fits = point_lane(finite, x, y, cx, cy, pl, radius);  // whole warp
-        bool over = active && !fits;
-        pl.ub = cap;
+        bool over = active && !fits;  // left to the exact walks (these, and lost below)
+        bool crowded = false;         // left to the second pass
+        bool zero = false;            // (second pass) a pair at distance 0 was emitted
+        float lost = INFINITY;        // least lower bound (above 0) of the polygons the list had no room for
+        pl.ub = kCrowded && active ? __double2float_ru(a.best[row]) : cap;
         NearList list{s_near[warp], 0};
-        // bounds of one polygon
-        auto visit = [&](int slot) {
+        // one polygon: its bounds, or true when it is at distance 0 and the pair is to be emitted; within: the point
+        // may lie in its envelope
+        auto visit = [&](int slot, bool within) {
             ++n_cand;
+            if (kCrowded && within && point_in(a, x, y, slot, n_exact)) {
+                pl.ub = 0.f;
+                zero = !over;
+                return zero;
+            }
             const FacetBounds f = facet_bounds(x, y, a.xy, a.ring_off, a.part_off[a.geom_off[slot]],
                                                a.part_off[a.geom_off[slot + 1]]);
             pl.ub = fminf(pl.ub, f.hi);
             float lo = f.lo;
-            if (lo > 0.f) {
+            if (!kCrowded && lo > 0.f) {
                 // inside the envelope the point may be inside the polygon: distance 0
                 const vs_box b = a.nodes[a.level_off[0] + slot];
                 if (x >= b.minx && x <= b.maxx && y >= b.miny && y <= b.maxy) lo = 0.f;
             }
-            if (lo <= pl.ub && lo < INFINITY && !list.add(slot, lo, f.full ? -1.f : f.err, pl.ub)) {
-                over = true;
+            if (!(lo <= pl.ub && lo < INFINITY) || list.add(slot, lo, f.full ? -1.f : f.err, pl.ub)) return false;
+            if (lo > 0.f) {
+                lost = fminf(lost, lo);  // lost only if the bound stays above it
+            } else if (!kCrowded) {
+                crowded = true;
                 pl.walk = false;
+            } else {
+                if (zero) return polygon_distance(a, x, y, slot, n_exact) == 0.0;
+                over = true;
             }
+            return false;
         };
         int first = -1;  // the item a lane starts with: the nearest of the descent's block, ties to the nearer centre
         if (__any_sync(0xffffffffu, pl.walk)) {
+            bool at0 = false;
             const int slot0 = packet_descend(a, s_nodes, s_walk[warp], cx, cy);
             if (slot0 >= 0 && pl.walk) {
                 float bd = INFINITY;
@@ -887,41 +932,50 @@ __global__ void __launch_bounds__(kDistThreads, 3) near_kernel(const NearArgs na
                     }
                 }
                 if (first >= 0) {
-                    if (bd <= __fmul_ru(pl.ub, pl.ub)) visit(first);
+                    if (bd <= __fmul_ru(pl.ub, pl.ub))
+                        at0 = visit(first, box_low2(pl.q, s_walk[warp].items[first - slot0]) <= 0.f);
                     else first = -1;
                 }
             }
             __syncwarp();
+            if (kCrowded) wemit_sync(out, a.sink, at0, row, at0 ? a.item_geom[first] : 0);
         }
         packet_walk(a, s_nodes, s_walk[warp], pl, cx, cy, radius, [&](int slot0, unsigned mine) {
             while (__any_sync(0xffffffffu, mine != 0)) {
                 // the lane's next item within its bound
                 int item = -1;
+                bool at0 = false, within = false;
                 while (mine && item < 0) {
                     const int j = __ffs(mine) - 1;
                     mine &= mine - 1;
-                    if (slot0 + j != first && box_low2(pl.q, s_walk[warp].items[j]) <= __fmul_ru(pl.ub, pl.ub)) item = j;
+                    const float low2 = box_low2(pl.q, s_walk[warp].items[j]);
+                    if (slot0 + j != first && low2 <= __fmul_ru(pl.ub, pl.ub)) {
+                        item = j;
+                        within = low2 <= 0.f;
+                    }
                 }
                 __syncwarp();
-                if (item >= 0) visit(slot0 + item);
-                if (over) mine = 0;
+                if (item >= 0) at0 = visit(slot0 + item, within);
                 __syncwarp();
+                if (kCrowded) wemit_sync(out, a.sink, at0, row, at0 ? a.item_geom[slot0 + item] : 0);
+                else if (crowded) mine = 0;
             }
         });
         __syncwarp();
+        over = over || (!crowded && lost < INFINITY && lost <= pl.ub);
         // the exact distances of what is left of the list
-        double best = INFINITY;
+        double best = zero ? 0.0 : INFINITY;
         unsigned left = 0, ties = 0;  // list entries
         for (int k = 0; k < list.cnt; ++k)
             if (s_near[warp].lo[k][lane] <= pl.ub) left |= 1u << k;
-        if (!pl.walk) left = 0;
+        if (over || crowded) left = 0;
         __syncwarp();
         while (__any_sync(0xffffffffu, left != 0)) {
             if (left) {
                 const int k = __ffs(left) - 1;
                 left &= left - 1;
-                const double d = listed_distance(a, x, y, s_near[warp].slot[k][lane], s_near[warp].err[k][lane],
-                                                 pl.ub, n_exact);
+                const double d = listed_distance<kCrowded>(a, x, y, s_near[warp].slot[k][lane],
+                                                           s_near[warp].err[k][lane], pl.ub, n_exact);
                 if (d < best) ties = 0;
                 best = d < best ? d : best;
                 if (d == best) ties |= 1u << k;
@@ -929,7 +983,7 @@ __global__ void __launch_bounds__(kDistThreads, 3) near_kernel(const NearArgs na
             __syncwarp();
         }
         if (!(best <= a.radius)) best = INFINITY;
-        if (active) a.best[row] = over ? fmin((double)pl.ub, a.radius) : best;
+        if (active) a.best[row] = over || crowded ? fmin((double)pl.ub, a.radius) : best;
         if (!(best < INFINITY)) ties = 0;
         while (__any_sync(0xffffffffu, ties != 0)) {
             const bool want = ties != 0;
@@ -937,6 +991,7 @@ __global__ void __launch_bounds__(kDistThreads, 3) near_kernel(const NearArgs na
             ties &= ties - 1;
             wemit_sync(out, a.sink, want, row, want ? a.item_geom[s_near[warp].slot[k][lane]] : 0);
         }
+        if (!kCrowded) na.crowded.add(crowded, b0);
         na.over.add(over, b0);
         wflush(out, a.sink, false);
     }
@@ -1049,16 +1104,28 @@ DistArgs dist_args(vs_context* ctx, const vs_index* idx, const vs_points* pts, c
     return a;
 }
 
+// A walk over up to n_items queries; `work`: its own counter of the context's, zero.
 template <int kMode>
-int launch_dist(vs_context* ctx, const DistArgs& a, size_t smem, int64_t n_items) {
+int launch_dist(vs_context* ctx, DistArgs a, size_t smem, int64_t n_items, int work) {
     cudaStream_t s = ctx->stream;
-    VS_CUDA_TRY(cudaMemsetAsync(&ctx->d_counters[kWorkCounter], 0, sizeof(unsigned long long), s));
+    a.work = &ctx->d_counters[work];
     auto* kernel = dist_join_kernel<kMode>;
     VS_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     kernel<<<resident_grid(kernel, n_items > 0 ? n_items : 1, kDistThreads, smem), kDistThreads, smem, s>>>(a);
     VS_LAUNCHED(kMode == kDwithin ? "dist_join<dwithin>" : kMode == kNearestMin ? "dist_join<nearest_min>"
                                                                                 : "dist_join<nearest_emit>",
                 s);
+    return VS_OK;
+}
+
+template <bool kCrowded>
+int launch_near(vs_context* ctx, NearArgs na, size_t smem, int64_t n_items, int work) {
+    cudaStream_t s = ctx->stream;
+    na.d.work = &ctx->d_counters[work];
+    auto* kernel = near_kernel<kCrowded>;
+    VS_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kernel<<<resident_grid(kernel, n_items, kDistThreads, smem), kDistThreads, smem, s>>>(na);
+    VS_LAUNCHED(kCrowded ? "near<crowded>" : "near", s);
     return VS_OK;
 }
 
@@ -1460,11 +1527,12 @@ struct PolyPacket {
     int32_t row[32];
     int r0[32], r1[32];
     unsigned ub[32];     // bound (non-negative float bits)
+    unsigned lost[32];   // least lower bound (above 0) of the points the list had no room for (float bits)
     int cnt[32];         // list entries
     int state[32];       // kPoly*
     int2 queue[64];      // (lane, slot)
 };
-enum : int { kPolyOver = 1, kPolyZero = 2 };  // left to the two walks; a pair at distance 0 was emitted
+enum : int { kPolyOver = 1, kPolyZero = 2 };  // left to the two walks; a pair at distance 0 was emitted (never both)
 
 __global__ void __launch_bounds__(kDistThreads, 3) poly_near_kernel(const PolyNearArgs na) {
     const PolyArgs& a = na.d;
@@ -1490,7 +1558,8 @@ __global__ void __launch_bounds__(kDistThreads, 3) poly_near_kernel(const PolyNe
     unsigned n_exact = 0;
     // evaluate up to 32 queued pairs, one a lane
     auto drain = [&](int cnt) {
-        bool use = lane < cnt, at0 = false;
+        const bool use = lane < cnt;
+        bool at0 = false, done = false;  // to be emitted; the point is in the polygon
         int src = 0, slot = 0, row = 0;
         double px = 0.0, py = 0.0;
         FacetBounds f{INFINITY, INFINITY, 0.f, false};
@@ -1499,9 +1568,6 @@ __global__ void __launch_bounds__(kDistThreads, 3) poly_near_kernel(const PolyNe
             src = e.x;
             slot = e.y;
             row = pp.row[src];
-            use = !(pp.state[src] & kPolyOver);
-        }
-        if (use) {
             ++n_cand;
             const vs_box pb = a.nodes[a.level_off[0] + slot];  // a leaf box is its point
             px = pb.minx;
@@ -1510,15 +1576,17 @@ __global__ void __launch_bounds__(kDistThreads, 3) poly_near_kernel(const PolyNe
             if (px >= qb.minx && px <= qb.maxx && py >= qb.miny && py <= qb.maxy)
                 at0 = located_in(a, px, py, row, n_exact);
             if (at0) {
-                atomicOr(&pp.state[src], kPolyZero);
+                at0 = !(pp.state[src] & kPolyOver);
+                if (at0) atomicOr(&pp.state[src], kPolyZero);
                 pp.ub[src] = 0u;
+                done = true;
             } else {
                 f = facet_bounds(px, py, xy, a.ring_off, pp.r0[src], pp.r1[src]);
                 if (!f.full) atomicMin(&pp.ub[src], __float_as_uint(f.hi));
             }
         }
         __syncwarp();
-        if (use && at0) pp.ub[src] = 0u;  // whatever order the bounds arrived in
+        if (done) pp.ub[src] = 0u;  // whatever order the bounds arrived in
         __syncwarp();
         // drop what the bounds have passed from the lists (these pairs lowered them), so that they have room
         {
@@ -1534,10 +1602,11 @@ __global__ void __launch_bounds__(kDistThreads, 3) poly_near_kernel(const PolyNe
             pp.cnt[lane] = keep;
         }
         __syncwarp();
-        // the list of the pair's polygon; without room (or bounds) the polygon is left to the two walks, unless pairs
-        // of it have been emitted: its distance is then 0 and the pair is decided here
+        // the list of the pair's polygon; without room (or bounds) the polygon is left to the two walks if the pair
+        // stays within its bound, unless pairs of it have been emitted: its distance is then 0 and the pair is decided
+        // here
         bool failed = false;
-        if (use && !at0 && f.lo < INFINITY && f.lo <= __uint_as_float(pp.ub[src])) {
+        if (use && !done && f.lo < INFINITY && f.lo <= __uint_as_float(pp.ub[src])) {
             const int k = f.full ? kNearList : atomicAdd(&pp.cnt[src], 1);
             if (k < kNearList) {
                 near.slot[k][src] = slot;
@@ -1551,6 +1620,7 @@ __global__ void __launch_bounds__(kDistThreads, 3) poly_near_kernel(const PolyNe
         pp.cnt[lane] = pp.cnt[lane] < kNearList ? pp.cnt[lane] : kNearList;
         if (failed) {
             if (pp.state[src] & kPolyZero) at0 = point_polygon_soa(a, px, py, row, n_exact) == 0.0;
+            else if (f.lo > 0.f) atomicMin(&pp.lost[src], __float_as_uint(f.lo));
             else atomicOr(&pp.state[src], kPolyOver);
         }
         __syncwarp();
@@ -1581,6 +1651,7 @@ __global__ void __launch_bounds__(kDistThreads, 3) poly_near_kernel(const PolyNe
         const float radius = warp_max_nonneg(pl.walk ? __fmul_ru(far, 1.42f) : 0.f);
         pp.row[lane] = row;
         pp.ub[lane] = __float_as_uint(cap);
+        pp.lost[lane] = __float_as_uint(INFINITY);
         pp.cnt[lane] = 0;
         pp.state[lane] = active && !pl.walk ? kPolyOver : 0;
         int nq = 0;      // warp-uniform queue length
@@ -1599,10 +1670,7 @@ __global__ void __launch_bounds__(kDistThreads, 3) poly_near_kernel(const PolyNe
                 __syncwarp();
             }
         };
-        auto take_bounds = [&]() {
-            pl.ub = __uint_as_float(pp.ub[lane]);
-            if (pp.state[lane] & kPolyOver) pl.walk = false;
-        };
+        auto take_bounds = [&]() { pl.ub = __uint_as_float(pp.ub[lane]); };
         if (__any_sync(0xffffffffu, pl.walk)) {
             // each lane starts with the point of the descent's block nearest to its envelope's centre
             const int slot0 = packet_descend(a, s_nodes, s_walk[warp], cx, cy);
@@ -1636,20 +1704,20 @@ __global__ void __launch_bounds__(kDistThreads, 3) poly_near_kernel(const PolyNe
                 __syncwarp();
                 push(item >= 0, slot0 + item);
                 take_bounds();
-                if (!pl.walk) mine = 0;
             }
         });
         __syncwarp();
         if (nq > 0) drain(nq);
         __syncwarp();
         take_bounds();
-        const bool over = (pp.state[lane] & kPolyOver) != 0;
+        const float lost = __uint_as_float(pp.lost[lane]);
+        const bool over = (pp.state[lane] & kPolyOver) != 0 || (lost < INFINITY && lost <= pl.ub);
         // the exact distances of what is left of the lists
         double best = (pp.state[lane] & kPolyZero) ? 0.0 : INFINITY;
         unsigned left = 0, ties = 0;
         for (int k = 0; k < pp.cnt[lane]; ++k)
             if (near.lo[k][lane] <= pl.ub) left |= 1u << k;
-        if (!pl.walk) left = 0;
+        if (over) left = 0;
         __syncwarp();
         while (__any_sync(0xffffffffu, left != 0)) {
             if (left) {
@@ -1728,7 +1796,7 @@ int vs_join_dwithin(vs_context* ctx, const vs_index* idx, const vs_points* pts, 
     a.dist_geom = d_geom_distance;
     a.dist_scalar = distance;
     a.sink = PairSink{d_left, d_right, (unsigned long long)(capacity > 0 ? capacity : 0), &ctx->d_counters[0]};
-    VS_TRY(launch_dist<kDwithin>(ctx, a, smem, pts->n));
+    VS_TRY(launch_dist<kDwithin>(ctx, a, smem, pts->n, kWorkCounter));
     return finish_join(ctx, idx, pts, flags, d_left, d_right, capacity, n_pairs, stats, ev, launches0);
 }
 
@@ -1759,21 +1827,21 @@ int vs_join_nearest(vs_context* ctx, const vs_index* idx, const vs_points* pts, 
     a.best = best.p;
     a.radius = max_distance;  // the search cap
     a.sink = PairSink{d_left, d_right, (unsigned long long)(capacity > 0 ? capacity : 0), &ctx->d_counters[0]};
-    // one walk answers nearly every point; the rest (over) get each point's minimum distance, then every polygon at
-    // exactly that distance
-    Scratch<uint2> over;
+    // one walk answers nearly every point, a second those under many polygons; the rest (over) get each point's
+    // minimum distance, then every polygon at exactly that distance
+    const size_t packets = (size_t)(pts->n / kDistGrab + 1);
+    Scratch<uint2> over;  // [0, packets) crowded, then over (both passes leave some: up to twice the packets)
     Scratch<uint32_t> n_over;
-    VS_TRY(over.alloc((size_t)(pts->n / kDistGrab + 1), s));
-    VS_TRY(n_over.alloc(1, s));
-    VS_CUDA_TRY(cudaMemsetAsync(n_over.p, 0, sizeof(uint32_t), s));
-    const NearArgs near{a, {over.p, n_over.p}};
-    VS_CUDA_TRY(cudaFuncSetAttribute(near_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    near_kernel<<<resident_grid(near_kernel, pts->n, kDistThreads, smem), kDistThreads, smem, s>>>(near);
-    VS_LAUNCHED("near", s);
-    a.packets = over.p;
-    a.n_packets = n_over.p;
-    VS_TRY(launch_dist<kNearestMin>(ctx, a, smem, pts->n));
-    VS_TRY(launch_dist<kNearestEmit>(ctx, a, smem, pts->n));
+    VS_TRY(over.alloc(3 * packets, s));
+    VS_TRY(n_over.alloc(2, s));
+    VS_CUDA_TRY(cudaMemsetAsync(n_over.p, 0, 2 * sizeof(uint32_t), s));
+    const NearArgs near{a, {over.p, n_over.p}, {over.p + packets, n_over.p + 1}};
+    VS_TRY(launch_near<false>(ctx, near, smem, pts->n, kWorkCounter));
+    VS_TRY(launch_near<true>(ctx, near, smem, pts->n, kWorkCounter + 2));
+    a.packets = near.over.items;
+    a.n_packets = near.over.count;
+    VS_TRY(launch_dist<kNearestMin>(ctx, a, smem, pts->n, kWorkCounter + 3));
+    VS_TRY(launch_dist<kNearestEmit>(ctx, a, smem, pts->n, kWorkCounter + 4));
     const int st = finish_join(ctx, idx, pts, flags, d_left, d_right, capacity, n_pairs, stats, ev, launches0);
     if (st != VS_OK) return st;
     if (d_distance && *n_pairs > 0) {
