@@ -62,3 +62,27 @@ def test_join_order(vsabi, ctx, oracle):
     order = np.lexsort((ur, ul))
     assert np.array_equal(left.cpu().numpy(), ul[order])
     assert np.array_equal(right.cpu().numpy(), ur[order])
+
+
+@pytest.mark.parametrize("n", [8_193, 100_003, 400_001])
+@pytest.mark.parametrize("run", [3, 31, 32, 33, 63, 64, 65, 100, 129, 700, 1023, 1024, 1025, 3000])
+@pytest.mark.parametrize("share", [1.0, 0.5])
+def test_runs_of_equal_left_rows(vsabi, ctx, n, run, share):
+    """Runs of equal left rows, ordered by their right rows (some equal) where left rows have few pairs on average: as
+    long as a warp, two, what a tile holds of its neighbours, and up to the limit and beyond; every pair in one, or
+    half of them alone in theirs, so that runs of both kinds share warps and cross tiles."""
+    import torch
+
+    rng = np.random.default_rng(n + run)
+    in_runs = int(n * share) // run * run
+    left = np.concatenate([np.repeat(rng.choice(2**22, in_runs // run, replace=False), run),
+                           rng.integers(0, 2**22, n - in_runs)]).astype(np.int32)
+    right = rng.integers(0, 500, n).astype(np.int32)
+    left[-1] = 2**22  # (few pairs a left row)
+    mix = rng.permutation(n)
+    left, right = left[mix], right[mix]
+    dl, dr = torch.from_numpy(left).cuda(), torch.from_numpy(right).cuda()
+    vsabi.sort_pairs(ctx, dl, dr)
+    order = np.lexsort((right, left))
+    assert np.array_equal(dl.cpu().numpy(), left[order])
+    assert np.array_equal(dr.cpu().numpy(), right[order])

@@ -422,7 +422,7 @@ int vs_join(vs_context* ctx, const vs_index* idx, const vs_points* pts, int32_t 
         return VS_E_CAPACITY;
     }
     if (sort) {
-        VS_TRY(finish_sort_pairs(ctx, d_left, d_right, n, (uint64_t)pts->n, (uint64_t)idx->n_geoms));
+        VS_TRY(finish_sort_pairs(ctx, d_left, d_right, n, (uint64_t)pts->n, (uint64_t)idx->n_geoms, es.b));
         if (stats) {
             stats->sort_ms = es.ms();
             stats->kernel_launches = g_launches - launches0;

@@ -38,10 +38,11 @@
 // Exact distances are computed for the listed items only and decide.  Points
 // under many envelopes repeat the walk and locate each polygon as it is met.
 // Queries that end with more items within rounding of the nearest than the
-// list holds, or that FP32 cannot hold, take two exact walks: the first finds the query's minimum (a polygon nearer than the
-// minimum is always inside its box), the second emits every polygon at
-// exactly the minimum.  There, candidates whose envelope is certainly farther
-// than the bound are skipped before the exact distance.
+// list holds, or that FP32 cannot hold, take two exact walks: the first finds
+// the query's minimum (a polygon nearer than the minimum is always inside its
+// box), the second emits every polygon at exactly the minimum.  There,
+// candidates whose envelope is certainly farther than the bound are skipped
+// before the exact distance.
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>

@@ -524,11 +524,12 @@ int enqueue_sort_pairs(vs_context* ctx, int32_t* d_left, int32_t* d_right, int64
 }
 
 int finish_sort_pairs(vs_context* ctx, int32_t* d_left, int32_t* d_right, int64_t n, uint64_t max_left,
-                      uint64_t max_right) {
+                      uint64_t max_right, cudaEvent_t sorted) {
     VS_TRY(finish_status(ctx));
     if (!(ctx->h_counter[kHostCounters - 1] & 4)) return VS_OK;
     // a left row with very many pairs
     VS_TRY(enqueue_sort_pairs(ctx, d_left, d_right, n, max_left, max_right, false));
+    if (sorted) cudaEventRecord(sorted, ctx->stream);
     return finish_status(ctx);
 }
 

@@ -58,9 +58,10 @@ int sort_pairs(vs_context* ctx, int32_t* d_left, int32_t* d_right, int64_t n, ui
 // d_counters[kStatus], which clear_status zeroes).
 int enqueue_sort_pairs(vs_context* ctx, int32_t* d_left, int32_t* d_right, int64_t n, uint64_t max_left,
                        uint64_t max_right, bool by_runs);
-// Wait for an enqueued sort (by_runs), and sort by every digit what it left.
+// Wait for an enqueued sort (by_runs), and sort by every digit what it left
+// (`sorted`, an event behind the first sort, is then recorded again).
 int finish_sort_pairs(vs_context* ctx, int32_t* d_left, int32_t* d_right, int64_t n, uint64_t max_left,
-                      uint64_t max_right);
+                      uint64_t max_right, cudaEvent_t sorted = nullptr);
 // Zero the status word; wait for the stream and read it (to the last word of
 // h_counter; VS_E_TIMEOUT for a wait that gave up).
 int clear_status(vs_context* ctx);

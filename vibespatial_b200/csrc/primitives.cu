@@ -148,7 +148,7 @@ enum : int { kPairsFull = 0, kPairsRuns = 1, kPairsAuto = 2 };
 // 8 it reads a handful of neighbours, and saves the passes over right's digits
 // (half of them for 20-bit rows).
 constexpr int64_t kRunMean = 8;
-constexpr int kRunMax = 1024;  // longest run the run pass orders (each item compares itself with its run)
+constexpr int kRunMax = 1024;  // pairs of a run behind the tile it begins in that the run pass still orders
 
 // One sort.  The items are (key, value) arrays, or (left, right) pairs whose
 // key is left << rbits | right and which carry no value.  Arrays: slot 0 reads
@@ -474,62 +474,207 @@ __global__ void __launch_bounds__(kPassThreads) rs_pass_kernel(const SortArgs<K>
     }
 }
 
-// The pairs, sorted by left, back to the caller's arrays; in a run of equal
-// left rows each pair goes to the place its right row gives it (the number of
-// smaller ones in the run, equal ones in their order).  A run longer than
-// kRunMax is left as it is and reported (bit 2 of *too_long): such pairs are sorted
-// by right's digits instead.
-constexpr int kRunThreads = 256, kRunItems = 8, kRunTile = kRunThreads * kRunItems, kRunHalo = 64;
+// The pairs, sorted by left, back to the caller's arrays, each run of equal
+// left rows in the order of its right rows.  A run belongs to the block whose
+// tile it begins in, which holds it to its end, up to kRunMax pairs beyond the
+// tile; a run that goes on longer is left as it is and reported (bit 2 of
+// *too_long): such pairs are sorted by right's digits instead.
+//
+// Short runs: each pair counts the smaller ones of its run (equal ones in their
+// order).  A tile with a run longer than kRunLong, or with many longer than
+// kRunShort, sorts its pairs by run and right row in shared memory: the count
+// is quadratic in the run, the sort is not.  Whole sorts of 12M pairs (14M for
+// runs of 1000), us, with every tile counting / as it is: runs of 32 pairs
+// 664 / 658, 40 736 / 565, 64 933 / 629, 100 1121 / 568, 400 2711 / 572, 1000
+// 6914 / 686; with runs of 2000, and so a second sort, 10554 / 1241.  (Passes
+// over all digits, each with a histogram and a scan of its own, took 990 to
+// 1130.)
+constexpr int kRunThreads = 256, kRunItems = 8, kRunTile = kRunThreads * kRunItems, kRunWarps = kRunThreads / 32;
+constexpr int kRunHeld = kRunTile + kRunMax;
+constexpr int kRunRounds = kRunHeld / kRunThreads;
+constexpr int kRunShort = 24;
+constexpr int kRunLong = 192;
+static_assert(kRunHeld % kRunThreads == 0 && kRunHeld <= 0xffff, "a run's number fits 16 bits");
+static_assert(kRunLong + 16 <= kRunThreads, "the count looks at a tile and as many pairs behind it as it has threads");
 
-__global__ void __launch_bounds__(kRunThreads) rs_runs_kernel(const SortArgs<uint64_t> a) {
-    // a tile with kRunHalo neighbours on both sides
-    constexpr int kHeld = kRunTile + 2 * kRunHalo;
-    __shared__ uint32_t s_left[kHeld], s_right[kHeld];
-    const uint64_t* __restrict__ key = a.kbuf[(a.plan->n_slots - 1) & 1];
-    const uint64_t rmask = (1ull << a.rbits) - 1ull;
-    const bool full = a.plan->full != 0;
-    const int64_t tile0 = (int64_t)blockIdx.x * kRunTile;
-    const int64_t held0 = tile0 - kRunHalo;  // the pair s_left[0] holds
-    for (int j = threadIdx.x; j < kHeld; j += kRunThreads) {
-        const int64_t i = held0 + j;
-        if (i < 0 || i >= a.n) continue;
-        const uint64_t k = key[i];
-        s_left[j] = (uint32_t)(k >> a.rbits);
-        s_right[j] = (uint32_t)(k & rmask);
+struct RunShared {
+    uint32_t left[kRunHeld], right[kRunHeld];
+    uint16_t run[kRunHeld];
+    uint32_t cnt[kRunWarps][256];
+    uint32_t sum[kRunWarps];
+    int first, last, behind;
+    bool goes_on, long_before;  // the tile's first run begins before it; before the tile before it
+};
+
+// Sort the m pairs held from h0 on by (run, right): right rows only, a place's
+// left row stays what it is.  Whole block.
+__device__ __noinline__ void sort_held_runs(RunShared& sm, int h0, int m, int rbits) {
+    constexpr unsigned kAll = 0xffffffffu;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int at = warp * 32 * kRunRounds + lane;
+    uint32_t right[kRunRounds], run[kRunRounds], rank[kRunRounds];
+    // the number of a pair's run among those held
+    uint32_t heads = 0;
+#pragma unroll
+    for (int r = 0; r < kRunRounds; ++r) {
+        const int q = at + 32 * r;
+        const unsigned b = __ballot_sync(kAll, q > 0 && q < m && sm.left[h0 + q] != sm.left[h0 + q - 1]);
+        run[r] = heads + __popc(b & (kAll >> (31 - lane)));
+        heads += __popc(b);  // warp-uniform
+        right[r] = q < m ? sm.right[h0 + q] : kAll;  // (past the end: behind every pair)
+    }
+    if (lane == 0) sm.sum[warp] = heads;
+    __syncthreads();
+    uint32_t base = 0, runs = 0;
+    for (int w = 0; w < kRunWarps; ++w) {
+        base += w < warp ? sm.sum[w] : 0u;
+        runs += sm.sum[w];
+    }
+#pragma unroll
+    for (int r = 0; r < kRunRounds; ++r) run[r] = at + 32 * r < m ? base + run[r] : 0xffffu;
+    const int run_passes = runs == 0 ? 0 : runs < 0xffu ? 1 : 2;
+    for (int pass = -((rbits + 7) / 8); pass < run_passes; ++pass) {
+        const bool by_run = pass >= 0;
+        const int shift = by_run ? 8 * pass : 8 * (pass + (rbits + 7) / 8);
+        __syncthreads();
+        for (int i = tid; i < kRunWarps * 256; i += kRunThreads) (&sm.cnt[0][0])[i] = 0;
+        __syncthreads();
+        if (by_run) warp_rank<uint32_t, 8, kRunRounds>(run, shift, sm.cnt[warp], rank);
+        else warp_rank<uint32_t, 8, kRunRounds>(right, shift, sm.cnt[warp], rank);
+        __syncthreads();
+        uint32_t total = 0;  // of digit tid
+        for (int w = 0; w < kRunWarps; ++w) {
+            const uint32_t c = sm.cnt[w][tid];
+            sm.cnt[w][tid] = total;
+            total += c;
+        }
+        const uint32_t inc = warp_inclusive_scan(total);
+        if (lane == 31) sm.sum[warp] = inc;
+        __syncthreads();
+        uint32_t start = inc - total;
+        for (int w = 0; w < warp; ++w) start += sm.sum[w];
+        for (int w = 0; w < kRunWarps; ++w) sm.cnt[w][tid] += start;
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < kRunRounds; ++r) {
+            const unsigned d = ((by_run ? run[r] : right[r]) >> shift) & 255u;
+            const uint32_t pos = sm.cnt[warp][d] + rank[r];
+            if (pos < (uint32_t)m) {  // (those past the end come last)
+                sm.right[h0 + pos] = right[r];
+                sm.run[pos] = (uint16_t)run[r];
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < kRunRounds; ++r) {
+            const int q = at + 32 * r;
+            right[r] = q < m ? sm.right[h0 + q] : kAll;
+            run[r] = q < m ? (uint32_t)sm.run[q] : 0xffffu;
+        }
     }
     __syncthreads();
-    const int j_lo = held0 < 0 ? (int)-held0 : 0;
-    const int j_hi = a.n - held0 < kHeld ? (int)(a.n - held0) : kHeld;
-    bool too_long = false;
+}
+
+__global__ void __launch_bounds__(kRunThreads, 5) rs_runs_kernel(const SortArgs<uint64_t> a) {
+    __shared__ RunShared sm;
+    const uint64_t* __restrict__ key = a.kbuf[(a.plan->n_slots - 1) & 1];
+    const uint64_t rmask = (1ull << a.rbits) - 1ull;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int64_t tile0 = (int64_t)blockIdx.x * kRunTile;
+    const int count = (int)(a.n - tile0 < kRunTile ? a.n - tile0 : kRunTile);
+    if (a.plan->full != 0) {  // sorted by right too
+        for (int j = tid; j < count; j += kRunThreads) {
+            const uint64_t k = key[tile0 + j];
+            a.left[tile0 + j] = (int32_t)(k >> a.rbits);
+            a.right[tile0 + j] = (int32_t)(k & rmask);
+        }
+        return;
+    }
+    for (int j = tid; j < count; j += kRunThreads) {
+        const uint64_t k = key[tile0 + j];
+        sm.left[j] = (uint32_t)(k >> a.rbits);
+        sm.right[j] = (uint32_t)(k & rmask);
+    }
+    if (tid == 0) {
+        const uint32_t l0 = (uint32_t)(key[tile0] >> a.rbits);
+        sm.goes_on = tile0 > 0 && (uint32_t)(key[tile0 - 1] >> a.rbits) == l0;
+        sm.long_before = tile0 > kRunTile && (uint32_t)(key[tile0 - kRunTile - 1] >> a.rbits) == l0;
+        sm.first = count;
+        sm.last = -1;
+    }
+    if (warp == 1) {  // pairs of the tile's last run behind it (more than kRunMax: any such number)
+        const int64_t end = tile0 + count;
+        const uint32_t l1 = (uint32_t)(key[end - 1] >> a.rbits);
+        int behind = 0;
+        for (unsigned m = 0xffffffffu; m == 0xffffffffu && behind <= kRunMax;) {
+            const int64_t i = end + behind + lane;
+            m = __ballot_sync(0xffffffffu, i < a.n && (uint32_t)(key[i] >> a.rbits) == l1);
+            behind += m == 0xffffffffu ? 32 : __ffs(~m) - 1;
+        }
+        if (lane == 0) sm.behind = behind;
+    }
+    __syncthreads();
+    // the first and the last run that begin in the tile
+    int first = count, last = -1;
 #pragma unroll
     for (int u = 0; u < kRunItems; ++u) {
-        const int j0 = u * kRunThreads + (int)threadIdx.x + kRunHalo;
-        if (j0 >= j_hi) break;
-        const uint32_t l = s_left[j0], r = s_right[j0];
-        int64_t pos = held0 + j0;
-        if (!full) {
-            int move = 0;  // larger ones before move behind, smaller ones behind move before
-            int j = j0 - 1;
-            for (; j >= j_lo && s_left[j] == l; --j) move -= s_right[j] > r ? 1 : 0;
-            int len = j0 - j;
-            if (j < j_lo) {  // the run leaves what is held: on in global memory
-                for (int64_t i = held0 + j; i >= 0 && len <= kRunMax && (uint32_t)(key[i] >> a.rbits) == l; --i, ++len)
-                    move -= (uint32_t)(key[i] & rmask) > r ? 1 : 0;
-            }
-            j = j0 + 1;
-            for (; j < j_hi && s_left[j] == l; ++j) move += s_right[j] < r ? 1 : 0;
-            len += j - j0 - 1;
-            if (j >= j_hi) {
-                for (int64_t i = held0 + j; i < a.n && len <= kRunMax && (uint32_t)(key[i] >> a.rbits) == l; ++i, ++len)
-                    move += (uint32_t)(key[i] & rmask) < r ? 1 : 0;
-            }
-            if (len > kRunMax) too_long = true;
-            else pos += move;
+        const int j = tid + u * kRunThreads;
+        if (j < count && (j > 0 ? sm.left[j] != sm.left[j - 1] : !sm.goes_on)) {
+            first = min(first, j);
+            last = j;
         }
-        a.left[pos] = (int32_t)l;
-        a.right[pos] = (int32_t)r;
     }
-    if (too_long && a.too_long) atomicOr(a.too_long, 4ull);
+    first = __reduce_min_sync(0xffffffffu, first);
+    last = __reduce_max_sync(0xffffffffu, last);
+    if (lane == 0) {
+        if (first < count) atomicMin(&sm.first, first);
+        if (last >= 0) atomicMax(&sm.last, last);
+    }
+    __syncthreads();
+    const int h0 = sm.first, hl = sm.last, behind = sm.behind;
+    const bool first_long = sm.goes_on && (h0 > kRunMax || sm.long_before);
+    const bool last_long = hl >= 0 && behind > kRunMax;
+    const int end = hl < 0 ? h0 : last_long ? hl : count + behind;  // the tile's own runs: [h0, end)
+    if (!last_long && hl >= 0)
+        for (int j = count + tid; j < end; j += kRunThreads) {
+            const uint64_t k = key[tile0 + j];
+            sm.left[j] = (uint32_t)(k >> a.rbits);
+            sm.right[j] = (uint32_t)(k & rmask);
+        }
+    if (first_long || last_long) {
+        for (int j = tid; j < count; j += kRunThreads)
+            if (j < h0 ? first_long : j >= end) {
+                a.left[tile0 + j] = (int32_t)sm.left[j];
+                a.right[tile0 + j] = (int32_t)sm.right[j];
+            }
+        if (tid == 0 && a.too_long) atomicOr(a.too_long, 4ull);
+    }
+    __syncthreads();
+    // by samples: a run longer than kRunLong, or a quarter of the pairs with more than kRunShort of their run behind them
+    const int j = h0 + 16 * tid;
+    const bool longer = j + kRunShort < end && sm.left[j] == sm.left[j + kRunShort];
+    const int samples = (end - h0 + 15) / 16;
+    const bool one = longer && j + kRunLong < end && sm.left[j] == sm.left[j + kRunLong];
+    const int many = __syncthreads_count(longer);
+    if (__syncthreads_or(one) || 4 * many > samples) {
+        sort_held_runs(sm, h0, end - h0, a.rbits);
+        for (int i = h0 + tid; i < end; i += kRunThreads) {
+            a.left[tile0 + i] = (int32_t)sm.left[i];
+            a.right[tile0 + i] = (int32_t)sm.right[i];
+        }
+        return;
+    }
+#pragma unroll
+    for (int u = 0; u < kRunItems + 1; ++u) {
+        const int j0 = tid + u * kRunThreads;  // (the last run has kRunLong + 16 pairs at most)
+        if (j0 < h0 || j0 >= end) continue;
+        const uint32_t l = sm.left[j0], r = sm.right[j0];
+        int move = 0;  // larger ones before move behind, smaller ones behind move before
+        for (int i = j0 - 1; i >= h0 && sm.left[i] == l; --i) move -= sm.right[i] > r ? 1 : 0;
+        for (int i = j0 + 1; i < end && sm.left[i] == l; ++i) move += sm.right[i] < r ? 1 : 0;
+        a.left[tile0 + j0 + move] = (int32_t)l;
+        a.right[tile0 + j0 + move] = (int32_t)r;
+    }
 }
 
 // A sort of at most kSmallSort items in one block: every pass in shared
