@@ -46,7 +46,7 @@ def test_keys_with_values_are_stable(vsabi, ctx, n, bits):
 
 
 def test_join_order(vsabi, ctx, oracle):
-    """A sorted join's pairs (left rows below 2^19, 9-bit digits) equal the sorted unsorted join's."""
+    """A sorted join's pairs (left rows below 2^19: 8-bit digits) equal the sorted unsorted join's."""
     import torch
 
     from vibespatial_b200.testing import synthetic as syn
@@ -86,3 +86,50 @@ def test_runs_of_equal_left_rows(vsabi, ctx, n, run, share):
     order = np.lexsort((right, left))
     assert np.array_equal(dl.cpu().numpy(), left[order])
     assert np.array_equal(dr.cpu().numpy(), right[order])
+
+
+def _squares(n_points, counts):
+    """A join of n_points points with one square for each count, which holds that many of them (the first ones of a
+    fixed order, so that the squares share points)."""
+    from vibespatial_b200.testing import synthetic as syn
+
+    rng = np.random.default_rng(n_points)
+    at = rng.permutation(n_points)
+    px = np.empty(n_points)
+    px[at] = np.arange(n_points) + 0.5
+    half = np.asarray(counts, np.float64)
+    xs = np.stack([0 * half, half, half, 0 * half, 0 * half], 1).ravel()
+    ys = np.tile([0.0, 0.0, 1.0, 1.0, 0.0], len(half))
+    return px, np.full(n_points, 0.5), syn._rings_to_soa(np.full(len(half), 5), xs, ys)
+
+
+def _joined(vsabi, ctx, px, py, p):
+    import torch
+
+    dx, dy = torch.from_numpy(px).cuda(), torch.from_numpy(py).cuda()
+    t = [torch.from_numpy(getattr(p, k)).cuda() for k in ("x", "y", "ring_off", "part_off", "geom_off")]
+    idx = vsabi.DeviceIndex(ctx, vsabi.make_polygons(*t))
+    pts = vsabi.make_points(dx, dy)
+    got = [v.cpu().numpy() for v in idx.join(pts, vsabi.PRED_WITHIN, vsabi.METHOD_RTREE, sort=True)[:2]]
+    left, right = (v.cpu().numpy() for v in idx.join(pts, vsabi.PRED_WITHIN, vsabi.METHOD_RTREE, sort=False)[:2])
+    order = np.lexsort((right, left))
+    assert np.array_equal(got[0], left[order])
+    assert np.array_equal(got[1], right[order])
+    return len(left)
+
+
+# left rows of 17, 18, 25 and 26 bits: 9-bit digits; of 24: 8-bit ones
+@pytest.mark.parametrize("n_points", [100_007, 262_143, 2**24 + 1, 2**25 + 5, 2**23 + 3])
+# the edges of the small sort, of tiles of 1024 and 4096 pairs, and where the latter begin
+@pytest.mark.parametrize("pairs", [8_192, 8_193, 9 * 1024, 9 * 1024 + 1, 303_104, 303_105, 4096 * 80 - 1, 4096 * 80 + 1])
+def test_join_order_with_a_known_row_count(vsabi, ctx, n_points, pairs):
+    """The pairs of a join, whose point count tells the bits of their left rows, sorted by runs of left rows."""
+    each = pairs // 4
+    assert _joined(vsabi, ctx, *_squares(n_points, [each, each, each, pairs - 3 * each])) == pairs
+
+
+def test_join_order_with_one_row_of_many_pairs(vsabi, ctx):
+    """Few pairs a row on average, but some rows with more than the run pass orders: sorted again by all digits."""
+    n = 100_007
+    pairs = _joined(vsabi, ctx, *_squares(n, [n] * 2 + [7] * 3_500))
+    assert pairs == 2 * n + 7 * 3_500 and pairs < 8 * n
