@@ -39,9 +39,11 @@ struct ExportState {
     uint32_t pad;
 };
 
-// Pairs whose rows fall outside [0, n_left) x [0, n_right) are counted.
+// Without a filter every pair is kept; those whose rows fall outside
+// [0, n_left) x [0, n_right) are counted.
 __global__ void export_check_kernel(const int32_t* __restrict__ l, const int32_t* __restrict__ r, int64_t n,
                                     int64_t n_left, int64_t n_right, ExportState* __restrict__ st) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) st->kept = (uint32_t)n;
     uint32_t b = 0;
     for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x)
         b += (l[k] < 0 || l[k] >= n_left || r[k] < 0 || r[k] >= n_right) ? 1u : 0u;
@@ -404,8 +406,7 @@ int vs_join_export(vs_context* ctx, const int32_t* d_left, const int32_t* d_righ
     Scratch<ExportState> state;
     VS_TRY(state.alloc(1, s));
     ExportState h{};
-    h.kept = (uint32_t)n_pairs;  // without a filter
-    VS_CUDA_TRY(cudaMemcpyAsync(state.p, &h, sizeof(h), cudaMemcpyHostToDevice, s));
+    VS_CUDA_TRY(cudaMemsetAsync(state.p, 0, sizeof(h), s));
     // the state after all passes so far, and what it says of the pairs
     auto read_state = [&]() -> int {
         VS_CUDA_TRY(cudaMemcpyAsync(&h, state.p, sizeof(h), cudaMemcpyDeviceToHost, s));
