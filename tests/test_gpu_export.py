@@ -169,3 +169,28 @@ def test_export_of_shuffled_pairs_over_many_tiles(ctx, vsabi):
     assert torch.equal(gl, sl) and torch.equal(gr, sr)
     assert torch.equal(torch.where(gs >= 0, dm[gs.clamp(min=0)], gs), ss)
     assert t_mixed < 20 * t_sorted, (t_mixed, t_sorted)
+
+
+@pytest.mark.parametrize("how", ["left", "right", "outer"])
+@pytest.mark.parametrize("rows", [3, 2048, 2049, 5000])
+def test_export_tiles_of_many_pairs(ctx, vsabi, how, rows):
+    """Tiles whose pairs several blocks write (from 32768 pairs a tile on), up to more than one of them, with most
+    pairs in a few rows and some rows without."""
+    import torch
+
+    rng = np.random.default_rng(rows)
+    l = np.minimum(rng.integers(0, rows, 700_000), rng.integers(0, rows, 700_000))
+    r = rng.integers(0, 90_000, 700_000)
+    u = np.unique(l.astype(np.int64) * 90_000 + r)
+    u = u[u // 90_000 % 7 != 3]
+    l, r = (u // 90_000).astype(np.int32), (u % 90_000).astype(np.int32)
+    n_left, n_right = (rows, 90_000) if how != "right" else (90_000, rows)
+    if how == "right":
+        l, r = r, l
+        o = np.lexsort((r, l))
+        l, r = l[o], r[o]
+    el, er, es = vs_sjoin._join_indexers(l, r, n_left, n_right, how, None)
+    gl, gr, gs = vsabi.join_export(ctx, torch.from_numpy(l).cuda(), torch.from_numpy(r).cuda(), n_left, n_right, how)
+    np.testing.assert_array_equal(gl.cpu().numpy(), el)
+    np.testing.assert_array_equal(gr.cpu().numpy(), er)
+    np.testing.assert_array_equal(gs.cpu().numpy(), es)

@@ -20,6 +20,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
+
 #include "join.cuh"
 #include "primitives.cuh"
 #include "vs_common.cuh"
@@ -241,7 +243,12 @@ __device__ __forceinline__ uint64_t row_pack(uint32_t c) { return (uint64_t)c | 
 // is marked in shared memory (searched for in tiles with more outputs).
 // Bound by the 24 bytes a row it writes.  21M rows: 165 us with per-row counts
 // read from memory and a search for every output row.
+// Tiles of many pairs take several blocks (gridDim.y), each of which counts
+// the tile's pairs and writes its share of the output: 1000 rows of 400 pairs,
+// one tile, are a call of 1328 us with one block and of 201 with 24.
 constexpr int kOwners = 4096;
+constexpr int64_t kBlockPairs = 16384;  // pairs a tile has on average for each of its blocks, at most kTileBlocks
+constexpr int kTileBlocks = 64;
 
 __global__ void __launch_bounds__(kTileThreads) export_write_kernel(
     const ExportPairs pairs, int64_t n_drive, const uint32_t* __restrict__ first, const uint32_t* __restrict__ matched,
@@ -293,7 +300,7 @@ __global__ void __launch_bounds__(kTileThreads) export_write_kernel(
     __syncthreads();
     const int64_t out_base = p0 + (base - (int64_t)matched[blockIdx.x]);
     const uint32_t total = s_start[kTileRows];
-    for (uint32_t o = t; o < total; o += kTileThreads) {
+    for (uint32_t o = blockIdx.y * kTileThreads + t; o < total; o += gridDim.y * kTileThreads) {
         // the row that owns o: s_start[lo] <= o < s_start[lo + 1]
         int lo = 0;
         if (o < (uint32_t)kOwners) {
@@ -514,7 +521,8 @@ int vs_join_export(vs_context* ctx, const int32_t* d_left, const int32_t* d_righ
         }
         VS_TRY(exclusive_scan_u32(matched.p, matched.p, n_tiles, &state.p->distinct, s));
         if (n_tiles > 0) {
-            export_write_kernel<<<(unsigned)n_tiles, kTileThreads, 0, s>>>(
+            const int64_t blocks = std::min<int64_t>(std::max<int64_t>(n_pairs / (n_tiles * kBlockPairs), 1), kTileBlocks);
+            export_write_kernel<<<dim3((unsigned)n_tiles, (unsigned)blocks), kTileThreads, 0, s>>>(
                 pairs, n_drive, first.p, matched.p, state.p, capacity, right ? d_out_right : d_out_left,
                 right ? d_out_left : d_out_right, d_out_src);
             VS_LAUNCHED("export_write", s);
