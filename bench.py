@@ -650,8 +650,7 @@ def run_distance(args, rank, world, local_rank):
         total_ms, e2e_med = float(t[0]), float(t[1])
     else:
         e2e_med = float(np.median(e2e_ms))
-    # points every rank processed per step: N each (weak), or the one dataset (sharded)
-    n_job = w.n_points if sharded else world * N
+    n_job = world * N  # points every rank processed per step: N each (weak)
     value = n_job * args.steps / (total_ms / 1e3)
     if rank != 0:
         return
