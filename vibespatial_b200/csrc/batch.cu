@@ -336,6 +336,7 @@ struct vs_batch_plan {
     vs::LearnedJob h_single{};  // the descriptor when the batch has one job
     int64_t n_cells = 0;        // batch-wide learned cells
     bool sparse = true;         // every job's learned index is sparse
+    bool occ_rows = false;      // some job's learned index is sparse
     bool has_ring_bins = false; // some job's index has binned rings long enough for the split walk
     void* lscratch = nullptr;
     vs::LearnedScratch lsc{};
@@ -402,6 +403,7 @@ int enqueue_batch(vs_batch_plan* p, cudaStream_t s, int mask, int32_t* left, int
         q.n_cells = p->n_cells;
         q.accept_mask = mask;
         q.sparse = p->sparse;
+        q.occ_rows = p->occ_rows;
         q.has_ring_bins = p->has_ring_bins;
         q.shape.map_blocks_per_sm = p->opts.learned_map_blocks_per_sm;
         q.shape.refine_blocks_per_sm = p->opts.learned_refine_blocks_per_sm;
@@ -579,6 +581,7 @@ int vs_batch_plan_create(vs_context* ctx, const vs_index* const* indexes, int32_
                 d.cell_base = (uint32_t)base;
                 base += ix->learned.n_cells;
                 if (d.occ_rows < 0) p->sparse = false;
+                else p->occ_rows = true;
             } else if (has_polys) {
                 set_error("job %d: index was built without its learned part", j);
                 delete p;

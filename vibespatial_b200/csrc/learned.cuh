@@ -36,6 +36,7 @@ struct LearnedQuery {
     int64_t n_cells;  // batch-wide cells
     int accept_mask;
     bool sparse;         // every job's index is sparse (its occupancy bitmap is in row order)
+    bool occ_rows;       // some job's index is
     bool has_ring_bins;  // some job's index has y-binned rings long enough for the split walk
     int64_t row_base;    // added to every emitted / deferred point row (chunked joins)
     LearnedShape shape;  // launch shape and ablation switches (zero = defaults)

@@ -267,9 +267,11 @@ __device__ __forceinline__ bool learned_occupied_rows(const LearnedJob& J, uint3
     return (J.occ[ob >> 5] >> (ob & 31)) & 1u;
 }
 
-// The same for either order; cell is the point's level-L cell key.
+// The same for a bitmap in key order, or with kRows in either; cell is the
+// point's level-L cell key.
+template <bool kRows>
 __device__ __forceinline__ bool learned_occupied(const LearnedJob& J, uint32_t gx, uint32_t gy, uint32_t cell) {
-    if (J.occ_rows >= 0) return learned_occupied_rows(J, gx, gy);
+    if (kRows && J.occ_rows >= 0) return learned_occupied_rows(J, gx, gy);
     const uint32_t ob = cell >> J.occ_shift;
     return (J.occ[ob >> 5] >> (ob & 31)) & 1u;
 }
@@ -371,7 +373,7 @@ __device__ __forceinline__ void map_pending(const LqArgs& a, const PendingPoint*
 
 // One point of the map pass: its batch-wide cell (-1: none) and its FP32
 // offsets from the cell's anchor (|offset| <= half a cell).
-template <bool kMulti, bool kBsearch>
+template <bool kMulti, bool kBsearch, bool kRows>
 __device__ __forceinline__ int map_point(const LqArgs& a, int64_t i, int job, const uint16_t* lut,
                                          unsigned long long& n_wide, float& qx, float& qy) {
     const LearnedQuery& q = a.q;
@@ -383,7 +385,7 @@ __device__ __forceinline__ int map_point(const LqArgs& a, int64_t i, int job, co
         return -1;
     const uint32_t gx = quantize(x, J.lox, J.sx), gy = quantize(y, J.loy, J.sy);
     const uint32_t cell = hilbert_key_lut(gx, gy, J.L, lut);
-    const int c = learned_lookup<kBsearch>(J, cell, n_wide, learned_occupied(J, gx, gy, cell));
+    const int c = learned_lookup<kBsearch>(J, cell, n_wide, learned_occupied<kRows>(J, gx, gy, cell));
     if (c < 0) return -1;
     const int sh = 32 - J.L;
     qx = __double2float_rn(__dsub_rn(x, cell_anchor(J.lox, J.cwx, gx >> sh)));
@@ -416,7 +418,9 @@ __device__ __forceinline__ void map_emit(const LqArgs& a, int64_t b0, int lane, 
 // CellPoints.  A warp takes kPackets packets of 32 points per iteration and
 // runs their lookups together, so that many independent chains of dependent
 // index loads (occupancy bit, root table, leaf, binary search) are in flight.
-template <bool kMulti, bool kBsearch, int kPackets>
+// kRows: some job's bitmap is in row order (a look at which took 10 us more on
+// Zipf: 902 -> 912 us).
+template <bool kMulti, bool kBsearch, bool kRows, int kPackets>
 __global__ void __launch_bounds__(kThreads, kPackets == 1 ? 8 : 6) learned_map_kernel(const LqArgs a) {
     __shared__ uint16_t s_lut[kHilbertLutSize];
     hilbert_lut_init(s_lut);
@@ -435,7 +439,7 @@ __global__ void __launch_bounds__(kThreads, kPackets == 1 ? 8 : 6) learned_map_k
             const int64_t bu = b0 + 32 * u;
             const int job = packet_job<kMulti>(q, bu < q.n ? bu : b0, bu + lane, lane);
             qx[u] = qy[u] = 0.f;
-            gc[u] = map_point<kMulti, kBsearch>(a, bu + lane, job, s_lut, n_wide, qx[u], qy[u]);
+            gc[u] = map_point<kMulti, kBsearch, kRows>(a, bu + lane, job, s_lut, n_wide, qx[u], qy[u]);
         }
 #pragma unroll
         for (int u = 0; u < kPackets; ++u) map_emit(a, b0 + 32 * u, lane, gc[u], qx[u], qy[u]);
@@ -607,7 +611,7 @@ __device__ __forceinline__ GroupedLane load_grouped(const LqArgs& a, int64_t j, 
         g.lo = J.cell_start[c];
         g.len = J.cell_start[c + 1] - g.lo;
     }
-    g.dq = point_error(g.p.qx, g.p.qy);
+    g.dq = __fmaf_ru(fmaxf(fabsf(g.p.qx), fabsf(g.p.qy)), 6.1e-8f, 1e-37f);  // point_error
     return g;
 }
 
@@ -802,10 +806,17 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) learned_refine_kernel(co
                 bool walk = false, direct = false;
                 if (inbox) {
                     ++n_cand;
-                    slot_offset(r, g.p.qx, g.p.qy, g.dq, sx, sy, t);
+                    // (slot_offset and in_interior_box, written out: through them
+                    // this kernel took 1% longer, 1597 against 1578 us on Zipf)
+                    sx = __fadd_rn(g.p.qx, r.offx);
+                    sy = __fadd_rn(g.p.qy, r.offy);
+                    const float es = __fmaf_ru(fmaxf(fabsf(sx), fabsf(sy)), 6.1e-8f, 1e-37f);
+                    t = __fmul_ru(__fadd_ru(__fadd_ru(r.err, g.dq), es), 1.0001f);
                     walk = true;
                     if (!a.no_interior && entry_has_interior(r)) {
-                        if (in_interior_box(ib32[entry_slot(r)], sx, sy, t)) {
+                        const float4 ib = ib32[entry_slot(r)];
+                        if (__fsub_rd(sx, t) > ib.x && __fadd_ru(sx, t) < ib.z && __fsub_rd(sy, t) > ib.y &&
+                            __fadd_ru(sy, t) < ib.w) {
                             walk = false;
                             direct = (a.q.accept_mask >> LOC_INTERIOR) & 1;
                         }
@@ -933,7 +944,7 @@ __global__ void __launch_bounds__(kDirectThreads) learned_direct_kernel(const Di
                 const uint32_t gx = quantize(x, J.lox, J.sx), gy = quantize(y, J.loy, J.sy);
                 unsigned long long wide = 0;
                 const uint32_t cell = (uint32_t)hilbert_key(gx, gy, J.L);
-                const int c = learned_lookup<false>(J, cell, wide, learned_occupied(J, gx, gy, cell));
+                const int c = learned_lookup<false>(J, cell, wide, learned_occupied<true>(J, gx, gy, cell));
                 n_wide += sub == 0 ? wide : 0;
                 if (c >= 0) {
                     const int sh = 32 - J.L;
@@ -1031,9 +1042,11 @@ __global__ void __launch_bounds__(kDirectThreads) learned_direct_kernel(const Di
     }
 }
 
+// Points a region has room for.  (A packet more than it holds, so that the
+// regions do not begin a multiple of 4 KB apart: place on Zipf 786 -> 772 us.)
 int64_t stripe_cap_for(int64_t n) {
     const int64_t points = 32 * (int64_t)unit_packets(n), units = (n + points - 1) / points;
-    return points * ((units + kStripes - 1) / kStripes);
+    return points * ((units + kStripes - 1) / kStripes) + 32;
 }
 
 size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
@@ -1095,13 +1108,16 @@ int launch_passes(cudaStream_t s, vs_context* ctx, const LqArgs& a) {
     const int map_grid = grid_for(n, kThreads, sh.map_blocks_per_sm > 0 ? sh.map_blocks_per_sm : 8);
     const bool two = sh.map_packets == 2;
     if (sh.flags & kLearnedBsearch) {
-        if (two) learned_map_kernel<kMulti, true, 2><<<map_grid, kThreads, 0, s>>>(a);
-        else learned_map_kernel<kMulti, true, 1><<<map_grid, kThreads, 0, s>>>(a);
+        if (two) learned_map_kernel<kMulti, true, true, 2><<<map_grid, kThreads, 0, s>>>(a);
+        else learned_map_kernel<kMulti, true, true, 1><<<map_grid, kThreads, 0, s>>>(a);
     } else if (a.q.sparse && n >= kSparseMapPoints) {
         learned_map_sparse_kernel<kMulti><<<map_grid, kThreads, 0, s>>>(a);
+    } else if (a.q.occ_rows) {
+        if (two) learned_map_kernel<kMulti, false, true, 2><<<map_grid, kThreads, 0, s>>>(a);
+        else learned_map_kernel<kMulti, false, true, 1><<<map_grid, kThreads, 0, s>>>(a);
     } else {
-        if (two) learned_map_kernel<kMulti, false, 2><<<map_grid, kThreads, 0, s>>>(a);
-        else learned_map_kernel<kMulti, false, 1><<<map_grid, kThreads, 0, s>>>(a);
+        if (two) learned_map_kernel<kMulti, false, false, 2><<<map_grid, kThreads, 0, s>>>(a);
+        else learned_map_kernel<kMulti, false, false, 1><<<map_grid, kThreads, 0, s>>>(a);
     }
     VS_LAUNCHED("learned_map", s);
     VS_TRY(exclusive_scan_u32(a.cell_count, a.cell_count, a.q.n_cells, (uint32_t*)a.n_grouped, s));
@@ -1196,7 +1212,7 @@ int launch_learned_join(vs_context* ctx, const vs_index* idx, const vs_points* p
     q.n_cells = li.n_cells;
     q.accept_mask = accept_mask;
     q.has_ring_bins = idx->n_split_binned_rings > 0;
-    q.sparse = li.h_desc.occ_rows >= 0;
+    q.sparse = q.occ_rows = li.h_desc.occ_rows >= 0;
     q.row_base = row_base;
     q.shape = shape;
     const PairSink sink{d_left, d_right, (unsigned long long)(capacity > 0 ? capacity : 0), &ctx->d_counters[0]};
