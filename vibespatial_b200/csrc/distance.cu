@@ -342,6 +342,7 @@ __global__ void __launch_bounds__(kDistThreads) dist_join_kernel(const DistArgs 
     __shared__ int s_stack[kDistWarps][kDistStack];
     __shared__ vs_box s_items[kDistWarps][kFanout];
     __shared__ DwPair s_dq[kDistWarps][kQ];
+    if (kMode != kDwithin && *a.n_packets == 0) return;  // (nearly every call of the nearest walks)
     const int64_t stage_base = a.level_off[a.stage_level];
     for (int k = threadIdx.x; k < a.staged; k += blockDim.x) s_nodes[k] = a.nodes[stage_base + k];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -849,6 +850,7 @@ __global__ void __launch_bounds__(kDistThreads, 3) near_kernel(const NearArgs na
     __shared__ unsigned s_cnt[kDistWarps];
     __shared__ PacketShared s_walk[kDistWarps];
     __shared__ NearShared s_near[kDistWarps];
+    if (kCrowded && *na.crowded.count == 0) return;
     const int64_t stage_base = a.level_off[a.stage_level];
     for (int k = threadIdx.x; k < a.staged; k += blockDim.x) s_nodes[k] = a.nodes[stage_base + k];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1295,6 +1297,7 @@ __global__ void __launch_bounds__(kDistThreads) poly_nearest_kernel(const PolyAr
     __shared__ int s_stack[kDistWarps][kDistStack];
     __shared__ vs_box s_items[kDistWarps][kFanout];
     __shared__ DwPair s_dq[kDistWarps][kQ];
+    if (*a.n_packets == 0) return;
     const int64_t stage_base = a.level_off[a.stage_level];
     for (int k = threadIdx.x; k < a.staged; k += blockDim.x) s_nodes[k] = a.nodes[stage_base + k];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
