@@ -5,7 +5,8 @@ parameters: join-kernel blocks per SM, 32-point packets a warp takes per grab
 of the work counter, and the Hilbert levels the points of a job are sorted by
 (more levels: coherent packets but more radix passes).  The learned batch
 (``VS_METHOD_LEARNED``) has four of its own: map-pass blocks per SM, the
-32-point packets a map warp looks up together (1 or 2), refine blocks per SM
+32-point packets a map warp looks up together (1 or 2; the map pass of sparse
+indexes has no use for it), refine blocks per SM
 (4 or fewer run the 64-register refine build, 5 the 48-register one), and the
 grouped points a refine warp takes per grab of its work counter.  The best values depend on the device and on the batch's shape
 (job count, points per job, polygons per job), so they are searched by timing

@@ -48,7 +48,8 @@ struct LearnedQuery {
 // us with and without: clustered footprints, share 0.004: 70 and 120, 0.021: 84
 // and 158, 0.073: 145 and 162, 0.15: 213 and 189; points where the footprints
 // are (most hit), share 0.010: 85 and 165, 0.037: 134 and 173, 0.082: 198 and
-// 184; a full grid (0.90): 266 and 229.
+// 184; a full grid (0.90): 266 and 229.  Points that all hit and come in random
+// order are the other side of this rule: 12M points, share 0.02, 428 and 387.
 inline bool sparse_map_pays(int64_t n_cells, int64_t grid_cells) { return n_cells < grid_cells / 16; }
 // Points from which it pays there: below, units large enough for whole lookups
 // are too few to go round, and smaller ones wait for their counter.  One join

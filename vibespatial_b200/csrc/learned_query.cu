@@ -862,8 +862,8 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) learned_refine_kernel(co
 // call is one launch and one wait.
 //
 // Bound by latency: the chain of dependent index loads, then the launch and
-// the wait themselves (1003 points x 10 stars: 31 us a call; the grouped
-// passes, their counters, events and sort took 121).
+// the wait themselves (1003 points x 10 stars: 25 us a call; the grouped
+// passes, their counters, events and sort took 129).
 constexpr int kDirectThreads = 256;
 constexpr int kDirectSort = 512;  // pairs the last block sorts (each compared with all others)
 
